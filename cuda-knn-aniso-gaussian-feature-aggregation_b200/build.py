@@ -28,7 +28,7 @@ BUILD = os.path.join(HERE, "_build")
 CUDA_HOME = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 NVCC = os.path.join(CUDA_HOME, "bin", "nvcc")
 
-CU_SOURCES = ["knn_search.cu", "knn_search_tc.cu", "knn_spatial.cu", "knn_adjoint.cu", "knn_capi.cu", "knn_noalloc.cu", "knn_variants.cu",
+CU_SOURCES = ["knn_search.cu", "knn_search_warp.cu", "knn_search_tc.cu", "knn_spatial.cu", "knn_adjoint.cu", "knn_capi.cu", "knn_noalloc.cu", "knn_variants.cu",
               "knn_ragged.cu"]
 HEADERS = ["knn_common.cuh", "knn_internal.h", "knn_ragged.h", "knn_search_dev.cuh"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -51,7 +51,7 @@ def _run(cmd, verbose):
     subprocess.check_call(cmd)
 
 
-def build_lib(force=False, jobs=3, verbose=True) -> str:
+def build_lib(force=False, jobs=4, verbose=True) -> str:
     os.makedirs(BUILD, exist_ok=True)
     hdrs = [os.path.join(CSRC, h) for h in HEADERS] + [os.path.join(INCLUDE, "knn_aniso.h")]
     objs, cmds = [], []
@@ -93,7 +93,7 @@ def build_ext(force=False, verbose=True) -> str:
     return EXT
 
 
-def build(force=False, jobs=3, verbose=True):
+def build(force=False, jobs=4, verbose=True):
     build_lib(force, jobs, verbose)
     build_ext(force, verbose)
     return LIB, EXT
@@ -102,7 +102,7 @@ def build(force=False, jobs=3, verbose=True):
 if __name__ == "__main__":
     ap = argparse.ArgumentParser()
     ap.add_argument("--force", action="store_true")
-    ap.add_argument("--jobs", type=int, default=3)
+    ap.add_argument("--jobs", type=int, default=4)
     a = ap.parse_args()
     build(a.force, a.jobs)
     sys.exit(0)

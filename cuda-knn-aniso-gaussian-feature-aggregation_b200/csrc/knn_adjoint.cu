@@ -141,14 +141,38 @@ __device__ __forceinline__ int block_exclusive_scan_1024(int local, int* warp_su
   return warp_sums[warp] + incl - local;
 }
 
+// Eight consecutive ints from base (0 past n): two 128-bit loads where the
+// address allows.
+__device__ __forceinline__ void load8(const int* __restrict__ p, int64_t base, int64_t n, int (&v)[8]) {
+  if (base + 8 <= n && (reinterpret_cast<uintptr_t>(p + base) & 15u) == 0) {
+    const int4 a = *reinterpret_cast<const int4*>(p + base), b = *reinterpret_cast<const int4*>(p + base + 4);
+    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
+    v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+  } else {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = base + u < n ? p[base + u] : 0;
+  }
+}
+__device__ __forceinline__ void store8(int* __restrict__ p, int64_t base, int64_t n, const int (&v)[8]) {
+  if (base + 8 <= n && (reinterpret_cast<uintptr_t>(p + base) & 15u) == 0) {
+    *reinterpret_cast<int4*>(p + base) = make_int4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<int4*>(p + base + 4) = make_int4(v[4], v[5], v[6], v[7]);
+  } else {
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (base + u < n) p[base + u] = v[u];
+  }
+}
+
 __global__ void __launch_bounds__(1024) scan_chunk_sums_kernel(const int* __restrict__ count, int64_t n,
                                                                int* __restrict__ out) {
   __shared__ int warp_sums[33];
   const int64_t base = (int64_t)blockIdx.x * kScanChunk + (int64_t)threadIdx.x * 8;
+  int v[8];
+  load8(count, base, n, v);
   int local = 0;
 #pragma unroll
-  for (int u = 0; u < 8; ++u)
-    if (base + u < n) local += count[base + u];
+  for (int u = 0; u < 8; ++u) local += v[u];
   int total;
   block_exclusive_scan_1024(local, warp_sums, total);
   if (threadIdx.x == 0) out[(int64_t)blockIdx.x * kScanChunk] = total;
@@ -180,22 +204,22 @@ __global__ void __launch_bounds__(1024) scan_chunk_apply_kernel(int* __restrict_
   if (threadIdx.x == 0) prefix_s = out[chunk0];
   const int64_t base = chunk0 + (int64_t)threadIdx.x * 8;
   int v[8];
+  load8(count, base, n, v);
   int local = 0;
 #pragma unroll
-  for (int u = 0; u < 8; ++u) {
-    v[u] = base + u < n ? count[base + u] : 0;
-    local += v[u];
-  }
+  for (int u = 0; u < 8; ++u) local += v[u];
   int total;
   int run = block_exclusive_scan_1024(local, warp_sums, total) + prefix_s;  // barriers order the prefix read
+  int zero[8];
 #pragma unroll
   for (int u = 0; u < 8; ++u) {
-    if (base + u < n) {
-      out[base + u] = run;
-      count[base + u] = 0;
-    }
-    run += v[u];
+    const int c = v[u];
+    v[u] = run;
+    run += c;
+    zero[u] = 0;
   }
+  store8(out, base, n, v);
+  store8(count, base, n, zero);
 }
 
 __global__ void adj_fill_kernel(const int64_t* __restrict__ idxs, int n, int qk, int P, const int* __restrict__ rowptr,

@@ -110,7 +110,7 @@ int knnag_version(void) { return 10000; }
 size_t knnag_forward_workspace_bytes(int B, int Q, int P, int F, int K, int dtype) {
   (void)F;
   if (B < 0 || Q < 0 || P < 0 || K < 1) return 0;
-  return fwd_layout(B, Q, P, K, dtype, true).total;
+  return fwd_layout(B, Q, P, K, dtype, true, forward_indexed(B, P, K, dtype)).total;
 }
 
 size_t knnag_points_bytes(int B, int P, int dtype) {
@@ -132,11 +132,9 @@ int knnag_forward(const void* q, const void* p, const void* f, const void* sigma
   if ((int64_t)B * Q == 0) return KNNAG_OK;
   if (!q || !p || !sigma || !R || !w_out || !dists || !idxs || !workspace) return KNNAG_ERR_ARG;
   if (F > 0 && (!f || !f_out)) return KNNAG_ERR_ARG;
-  if (workspace_bytes < fwd_layout(B, Q, P, K, dtype, points == nullptr).total || !aligned16(workspace) ||
-      (points && !aligned16(points)))
-    return KNNAG_ERR_WORKSPACE;
+  if (!aligned16(workspace) || (points && !aligned16(points))) return KNNAG_ERR_WORKSPACE;
   return forward_impl(q, p, f, sigma, R, B, Q, P, F, K, dtype, f_out, w_out, dists, idxs, points, workspace,
-                      static_cast<cudaStream_t>(stream));
+                      workspace_bytes, static_cast<cudaStream_t>(stream));
 }
 
 int knnag_forward_counted(const void* q, const void* p, const void* f, const void* sigma, const void* R, int B,
@@ -148,11 +146,9 @@ int knnag_forward_counted(const void* q, const void* p, const void* f, const voi
   if ((int64_t)B * Q == 0) return KNNAG_OK;
   if (!q || !p || !sigma || !R || !w_out || !dists || !idxs || !workspace || !adjacency) return KNNAG_ERR_ARG;
   if (F > 0 && (!f || !f_out)) return KNNAG_ERR_ARG;
-  if (workspace_bytes < fwd_layout(B, Q, P, K, dtype, points == nullptr).total || !aligned16(workspace) ||
-      (points && !aligned16(points)) || !aligned16(adjacency))
-    return KNNAG_ERR_WORKSPACE;
+  if (!aligned16(workspace) || (points && !aligned16(points)) || !aligned16(adjacency)) return KNNAG_ERR_WORKSPACE;
   return forward_impl(q, p, f, sigma, R, B, Q, P, F, K, dtype, f_out, w_out, dists, idxs, points, workspace,
-                      static_cast<cudaStream_t>(stream), adjacency);
+                      workspace_bytes, static_cast<cudaStream_t>(stream), adjacency);
 }
 
 int knnag_build_adjacency_counted(const int64_t* idxs, int B, int Q, int P, int K, void* adjacency, void* stream) {

@@ -7,6 +7,7 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include "knn_aniso.h"
 #include "knn_ragged.h"
 
 namespace knnag {
@@ -101,29 +102,60 @@ struct SearchParams {
   const float* tcinfo;
 };
 
-// Search CTA: WPC warps (1, 2 or 4), each owning QPW queries (32, 16 or 8;
-// lane j < QPW keeps query j's list) and sharing the CTA's tile ring; a work
-// item is the CTA's WPC * QPW queries.  The C ABI's launch-shape code s
-// (knnag_set_search_splits, the segment tables' `splits`) selects
-//   s = 1: 4 warps x 32    s = 2: 2 x 32    s = 4: 1 x 32
-//   s = 8: 2 warps x 16    s = 16: 4 x 8    s = 32: 1 x 16    s = 64: 1 x 8
-// i.e. 128, 64, 32, 32, 32, 16 and 8 queries per CTA.
-constexpr int kSearchMaxThreads = 128;
-// Candidate queue entries per query: 64 points (the points a query meets
-// between two folds of its queue) always fit.
-constexpr int kQCap = 64;
-// Tile buffers of the search ring: visit v lands in buffer v % kTileBufs,
-// so kTileBufs - 1 copies are in flight while a tile is being read.
-constexpr int kTileBufs = 2;
-constexpr size_t kSearchTileBytes = 8192;  // 128 points x 16 floats
-static_assert(kTileBufs * 12 + 8 <= 64, "search ring bookkeeping exceeds its 64 bytes");
-__host__ __device__ inline constexpr int search_wpc(int shape) {
-  return shape == 1 ? 4 : shape == 2 ? 2 : shape == 4 ? 1 : shape == 8 ? 2 : shape == 16 ? 4 : 1;
+// One-warp-per-query search (knn_search_warp.cu).
+template <typename T>
+struct WarpSearchParams {
+  const T* q;
+  const int* perm_q;   // sorted position -> query index, per batch element
+  const int* qseed;    // uniform calls: per sorted query, a near position in the sorted points
+  const T* rec;        // per-point records [B*P*16]
+  const T* pairs;      // field-major tiles [B][ntile][16][64 pairs][2]
+  const float* tbox;   // tile boxes, 7 planes of B*ntile: min xyz, max xyz, mu
+  const float* gbox;   // boxes of groups of 32 tiles, 7 planes of B*ngroup
+  const float4* sbox;  // per tile 4 x (min xyz, mu), then 4 x (max xyz, 0) of its sub-boxes
+  const T* f;
+  int B, Q, P, F, K, ntile, ngroup;  // ragged: K and ntile are the most of any segment / cloud
+  int vec;             // f and f_out rows may be accessed 16 bytes at a time
+  T* f_out;
+  T* w_out;
+  T* dists;
+  int64_t* idxs;
+  int* status;
+  int* flag_count;
+  int* flag_list;      // flagged queries: global query rows
+  int* adj_count;      // optional (uniform calls): entries per point row, counted as written
+  // ragged calls: everything per cloud comes from the cloud set, sizes and
+  // offsets from the segment table, work items from item_counter
+  const char* cs;
+  const void* segs;
+  int* item_counter;
+};
+constexpr int kWarpSearchMaxK = 128;
+// Most tiles per cloud a search takes (P <= 2 097 152), as before this
+// kernel: larger clouds are refused with KNNAG_ERR_TOO_LARGE (FP32, K <= 32)
+// or go to the exact kernel (FP64, K > 32), which takes any size.
+constexpr int kSearchMaxTiles = 16384;
+// Warps (CTAs of one warp) per SM the registers are held to.  More warps hide
+// more of each one's latency, fewer spill less: 24, 28 and 32 warps took 62,
+// 64 and 62 us (table workload), 431, 433 and 420 us (65536 surface queries,
+// K = 32), 1.78, 1.74 and 1.67 ms (524288 sphere queries).
+template <typename T, int V>
+struct WarpSearchShape {
+  static constexpr int warps = sizeof(T) == 4 ? (V == 1 ? 32 : 16) : 8;
+};
+template <typename T>
+int launch_search_warp(const WarpSearchParams<T>& a, int shape, cudaStream_t st);
+int launch_search_warp_ragged(const WarpSearchParams<float>& a, int shape, int64_t cap_items, cudaStream_t st);
+
+// Launch shape of the search.  The C ABI's launch-shape code s
+// (knnag_set_search_splits, the segment tables' `splits`) selects the queries
+// a warp of a uniform call takes: 16, 8, 4, 4, 4, 2 and 1 for s = 1, 2, 4, 8,
+// 16, 32 and 64.  In segment tables it sets the size of the work items (128,
+// 64, 32, 32, 32, 16 and 8 queries), which the search takes a unit at a time.
+inline constexpr int search_qpc(int shape) {
+  return shape == 1 ? 128 : shape == 2 ? 64 : shape == 32 ? 16 : shape == 64 ? 8 : 32;
 }
-__host__ __device__ inline constexpr int search_qpw(int shape) {
-  return shape <= 4 ? 32 : (shape == 8 || shape == 32) ? 16 : 8;
-}
-__host__ __device__ inline constexpr int search_qpc(int shape) { return search_wpc(shape) * search_qpw(shape); }
+inline constexpr int search_qpw(int shape) { return search_qpc(shape) / 8; }
 inline bool search_shape_ok(int shape) {
   return shape == 1 || shape == 2 || shape == 4 || shape == 8 || shape == 16 || shape == 32 || shape == 64;
 }
@@ -133,46 +165,6 @@ inline bool search_shape_ok(int shape) {
 // codes above).
 constexpr int kShapeTensorFilter = 128;
 inline bool search_setting_ok(int shape) { return search_shape_ok(shape) || shape == kShapeTensorFilter; }
-
-// Shared-memory layout of the search kernel with `wpc` warps of `qpw` queries:
-//   ring      kTileBufs tiles
-//   queues    wpc x [qpw queries][kQCap] keys, then indices (after the tile
-//             loop: the CTA's sorted lists, weights and flags)
-//   qtab      [wpc qpw] float4 (x, y, z, threshold) of the CTA's queries
-//   ctab      per warp, the queries a pass matters to, compacted: [qpw]
-//             float4 (x, y, z, threshold) of the warp, then [qpw] their lanes
-//   tring     kTileBufs tile infos (box and sub-boxes), copied with the tiles
-//   misc      [wpc qpw] original query index, [wpc][6] warp query boxes,
-//             64 bytes of mbarriers / counters / flags
-//   region C  tile bounds and visit order [NTP x 8 B] + visit counter
-__host__ __device__ inline constexpr size_t search_queue_off() { return (size_t)kTileBufs * kSearchTileBytes; }
-__host__ __device__ inline constexpr size_t search_warp_queue_bytes(int qpw) { return (size_t)qpw * kQCap * 8; }
-__host__ __device__ inline constexpr size_t search_qtab_off(int wpc, int qpw) {
-  return search_queue_off() + (size_t)wpc * search_warp_queue_bytes(qpw);
-}
-__host__ __device__ inline constexpr size_t search_ctab_off(int wpc, int qpw) {
-  return search_qtab_off(wpc, qpw) + (size_t)wpc * qpw * 16;
-}
-__host__ __device__ inline constexpr size_t search_tring_off(int wpc, int qpw) {
-  return search_ctab_off(wpc, qpw) + (size_t)wpc * qpw * 20;
-}
-__host__ __device__ inline constexpr size_t search_misc_off(int wpc, int qpw) {
-  return search_tring_off(wpc, qpw) + (size_t)kTileBufs * kTinfoBytes;
-}
-__host__ __device__ inline constexpr size_t search_bars_off(int wpc, int qpw) {
-  return search_misc_off(wpc, qpw) + (size_t)wpc * qpw * 4 + (size_t)wpc * 6 * 4;
-}
-__host__ __device__ inline constexpr size_t search_smem_bytes(int wpc, int qpw) { return search_bars_off(wpc, qpw) + 64; }
-// Tiles per cloud rounded up to a power of two (the visit-order sort).
-__host__ __device__ inline int search_tiles_pow2(int ntile) {
-  int n = 1;
-  while (n < ntile) n <<= 1;
-  return n;
-}
-__host__ __device__ inline size_t search_region_c_bytes(int ntile) { return (size_t)search_tiles_pow2(ntile) * 8 + 16; }
-// The sorted lists of a query (keys, indices, weights) and its flag, staged
-// for the epilogue, must fit the query's share of the queue region.
-static_assert((size_t)33 * 12 + 4 <= (size_t)kQCap * 8, "epilogue staging exceeds the queue region");
 
 // ------------------------------------------------------------- workspace
 // Forward workspace: [status, flag_count] | flag_list [B*Q] | records (when
@@ -185,12 +177,32 @@ struct FwdLayout {
   size_t qseed;  // [B*Q] ints: seed positions of the sorted queries
   size_t tau0, plan_est, items;  // search plan: seeds [B*Q], estimates, CTA items
   size_t tcops, tcinfo;          // tensor-core filter: per tile B operand and bound terms
+  size_t tbox, gbox, sbox;       // boxes of tiles, groups of tiles, sub-boxes (see WarpSearchParams)
+  size_t pf, qf;                 // FP64: points and queries rounded to FP32 (what the cells are taken from)
   int P_pad, bits;
 };
-int spatial_bits(int P);
+// Whether a call is served through the spatial index (else by the exact
+// kernel).  FP64 and K > 32 had only the exact kernel and its small
+// workspace: they take the index where its padded tiles at most double the
+// points and the launches' grids hold the batch.
+inline bool forward_indexed(int B, int P, int K, int dtype) {
+  if (dtype == KNNAG_F32 && K <= 32) return true;
+  return K <= kWarpSearchMaxK && P >= kTilePoints && B <= 65535 && (int64_t)P <= (int64_t)kSearchMaxTiles * kTilePoints;
+}
+// Grid bits per axis of n elements: 8^bits cells hold at most 8 of them each on
+// average.
+int spatial_bits(int n);
+// The same for P points: at least one cell per point beyond 4096 points.
+// Points that fill no volume (surfaces, clusters) crowd into few cells, whose
+// inner order is random; with the finer grid a query of the 131072-point
+// sphere visits 14 instead of 15 sub-boxes and the unit of four 18 instead of
+// 22, one of a cluster mixture (P = 30000, K = 32) 37 instead of 51.  Up to
+// 4096 points the coarse grid keeps the scan inside the scatter launch.
+int point_bits(int P);
 // tc_ops: also write the tensor-core filter's per-tile operands (L.tcops, L.tcinfo)
-int launch_spatial_index(const float* q, const float* rec, int B, int Q, int P, int P_pad, char* ws, const FwdLayout& L,
-                         cudaStream_t st, bool tc_ops = false);
+template <typename T>
+int launch_spatial_index(const float* qf, const float* pf, const T* rec, int B, int Q, int P, int P_pad, char* ws,
+                         const FwdLayout& L, cudaStream_t st, bool tc_ops = false);
 int launch_exclusive_scan(int* count, int n, int* out, cudaStream_t st);
 int launch_cloudset_index(char* cs, const CloudSetHeader& h, const CloudDesc* cd_dev, int max_p, int max_ntile,
                           int* cnt, int* perm_p, cudaStream_t st);
@@ -222,7 +234,11 @@ int variants_precomputed(const void* q, const void* f, const void* rec, const in
 int variants_lookup(const void* q, const void* p, const void* f, const void* rec, const int64_t* table, int tstride, int B, int Q,
                     int P, int F, int K, int dtype, int* nearest, void* f_out, void* w_out, void* dists,
                     int64_t* idxs, cudaStream_t st);
-FwdLayout fwd_layout(int B, int Q, int P, int K, int dtype, bool own_rec);
+FwdLayout fwd_layout(int B, int Q, int P, int K, int dtype, bool own_rec, bool indexed);
+// The layout a workspace of `bytes` holds: the indexed one where the call is
+// served through the index and it fits, else the exact kernel's (FP64 and
+// K > 32 only); L.total > bytes when neither fits.
+FwdLayout fwd_layout_in(int B, int Q, int P, int K, int dtype, bool own_rec, size_t bytes, bool* indexed);
 
 // Adjacency (CSR) layout: rowptr [B*P+1] | cursor [B*P] | unsorted [N] | entries [N].
 struct AdjLayout {
@@ -285,14 +301,15 @@ int launch_pack_points(const void* p, const void* sigma, const void* R, int B, i
 // points: chunk c of element b writes its box to parts[(b * kBoundParts +
 // c) * 8 ...] (min xyz, max xyz), which the cell kernels reduce.
 constexpr int kBoundParts = 32;
-int launch_pack_points_bounded(const float* p, const float* sigma, const float* R, int B, int P, float* rec,
-                               float* parts, cudaStream_t st, int* zero_words, int n_zero, int* zero_rows,
-                               int* zero_cells, int64_t n_cells);
+template <typename T>
+int launch_pack_points_bounded(const T* p, const T* sigma, const T* R, const T* q, int B, int Q, int P, T* rec,
+                               float* parts, float* pf, float* qf, cudaStream_t st, int* zero_words, int n_zero,
+                               int* zero_rows, int* zero_cells, int64_t n_cells);
 // adjacency: optional buffer (adj_layout) whose per-point entry counts the
 // forward writes, for launch_build_adjacency(..., counted = true)
 int forward_impl(const void* q, const void* p, const void* f, const void* sigma, const void* R, int B, int Q,
                  int P, int F, int K, int dtype, void* f_out, void* w_out, void* dists, int64_t* idxs,
-                 void* points, void* workspace, cudaStream_t st, void* adjacency = nullptr);
+                 void* points, void* workspace, size_t workspace_bytes, cudaStream_t st, void* adjacency = nullptr);
 int launch_build_adjacency(const int64_t* idxs, int B, int Q, int P, int K, void* adjacency, cudaStream_t st,
                            bool counted = false);
 

@@ -80,11 +80,14 @@ extern "C" int knnag_forward_noalloc(const void* q, const void* p, const void* f
   if ((int64_t)B * Q == 0) return KNNAG_OK;
   if (!q || !p || !sigma || !R || !w_out || !dists || !idxs) return KNNAG_ERR_ARG;
   if (F > 0 && (!f || !f_out)) return KNNAG_ERR_ARG;
-  if (fwd_layout(B, Q, P, K, dtype, true).total > kNoallocScratchBytes) return KNNAG_ERR_SCRATCH_LIMIT;
+  // FP64 and K > 32 calls whose index does not fit run the exact kernel alone
+  bool indexed = false;
+  if (fwd_layout_in(B, Q, P, K, dtype, true, kNoallocScratchBytes, &indexed).total > kNoallocScratchBytes)
+    return KNNAG_ERR_SCRATCH_LIMIT;
   void* scratch = noalloc_scratch_on_current_device();
   if (!scratch) return KNNAG_ERR_CUDA;
   return forward_impl(q, p, f, sigma, R, B, Q, P, F, K, dtype, f_out, w_out, dists, idxs, nullptr, scratch,
-                      static_cast<cudaStream_t>(stream));
+                      kNoallocScratchBytes, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int knnag_noalloc_read_device_status(void* stream) {

@@ -29,7 +29,7 @@ size_t cloudset_layout(int C, const int* P, CloudSetHeader* h, CloudDesc* descs)
   int max_ntile = 0;
   for (int c = 0; c < C; ++c) {
     if (P[c] < 1) return 0;
-    const int bits = spatial_bits(P[c]);
+    const int bits = point_bits(P[c]);
     const int ntile = (int)((P[c] + kTilePoints - 1) / kTilePoints);
     if (descs) descs[c] = CloudDesc{total_p, total_tiles, P[c], ntile, bits, (int)total_cells};
     total_p += P[c];
@@ -51,7 +51,10 @@ size_t cloudset_layout(int C, const int* P, CloudSetHeader* h, CloudDesc* descs)
   x.tinfo_off = x.pairs_off + (int64_t)align256((size_t)total_tiles * kTilePoints * kRecLen * 4);
   x.bnd_off = x.tinfo_off + (int64_t)align256((size_t)total_tiles * kTinfoBytes);
   x.celloff_off = x.bnd_off + (int64_t)align256((size_t)C * 8 * 4);
-  x.total_bytes = x.celloff_off + (int64_t)align256(((size_t)total_cells + 1) * 4);
+  x.tbox_off = x.celloff_off + (int64_t)align256(((size_t)total_cells + 1) * 4);
+  x.sbox_off = x.tbox_off + (int64_t)align256((size_t)total_tiles * 7 * 4);
+  x.gbox_off = x.sbox_off + (int64_t)align256((size_t)total_tiles * 8 * 16);
+  x.total_bytes = x.gbox_off + (int64_t)align256((size_t)tile_groups(total_tiles, C) * 7 * 4);
   if (h) *h = x;
   return (size_t)x.total_bytes;
 }

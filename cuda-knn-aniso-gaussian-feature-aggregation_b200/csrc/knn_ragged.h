@@ -38,7 +38,16 @@ struct CloudSetHeader {
   // [total_cells + 1] (global point positions): where a query's cell starts
   // in its cloud's sorted points, for the search's seed windows
   int64_t celloff_off;
+  // tile boxes (7 planes of total_tiles floats: min xyz, max xyz, mu) and
+  // sub-boxes (8 float4 per tile: 4 x (min xyz, mu), 4 x (max xyz, 0)); boxes
+  // of groups of 32 tiles (7 planes of tile_groups() floats)
+  int64_t tbox_off, sbox_off, gbox_off;
 };
+
+// Groups of 32 tiles: cloud c's start at first_group(tile_off, c) (disjoint
+// for any tile counts), out of tile_groups() in all.
+__host__ __device__ inline int64_t first_group(int64_t tile_off, int c) { return tile_off / 32 + c; }
+__host__ __device__ inline int64_t tile_groups(int64_t total_tiles, int C) { return total_tiles / 32 + C; }
 
 struct SegDesc {
   int64_t q_off;    // first query row

@@ -44,31 +44,38 @@ __device__ __forceinline__ void pack_one(const T* __restrict__ p, const T* __res
   store_rec(rec + i * kRecLen, v);
 }
 
-// FP32 packing of the search path, grid (kBoundParts, B): CTA (c, b) packs
+// Packing of the search path, grid (kBoundParts, B): CTA (c, b) packs
 // chunk c of batch element b's points, writes the chunk's bounding box to
 // parts (what the cell kernels reduce to the element's box), zeroes the
 // chunk's adjacency counts (zero_rows, optional) and its share of the cell
-// counts; CTA (0, 0) zeroes the call's status words.
+// counts; CTA (0, 0) zeroes the call's status words.  FP64 calls also get
+// their points and queries rounded to FP32 (pf, qf): the cells are taken
+// from those, and so are the boxes of the cells' grid.
+template <typename T>
 __global__ void __launch_bounds__(256) pack_points_bounded_kernel(
-    const float* __restrict__ p, const float* __restrict__ sigma, const float* __restrict__ R, int P,
-    float* __restrict__ rec, float* __restrict__ parts, int* __restrict__ zero_words, int n_zero,
-    int* __restrict__ zero_rows, int* __restrict__ zero_cells, int64_t n_cells) {
+    const T* __restrict__ p, const T* __restrict__ sigma, const T* __restrict__ R, const T* __restrict__ q, int Q,
+    int P, T* __restrict__ rec, float* __restrict__ parts, float* __restrict__ pf, float* __restrict__ qf,
+    int* __restrict__ zero_words, int n_zero, int* __restrict__ zero_rows, int* __restrict__ zero_cells,
+    int64_t n_cells) {
   __shared__ float red[6][8];
   const int c = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (c == 0 && b == 0 && tid < n_zero) zero_words[tid] = 0;
   const int64_t flat = ((int64_t)b * gridDim.x + c) * blockDim.x + tid;
   const int64_t nthreads = (int64_t)gridDim.x * gridDim.y * blockDim.x;
   for (int64_t i = flat; i < n_cells; i += nthreads) zero_cells[i] = 0;
+  if constexpr (sizeof(T) == 8)
+    for (int64_t i = flat; i < (int64_t)gridDim.y * Q * 3; i += nthreads) qf[i] = (float)q[i];
   const int chunk = (P + kBoundParts - 1) / kBoundParts;
   const int i0 = min(P, c * chunk), i1 = min(P, i0 + chunk);
   float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
   for (int k = i0 + tid; k < i1; k += blockDim.x) {
     const int64_t i = (int64_t)b * P + k;
-    pack_one<float>(p, sigma, R, i, rec);
+    pack_one<T>(p, sigma, R, i, rec);
     if (zero_rows) zero_rows[i] = 0;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      const float v = p[i * 3 + a];
+      const float v = (float)p[i * 3 + a];
+      if constexpr (sizeof(T) == 8) pf[i * 3 + a] = v;
       mn[a] = fminf(mn[a], v);
       mx[a] = fmaxf(mx[a], v);
     }
@@ -396,658 +403,6 @@ __global__ void __launch_bounds__(NTH) mink_replay_kernel(ExactParams<T> a) {
   }
 }
 
-// ------------------------------------------------------- fused FP32 search
-//
-// CTA = WPC warps (1, 2 or 4).  Each warp owns QPW queries (32, 16 or 8) --
-// lane j < QPW keeps query j's sorted register list -- and all warps share
-// the CTA's ring of point tiles (128 points, 8 KB, field-major: field f of
-// pair m at float2 f * 64 + m), streamed into shared memory by
-// one-dimensional bulk copies (TMA, no multicast), double-buffered on
-// mbarriers.  Fewer queries per warp give more warps for small query sets.
-//
-// Keys are computed with lanes over POINTS: the warp's lanes form 32 / QPW
-// slots of QPW lanes; in one pass a lane holds one point pair (16 float2
-// registers, pair pass * QPW + lane % QPW of the tile) and every slot takes
-// a different query the tile may matter to, broadcast from a shared table
-// (x, y, z, threshold); one packed f32x2 evaluation gives the lane both of
-// its points' keys, so a warp instruction covers 64 (query, point) pairs.
-// Keys at or below the query's threshold are appended (ballot + popc
-// positions) to the query's candidate queue in shared memory, and after
-// every 64 points of a query each owner lane folds its queue into its
-// list.  A query skips a tile whose lower bound against the query point
-// exceeds its threshold.
-//
-// Selection.  Each list holds the K+1 smallest keys accepted so far in
-// KMAX+1 slots whose lowest KMAX-K slots are -inf sentinels, so the
-// (K+1)-th smallest real key is always the last slot; the threshold is that
-// slot (stale values are still valid: lists only gain smaller keys).
-//
-// Exactness.  The result equals the reference's MinK selection whenever the
-// K+1 smallest keys are pairwise distinct (then the top-K set and its order
-// are unique) and no NaN key falls in MinK's fill phase (points 0..K-1).
-// Every key that leaves a list or is not queued is either strictly above a
-// threshold that is >= the (K+1)-th key, or equal to the threshold it was
-// compared with; the smallest such "equal" key is tracked (tie_key).  A
-// query is flagged for the exact replay kernel when its top-(K+1) holds
-// equal keys or an empty slot, when tie_key <= its (K+1)-th key, or when a
-// fill-phase key is NaN.
-
-// The tile-ring mbarriers of a search CTA.
-template <int WPC, int QPW>
-__device__ __forceinline__ uint64_t* search_barriers(unsigned char* smem) {
-  return reinterpret_cast<uint64_t*>(smem + search_bars_off(WPC, QPW));
-}
-
-// Search + aggregation of one work item.  The mbarriers are initialised by
-// the kernel; uses[buf] counts the phases buffer buf has completed so far
-// (a persistent CTA runs many items on the same barriers).  Returns false
-// when a tile copy timed out (status flagged; the CTA must stop).
-template <int KMAX, int WPC, int QPW>
-__device__ __forceinline__ bool search_item(const SearchParams& a, const SearchItem& it, unsigned char* smem,
-                                            int ntp_cap, uint32_t (&uses)[kTileBufs]) {
-  constexpr int L = KMAX + 1;
-  constexpr int NT = QPW * WPC;         // queries of the item
-  constexpr int NTH = 32 * WPC;         // threads
-  constexpr int H = 32 / QPW;           // lane slots per warp (queries evaluated at once)
-  constexpr int PPT = kTilePoints / 2;  // pairs per tile
-  constexpr int NPASS = PPT / QPW;      // passes per tile (QPW pairs each)
-  constexpr unsigned FULL = 0xffffffffu;
-  constexpr unsigned SLOT_MASK = QPW == 32 ? 0xffffffffu : ((1u << QPW) - 1u);
-  static_assert(QPW == 32 || QPW == 16 || QPW == 8, "queries per warp");
-  static_assert((size_t)NT * L * 12 + NT * 4 <= (size_t)WPC * search_warp_queue_bytes(QPW), "epilogue staging");
-
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const bool owner = lane < QPW;       // lane keeps query `lane` of the warp
-  unsigned char* ring = smem;
-  float* qk = reinterpret_cast<float*>(smem + search_queue_off() + (size_t)warp * search_warp_queue_bytes(QPW));
-  int* qv = reinterpret_cast<int*>(qk + QPW * kQCap);
-  float4* qtab = reinterpret_cast<float4*>(smem + search_qtab_off(WPC, QPW));  // [NT]
-  float4* ctab = reinterpret_cast<float4*>(smem + search_ctab_off(WPC, QPW)) + warp * QPW;  // this warp's
-  int* cidx = reinterpret_cast<int*>(smem + search_ctab_off(WPC, QPW) + (size_t)NT * 16) + warp * QPW;
-  float* tring = reinterpret_cast<float*>(smem + search_tring_off(WPC, QPW));  // [kTileBufs][kTinfoFloats]
-  int* qorig = reinterpret_cast<int*>(smem + search_misc_off(WPC, QPW));       // [NT] original query index (-1: none)
-  float* qbox = reinterpret_cast<float*>(qorig + NT);                          // [WPC][6]
-  uint64_t* full = search_barriers<WPC, QPW>(smem);
-  int* cnt = reinterpret_cast<int*>(full + kTileBufs);               // warps done per buffer
-  volatile int* s_final = reinterpret_cast<volatile int*>(cnt + kTileBufs);  // visit count once stopped
-  volatile int* s_abort = s_final + 1;                               // a wait gave up
-  // region C: per-tile lower bounds (sorted), visit order, visit counter
-  const int NTP = search_tiles_pow2(it.ntile);
-  float* lbk = reinterpret_cast<float*>(smem + search_smem_bytes(WPC, QPW));
-  int* lbt = reinterpret_cast<int*>(lbk + ntp_cap);
-  volatile int* s_nvisit = reinterpret_cast<volatile int*>(lbt + ntp_cap);
-  volatile int* s_ncand = s_nvisit + 1;  // tiles in the visit order (the rest are never needed)
-  // epilogue views of the queue region (after the tile loop)
-  float* out_k = reinterpret_cast<float*>(smem + search_queue_off());
-  int* out_i = reinterpret_cast<int*>(out_k + NT * L);
-  float* out_w = reinterpret_cast<float*>(out_i + NT * L);
-  int* out_f = reinterpret_cast<int*>(out_w + NT * L);
-
-  // the item's queries split evenly over the warps (m <= QPW each: a split
-  // item gives each warp fewer queries and so a shorter critical path)
-  const int m = (it.q1 - it.q0 + WPC - 1) / WPC;
-  const int lq = warp * QPW + lane;         // slot of this (owner) lane's query within the item
-  const int sp = it.q0 + warp * m + lane;   // position in the spatial order
-  bool valid = owner && lane < m && sp < it.q1;
-  int qi = it.perm_q[valid ? sp : it.Q - 1];
-  if ((unsigned)qi >= (unsigned)it.Q) {  // the query order is a permutation: never taken
-    if (valid) atomicOr(a.status, kStatusBadIndex);
-    qi = 0;
-    valid = false;
-  }
-  const int K = it.K, P = it.P;
-  const float qx = it.q[(int64_t)qi * 3 + 0], qy = it.q[(int64_t)qi * 3 + 1], qz = it.q[(int64_t)qi * 3 + 2];
-  const float* recb = it.rec;
-  if (owner) {
-    qorig[lq] = valid ? qi : -1;
-    qtab[lq] = make_float4(qx, qy, qz, valid ? INFINITY : -INFINITY);
-  }
-
-  // ---- seed thresholds (seed_warp): from the plan kernel when it ran,
-  // else computed here from the query's cell
-  const bool seeded = it.tau0 || it.qseed || it.cell_start;
-  if (it.tau0) {  // computed by the plan kernel
-    if (valid) qtab[lq].w = it.tau0[sp];
-    __syncwarp();
-  } else if (seeded) {
-    int my_seed = 0;  // the middle of the query's cell in the sorted points
-    if (valid) {
-      if (it.qseed) {
-        my_seed = it.qseed[sp];
-      } else {
-        const int c = (int)cell_of(qx, qy, qz, it.cbox, it.cbits);
-        my_seed = ((it.cell_start[c] + it.cell_start[c + 1]) >> 1) - it.cell_start[0];
-      }
-    }
-    __syncwarp();
-    seed_warp<KMAX, QPW>(qtab + warp * QPW, my_seed, valid, it.pairs, P, K, lane);
-    __syncwarp();
-  }
-
-  // MinK's fill phase stores points 0..K-1 whatever their key: a NaN there
-  // changes the result in ways only the replay reproduces.  With those
-  // records finite and at most 1e6 in magnitude, and the query too, no key
-  // can overflow or be NaN (|key| < 1.2e32), so the keys are evaluated only
-  // otherwise (lane i checks record i, K <= 32).
-  bool fill_ok = true;
-  if (lane < K) {
-    float r[kRecLen];
-    load_rec(recb + (int64_t)lane * kRecLen, r);
-#pragma unroll
-    for (int m = 0; m < kRecLen - 1; ++m) fill_ok = fill_ok && fabsf(r[m]) <= 1e6f;  // NaN fails
-  }
-  fill_ok = __all_sync(FULL, fill_ok) && fabsf(qx) <= 1e6f && fabsf(qy) <= 1e6f && fabsf(qz) <= 1e6f;
-  bool nan_fill = false;
-  if (owner && !fill_ok)
-    for (int i = 0; i < K; ++i) {
-      const float s = key_rec<float>(qx, qy, qz, recb + (int64_t)i * kRecLen);
-      if (s != s) nan_fill = true;
-    }
-
-  // ---- box of this CTA's queries and the tile visit order
-  {
-    float bx[6] = {qx, qy, qz, qx, qy, qz};
-    if (!valid) {
-      bx[0] = bx[1] = bx[2] = INFINITY;
-      bx[3] = bx[4] = bx[5] = -INFINITY;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        bx[c] = fminf(bx[c], __shfl_xor_sync(FULL, bx[c], o));
-        bx[3 + c] = fmaxf(bx[3 + c], __shfl_xor_sync(FULL, bx[3 + c], o));
-      }
-    }
-    if (lane == 0)
-#pragma unroll
-      for (int c = 0; c < 6; ++c) qbox[warp * 6 + c] = bx[c];
-  }
-  __syncthreads();
-  float bmin[3], bmax[3];
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    bmin[c] = qbox[c];
-    bmax[c] = qbox[3 + c];
-#pragma unroll
-    for (int w = 1; w < WPC; ++w) {
-      bmin[c] = fminf(bmin[c], qbox[w * 6 + c]);
-      bmax[c] = fmaxf(bmax[c], qbox[w * 6 + 3 + c]);
-    }
-  }
-  const float* tinfo_b = it.tinfo;
-  // Seeded queries bound the tiles worth visiting: a tile whose bound
-  // against the CTA's box exceeds every query's seed holds no point below
-  // any threshold the search will ever use.  Only the tiles at or below the
-  // largest seed are sorted (all of them without seeds).
-  float tmax0 = INFINITY;
-  if (seeded) {
-    tmax0 = -INFINITY;
-    for (int i = lane; i < NT; i += 32) tmax0 = fmaxf(tmax0, qtab[i].w);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) tmax0 = fmaxf(tmax0, __shfl_xor_sync(FULL, tmax0, o));
-  }
-  // (bound, tile) ascending, ties by tile, in registers across warp 0's
-  // lanes (shuffle bitonic network); invalid entries carry +inf.
-  auto warp_sort_tiles = [&](float& lb, int& ti) {
-#pragma unroll
-    for (int kk = 2; kk <= 32; kk <<= 1) {
-#pragma unroll
-      for (int j = kk >> 1; j > 0; j >>= 1) {
-        const float ok = __shfl_xor_sync(FULL, lb, j);
-        const int oi = __shfl_xor_sync(FULL, ti, j);
-        const bool up = (lane & kk) == 0;
-        const bool lower = (lane & j) == 0;
-        const bool other_less = ok < lb || (ok == lb && oi < ti);
-        if (lower == up ? other_less : !other_less) {
-          lb = ok;
-          ti = oi;
-        }
-      }
-    }
-  };
-  if (NTP <= 32) {
-    // Up to 32 tiles: warp 0 computes the bounds and sorts them in registers.
-    if (warp == 0) {
-      float lb = INFINITY;
-      int ti = lane;
-      bool keep = false;
-      if (lane < it.ntile) {
-        lb = tile_lower_bound(tinfo_b + lane * kTinfoFloats, bmin, bmax);
-        keep = !(lb > tmax0);
-        lb = keep ? fminf(lb, 3.4e38f) : INFINITY;  // kept tiles sort before the rest
-      }
-      const int nkeep = __popc(__ballot_sync(FULL, keep));
-      warp_sort_tiles(lb, ti);
-      if (lane < NTP) {
-        lbk[lane] = lb;
-        lbt[lane] = ti;
-      }
-      if (lane == 0) *s_ncand = nkeep;
-    }
-    __syncthreads();
-  } else {
-    // Compact the kept tiles (in any order), then sort them: in warp 0's
-    // registers when at most 32, else in shared memory over the next power
-    // of two (padding +inf).
-    if (tid == 0) *s_ncand = 0;
-    __syncthreads();
-    for (int t = tid; t < it.ntile; t += NTH) {
-      const float lb = tile_lower_bound(tinfo_b + (int64_t)t * kTinfoFloats, bmin, bmax);
-      if (!(lb > tmax0)) {
-        const int pos = atomicAdd(const_cast<int*>(s_ncand), 1);
-        lbk[pos] = fminf(lb, 3.4e38f);
-        lbt[pos] = t;
-      }
-    }
-    __syncthreads();
-    const int nkeep = *s_ncand;
-    if (nkeep <= 32) {
-      if (warp == 0) {
-        float lb = lane < nkeep ? lbk[lane] : INFINITY;
-        int ti = lane < nkeep ? lbt[lane] : 0x7fffffff;
-        warp_sort_tiles(lb, ti);
-        if (lane < nkeep) {
-          lbk[lane] = lb;
-          lbt[lane] = ti;
-        }
-      }
-      __syncthreads();
-    } else {
-      const int ns = search_tiles_pow2(nkeep);  // <= NTP
-      for (int t = nkeep + tid; t < ns; t += NTH) {
-        lbk[t] = INFINITY;
-        lbt[t] = 0x7fffffff;
-      }
-      __syncthreads();
-      for (int kk = 2; kk <= ns; kk <<= 1) {  // bitonic sort of (bound, tile) ascending
-        for (int j = kk >> 1; j > 0; j >>= 1) {
-          for (int i = tid; i < ns; i += NTH) {
-            const int ixj = i ^ j;
-            if (ixj > i) {
-              const bool up = (i & kk) == 0;
-              const float ki = lbk[i], kj = lbk[ixj];
-              const int ti = lbt[i], tj = lbt[ixj];
-              if ((ki > kj || (ki == kj && ti > tj)) == up) {
-                lbk[i] = kj;
-                lbk[ixj] = ki;
-                lbt[i] = tj;
-                lbt[ixj] = ti;
-              }
-            }
-          }
-          __syncthreads();
-        }
-      }
-    }
-  }
-
-  float keys[L];
-  int vals[L];
-#pragma unroll
-  for (int s = 0; s < L; ++s) {
-    keys[s] = (s < KMAX - K) ? -INFINITY : INFINITY;
-    vals[s] = -1;
-  }
-  float tau = owner ? qtab[lq].w : -INFINITY, tie_key = INFINITY;  // the seed, +inf or -inf (no query)
-  int my_cnt = 0;  // queued candidates of this lane's query
-  const float qpt[3] = {qx, qy, qz};
-
-  const int ntile = it.ntile;
-  const float* pairs_b = it.pairs;
-  // visit position v reads tile lbt[v] into buffer v % kTileBufs
-  auto issue = [&](int v) {
-    const int buf = v % kTileBufs;
-    mbar_arrive_expect_tx(&full[buf], (uint32_t)kSearchTileBytes + kTinfoBytes);
-    if (v == a.stall_visit) return;  // test hook: this phase never completes
-    bulk_copy_g2s(ring + buf * kSearchTileBytes, pairs_b + (int64_t)lbt[v] * PPT * kPairFloats,
-                  (uint32_t)kSearchTileBytes, &full[buf]);
-    bulk_copy_g2s(tring + buf * kTinfoFloats, tinfo_b + (int64_t)lbt[v] * kTinfoFloats, kTinfoBytes, &full[buf]);
-  };
-  // Issue position v unless its bound exceeds every threshold (the order is
-  // ascending, so nothing after it is needed either).  Decisions are made
-  // one visit at a time, in order (see below), so *s_nvisit == v here.
-  auto decide = [&](int v, float tmax) {
-    if (v >= *s_ncand || *s_nvisit != v) return false;
-    if ((unsigned)lbt[v] >= (unsigned)ntile) {  // real tiles sort first: never taken
-      atomicOr(a.status, kStatusBadIndex);
-      return false;
-    }
-    if (lbk[v] > tmax) return false;
-    *s_nvisit = v + 1;
-    return true;
-  };
-  // No visit v: record the count and complete its buffer's next phase with
-  // a plain arrive, so the warps waiting for visit v wake up and stop.
-  auto stop = [&](int v) {
-    *s_final = v;
-    __threadfence_block();
-    mbar_arrive(&full[v % kTileBufs]);
-  };
-  if (tid == 0) {
-    *s_nvisit = 0;
-    *s_final = 0x7fffffff;
-    *s_abort = 0;
-    for (int b = 0; b < kTileBufs; ++b) cnt[b] = 0;
-    fence_proxy_async_smem();  // the ring was last written by generic stores
-    for (int v = 0; v < kTileBufs; ++v) {
-      if (decide(v, INFINITY)) {
-        issue(v);
-      } else {
-        stop(v);
-        break;
-      }
-    }
-  }
-  __syncthreads();
-
-  // Tile loop without CTA barriers.  Visit t sits in buffer t % kTileBufs;
-  // each warp waits for its copy, evaluates the tile for its queries that
-  // need it, publishes its thresholds and counts itself out of the tile.
-  // The warp that counts out last knows every warp is done with the
-  // buffer: it re-arms the counter and decides (and issues) visit
-  // t + kTileBufs into the same buffer.  A warp does that duty before it
-  // starts its next tile, so the decision for t + kTileBufs - 1 is complete
-  // before any warp can be last for tile t: decisions stay in order.
-  int t = 0;
-  for (;; ++t) {
-    const int buf = t % kTileBufs;
-    const bool ok = mbar_wait_bounded(&full[buf], (uses[buf] + t / kTileBufs) & 1, a.wait_spins);
-    if (!ok) {
-      if (lane == 0) {
-        atomicOr(a.status, kStatusWaitTimeout);
-        *s_abort = 1;
-      }
-      break;
-    }
-    if (*s_abort || t >= *s_final) break;
-    const float2* tile = reinterpret_cast<const float2*>(ring + buf * kSearchTileBytes);
-    // queries of this warp the tile may matter to: bound against the query
-    // point itself not above its threshold
-    const float* tinf = tring + buf * kTinfoFloats;  // the tile's box, then its sub-boxes
-    const float lbq = tile_lower_bound(tinf, qpt, qpt);
-    const unsigned need = __ballot_sync(FULL, valid && !(lbq > tau));
-    if (need) {
-      constexpr int SPP = QPW >= 16 ? QPW / 16 : 1;  // sub-boxes a pass covers (2 QPW points)
-      const int slot = lane / QPW;
-      const unsigned my_mask = SLOT_MASK << (slot * QPW);
-      const unsigned lt_mask = (1u << lane) - 1u;
-#pragma unroll 1
-      for (int pass = 0; pass < NPASS; ++pass) {
-        // The queries this pass matters to: the tile's, less those whose
-        // bound against the pass's sub-box exceeds their threshold,
-        // compacted in lane order (round r slot h takes entry r * H + h).
-        // Owner lanes publish their entry and keep its rank (refreshed
-        // thresholds go there too).
-        const int sb0 = (2 * pass * QPW) / 32;
-        float lbp = INFINITY;
-#pragma unroll
-        for (int u = 0; u < SPP; ++u) lbp = fminf(lbp, tile_lower_bound(tinf + 8 * (1 + sb0 + u), qpt, qpt));
-        const unsigned need_p = __ballot_sync(FULL, ((need >> lane) & 1u) && !(lbp > tau));
-        const int n_need = __popc(need_p);
-        const int my_rank = ((need_p >> lane) & 1u) ? __popc(need_p & lt_mask) : -1;
-        if (need_p) {
-          const int R = (n_need + H - 1) / H;  // rounds of this pass
-          const int my_round = my_rank >= 0 ? my_rank / H : -1;
-          const unsigned my_slot_mask = SLOT_MASK << ((my_rank >= 0 ? my_rank % H : 0) * QPW);
-          __syncwarp();  // the previous pass's readers are done with the table
-          if (my_rank >= 0) {
-            ctab[my_rank] = make_float4(qx, qy, qz, tau);
-            cidx[my_rank] = lane;
-          }
-          __syncwarp();
-          float2 pr[kRecLen];
-          const int pidx = pass * QPW + (lane & (QPW - 1));
-#pragma unroll
-          for (int f = 0; f < kRecLen; ++f) pr[f] = tile[f * PPT + pidx];
-          const int i0 = __float_as_int(pr[kRecPad].x), i1 = __float_as_int(pr[kRecPad].y);
-#pragma unroll 1
-          for (int r0 = 0; r0 < R; r0 += 2) {
-            // two rounds per iteration (independent key evaluations in flight)
-            int jr[2];
-            float4 qr[2];
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-              const int e = (r0 + u) * H + slot;
-              jr[u] = e < n_need ? cidx[e] : -1;
-              qr[u] = ctab[e < n_need ? e : 0];
-            }
-            float2 sr[2];
-#pragma unroll
-            for (int u = 0; u < 2; ++u)
-              sr[u] = key_pair(make_float2(qr[u].x, qr[u].x), make_float2(qr[u].y, qr[u].y),
-                               make_float2(qr[u].z, qr[u].z), pr);
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-              if (u == 1 && r0 + 1 >= R) break;  // warp-uniform: no round 1
-              const int j = jr[u];
-              const float2 s2 = sr[u];
-              const bool c0 = j >= 0 && s2.x <= qr[u].w, c1 = j >= 0 && s2.y <= qr[u].w;
-              const unsigned b0 = __ballot_sync(FULL, c0), b1 = __ballot_sync(FULL, c1);
-              if (b0 | b1) {
-                const int n = __popc(b0 & my_mask) + __popc(b1 & my_mask);
-                int c = __shfl_sync(FULL, my_cnt, j >= 0 ? j : 0);
-                if (__any_sync(FULL, j >= 0 && c + n > kQCap)) {  // a queue would overflow: fold every queue first
-                  __syncwarp();
-                  drain_queue<L>(keys, vals, tie_key, tau, my_cnt, qk, qv, lane);
-                  my_cnt = 0;
-                  if (owner) qtab[lq].w = tau;
-                  if (my_rank >= 0) ctab[my_rank].w = tau;
-                  __syncwarp();
-                  c = 0;
-                }
-                if (c0) {
-                  const int e = queue_slot(j, c + __popc(b0 & my_mask & lt_mask));
-                  qk[e] = s2.x;
-                  qv[e] = i0;
-                }
-                if (c1) {
-                  const int e = queue_slot(j, c + __popc(b0 & my_mask) + __popc(b1 & my_mask & lt_mask));
-                  qk[e] = s2.y;
-                  qv[e] = i1;
-                }
-                if (my_round == r0 + u) my_cnt += __popc(b0 & my_slot_mask) + __popc(b1 & my_slot_mask);
-              }
-            }
-          }
-        }
-        if ((pass + 1) % H == 0) {  // every query met at most 64 more points since the last fold
-          __syncwarp();
-          drain_queue<L>(keys, vals, tie_key, tau, my_cnt, qk, qv, lane);
-          my_cnt = 0;
-          if (owner) qtab[lq].w = tau;
-          if (my_rank >= 0) ctab[my_rank].w = tau;
-          __syncwarp();
-        }
-      }
-    }
-    // count this warp out of the tile (release: its reads of the buffer and
-    // its threshold writes come first)
-    __syncwarp();
-    int last = 0;
-    if (lane == 0) {
-      __threadfence_block();
-      last = atomicAdd(&cnt[buf], 1) == WPC - 1;
-      if (last) __threadfence_block();
-    }
-    last = __shfl_sync(FULL, last, 0);
-    if (last) {
-      // every warp is done with this buffer: re-arm its counter, then decide
-      // visit t + kTileBufs unless a stop was made; a tile is needed while
-      // its bound is below some query's threshold
-      float tmax = -INFINITY;
-      for (int i = lane; i < NT; i += 32) tmax = fmaxf(tmax, qtab[i].w);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) tmax = fmaxf(tmax, __shfl_xor_sync(FULL, tmax, o));
-      if (lane == 0) {
-        cnt[buf] = 0;
-        if (*s_final == 0x7fffffff && !*s_abort) {
-          if (decide(t + kTileBufs, tmax)) {
-            fence_proxy_async_smem();
-            issue(t + kTileBufs);
-          } else {
-            stop(t + kTileBufs);
-          }
-        }
-      }
-    }
-  }
-  // Every warp has left the loop once all meet here; no copy is in flight
-  // then (each issued visit was waited for by every warp), unless a wait
-  // gave up.
-  __syncthreads();
-  if (*s_abort) {
-    if (tid == 0) {
-      // best effort: let the copies of the last issued visits land
-      for (int v = *s_nvisit - kTileBufs; v < *s_nvisit; ++v)
-        if (v >= 0) mbar_wait_bounded(&full[v % kTileBufs], (uses[v % kTileBufs] + v / kTileBufs) & 1, a.wait_spins);
-    }
-    return false;
-  }
-  {
-    const int n = t + 1;  // phases waited on: visits 0..t (t = the stop visit)
-#pragma unroll
-    for (int b = 0; b < kTileBufs; ++b) uses[b] += n > b ? (n - b + kTileBufs - 1) / kTileBufs : 0;
-  }
-
-  // ---- flags and staging; the queue region is free (every drain ended
-  // before the last barrier)
-  if (owner) {
-#pragma unroll
-    for (int s = 0; s < L; ++s) {
-      const int j = s - (KMAX - K);
-      if (j >= 0) {
-        out_k[lq * L + j] = keys[s];
-        out_i[lq * L + j] = vals[s];
-      }
-    }
-
-    const int nneed = (P > K) ? K + 1 : K;
-    bool fl = nan_fill, bad = false;
-    for (int j = 0; j < nneed; ++j) {
-      const int idx = out_i[lq * L + j];
-      if (idx < 0) fl = true;
-      if (idx >= P) bad = true;  // tiles carry indices of their own cloud: never taken
-    }
-    if (bad && valid) atomicOr(a.status, kStatusBadIndex);
-    for (int j = 0; j + 1 < nneed; ++j)
-      if (out_k[lq * L + j] == out_k[lq * L + j + 1]) fl = true;
-    const float m = (P > K) ? out_k[lq * L + K] : INFINITY;
-    if (tie_key <= m) fl = true;
-    for (int j = 0; j < K; ++j) out_w[lq * L + j] = weight_of(out_k[lq * L + j]);
-    out_f[lq] = (fl || bad || !valid) ? 1 : 0;
-    if (valid && fl && !bad) {
-      const int pos = atomicAdd(a.flag_count, 1);
-      a.flag_list[pos] = (int)(it.row0 + qi);
-    }
-  }
-  __syncthreads();
-
-  // ---- epilogue: dists / idxs / w_out, then f_out = sum_k w_k f[idx_k]
-  // accumulated in k order with fma, 128-bit gathers of f rows.  Rows go to
-  // the queries' original positions.
-  for (int x = tid; x < NT * K; x += NTH) {
-    const int l = x / K, k = x - l * K;
-    if (out_f[l]) continue;
-    const int64_t e = (int64_t)qorig[l] * K + k;
-    const int idx = out_i[l * L + k];
-    it.dists[e] = out_k[l * L + k];
-    it.idxs[e] = (int64_t)idx;
-    it.w_out[e] = out_w[l * L + k];
-    if (it.adj_count) atomicAdd(&it.adj_count[idx], 1);  // idx is in [0, P): unflagged
-  }
-  const int F = a.F;
-  const float* fb = it.f;
-  if (a.vec4) {
-    const int C4 = F >> 2;
-    for (int x = tid; x < NT * C4; x += NTH) {
-      const int l = x / C4, c = x - l * C4;
-      if (out_f[l]) continue;
-      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-      // sixteen rows in flight, summed in k order
-      constexpr int RB = 16;
-      for (int k0 = 0; k0 < K; k0 += RB) {
-        float4 v[RB];
-        float w[RB];
-#pragma unroll
-        for (int j = 0; j < RB; ++j) {
-          const bool in = k0 + j < K;
-          const int idx = in ? out_i[l * L + k0 + j] : 0;
-          w[j] = in ? out_w[l * L + k0 + j] : 0.f;
-          v[j] = in ? __ldg(reinterpret_cast<const float4*>(fb + (int64_t)idx * F) + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-#pragma unroll
-        for (int j = 0; j < RB; ++j) {
-          if (k0 + j < K) {
-            acc.x = __fmaf_rn(v[j].x, w[j], acc.x);
-            acc.y = __fmaf_rn(v[j].y, w[j], acc.y);
-            acc.z = __fmaf_rn(v[j].z, w[j], acc.z);
-            acc.w = __fmaf_rn(v[j].w, w[j], acc.w);
-          }
-        }
-      }
-      reinterpret_cast<float4*>(it.f_out + (int64_t)qorig[l] * F)[c] = acc;
-    }
-  } else {
-    for (int x = tid; x < NT * F; x += NTH) {
-      const int l = x / F, c = x - l * F;
-      if (out_f[l]) continue;
-      float acc = 0.f;
-      for (int k = 0; k < K; ++k)
-        acc = __fmaf_rn(__ldg(fb + (int64_t)out_i[l * L + k] * F + c), out_w[l * L + k], acc);
-      it.f_out[(int64_t)qorig[l] * F + c] = acc;
-    }
-  }
-  return true;
-}
-
-template <int KMAX, int WPC, int QPW>
-__global__ void __launch_bounds__(32 * WPC) search_f32_kernel(SearchParams a) {
-  extern __shared__ __align__(128) unsigned char smem[];
-  uint64_t* full = search_barriers<WPC, QPW>(smem);
-  if (threadIdx.x == 0) {
-    for (int b = 0; b < kTileBufs; ++b) mbar_init(&full[b], 1);
-    fence_mbar_init();
-  }
-  __syncthreads();
-  // the plan kernel's item (batch element, sorted query range), else block
-  // (blockIdx.x, blockIdx.y) of WPC * QPW queries
-  int64_t b = blockIdx.y;
-  int q0 = blockIdx.x * (WPC * QPW), q1 = min(q0 + WPC * QPW, a.Q);
-  if (a.items) {
-    const int4 itm = a.items[blockIdx.x];
-    b = itm.x;
-    q0 = itm.y;
-    q1 = itm.z;
-  }
-  SearchItem it;
-  it.q = a.q + b * a.Q * 3;
-  it.perm_q = a.perm_q + b * a.Q;
-  it.rec = a.rec + b * a.P * kRecLen;
-  it.pairs = a.pairs + b * (a.P_pad / 2) * kPairFloats;
-  it.tinfo = a.tinfo + b * a.ntile * kTinfoFloats;
-  it.f = a.f + b * a.P * a.F;
-  it.f_out = a.f_out + b * a.Q * a.F;
-  it.w_out = a.w_out + b * a.Q * a.K;
-  it.dists = a.dists + b * a.Q * a.K;
-  it.idxs = a.idxs + b * a.Q * a.K;
-  it.row0 = b * a.Q;
-  it.adj_count = a.adj_count ? a.adj_count + b * a.P : nullptr;
-  it.qseed = a.qseed ? a.qseed + b * a.Q : nullptr;
-  it.cell_start = nullptr;
-  it.cbox = nullptr;
-  it.cbits = 0;
-  it.Q = a.Q;
-  it.P = a.P;
-  it.K = a.K;
-  it.ntile = a.ntile;
-  it.q0 = q0;
-  it.q1 = q1;
-  it.tau0 = a.items ? a.tau0 + b * a.Q : nullptr;
-  uint32_t uses[kTileBufs] = {};
-  search_item<KMAX, WPC, QPW>(a, it, smem, search_tiles_pow2(a.ntile), uses);
-}
-
 // ------------------------------------------------------------ search plan
 //
 // search_plan_kernel, one CTA per block of qpc sorted queries (grid (nb, B),
@@ -1233,87 +588,6 @@ __global__ void __launch_bounds__(kPlanItemsThreads) search_items_kernel(SearchP
   }
 }
 
-// Ragged search: a persistent CTA takes work items in order from a counter
-// until the segment table's items run out.  Item i belongs to the last
-// segment whose item_off <= i; its queries are that segment's sorted
-// positions [(i - item_off) * WPC * QPW, ...).  Each item runs with the
-// register list of its own segment's K (8, 16 or 32 slots + 1), up to the
-// launch's KMAX.
-template <int KMAX, int WPC, int QPW>
-__global__ void __launch_bounds__(32 * WPC) search_ragged_kernel(SearchParams a) {
-  extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ int s_item;
-  if (*a.status) return;  // the table failed validation
-  uint64_t* full = search_barriers<WPC, QPW>(smem);
-  if (threadIdx.x == 0) {
-    for (int b = 0; b < kTileBufs; ++b) mbar_init(&full[b], 1);
-    fence_mbar_init();
-  }
-  __syncthreads();
-  const SegHeader* sh = static_cast<const SegHeader*>(a.segs);
-  const SegDesc* sd = seg_descs(a.segs);
-  const CloudSetHeader* ch = reinterpret_cast<const CloudSetHeader*>(a.cs);
-  const CloudDesc* cd = cloud_descs(a.cs);
-  const float* crec = reinterpret_cast<const float*>(a.cs + ch->rec_off);
-  const float* cpairs = reinterpret_cast<const float*>(a.cs + ch->pairs_off);
-  const float* ctinfo = reinterpret_cast<const float*>(a.cs + ch->tinfo_off);
-  const float* cbnd = reinterpret_cast<const float*>(a.cs + ch->bnd_off);
-  const int* ccell = reinterpret_cast<const int*>(a.cs + ch->celloff_off);
-  const int nseg = sh->nseg, n_items = sh->n_items;
-  const int ntp_cap = search_tiles_pow2(a.ntile);
-  constexpr int QPC = WPC * QPW;
-  uint32_t uses[kTileBufs] = {};
-  for (;;) {
-    if (threadIdx.x == 0) s_item = atomicAdd(a.item_counter, 1);
-    __syncthreads();
-    const int item = s_item;
-    if (item >= n_items) break;
-    if (item < 0) {  // the counter starts at 0 and only grows: never taken
-      if (threadIdx.x == 0) atomicOr(a.status, kStatusBadIndex);
-      break;
-    }
-    const SegDesc g = sd[seg_of_item(sd, nseg, item)];
-    const CloudDesc c = cd[g.cloud];
-    if (g.K < 1 || g.K > KMAX || g.K > c.P || c.ntile > a.ntile || sh->qpc != QPC) {
-      if (threadIdx.x == 0) atomicOr(a.status, kStatusBadTable);
-    } else {
-      SearchItem it;
-      it.q = a.q + g.q_off * 3;
-      it.perm_q = a.perm_q + g.q_off;
-      it.rec = crec + c.p_off * kRecLen;
-      it.pairs = cpairs + c.tile_off * (kTilePoints / 2) * kPairFloats;
-      it.tinfo = ctinfo + c.tile_off * kTinfoFloats;
-      it.f = a.f + c.p_off * a.F;
-      it.f_out = a.f_out + g.q_off * a.F;
-      it.w_out = a.w_out + g.e_off;
-      it.dists = a.dists + g.e_off;
-      it.idxs = a.idxs + g.e_off;
-      it.row0 = g.q_off;
-      it.adj_count = nullptr;
-      it.qseed = nullptr;
-      it.tau0 = nullptr;
-      it.cell_start = ccell + c.cell_off;
-      it.cbox = cbnd + (int64_t)g.cloud * 8;
-      it.cbits = c.bits;
-      it.Q = g.Q;
-      it.P = c.P;
-      it.K = g.K;
-      it.ntile = c.ntile;
-      it.q0 = (item - g.item_off) * QPC;
-      it.q1 = min(it.q0 + QPC, g.Q);
-      bool ok;
-      if (KMAX > 8 && g.K <= 8)
-        ok = search_item<8, WPC, QPW>(a, it, smem, ntp_cap, uses);
-      else if (KMAX > 16 && g.K <= 16)
-        ok = search_item<(KMAX > 16 ? 16 : KMAX), WPC, QPW>(a, it, smem, ntp_cap, uses);
-      else
-        ok = search_item<KMAX, WPC, QPW>(a, it, smem, ntp_cap, uses);
-      if (!ok) break;
-    }
-    __syncthreads();  // the next item reuses shared memory (and s_item)
-  }
-}
-
 // ------------------------------------------------------------------ host
 
 int num_sms(int dev) {
@@ -1329,145 +603,22 @@ int num_sms(int dev) {
 
 namespace {
 
-template <int KMAX, int WPC, int QPW>
-int launch_search_t(const SearchParams& a, cudaStream_t st) {
-  const size_t smem = search_smem_bytes(WPC, QPW) + search_region_c_bytes(a.ntile);
-  if (smem > 227 * 1024) return KNNAG_ERR_TOO_LARGE;
-  static int attr_set[64] = {0};  // largest size already allowed, per device
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev >= 0 && dev < 64 && attr_set[dev] < (int)smem) {
-    if (cudaFuncSetAttribute(search_f32_kernel<KMAX, WPC, QPW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem) != cudaSuccess)
-      return KNNAG_ERR_CUDA;
-    attr_set[dev] = (int)smem;
-  }
-  constexpr int QPC = WPC * QPW;
-  const int nb = (a.Q + QPC - 1) / QPC;
-  dim3 grid(nb, a.B);
-  const int64_t nbt = (int64_t)nb * a.B;
-  bool plan = false;
-  if (a.items && nbt <= kPlanMaxBlocks) {
-    // the plan pays when the blocks take more than one wave of the search
-    static int occ_smem[64], occ_val[64];
-    int occ = 0;
-    if (dev >= 0 && dev < 64 && occ_smem[dev] == (int)smem) {
-      occ = occ_val[dev];
-    } else {
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, search_f32_kernel<KMAX, WPC, QPW>, 32 * WPC, smem) !=
-          cudaSuccess)
-        return KNNAG_ERR_CUDA;
-      if (dev >= 0 && dev < 64) {
-        occ_smem[dev] = (int)smem;
-        occ_val[dev] = occ;
-      }
-    }
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    plan = nbt > (int64_t)occ * sms;
-  }
-  if (plan) {
-    grid = dim3((unsigned)nbt, 1);
-    static int items_smem[64];
-    if (dev >= 0 && dev < 64 && items_smem[dev] < kPlanMaxBlocks * 4) {
-      if (cudaFuncSetAttribute(search_items_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               kPlanMaxBlocks * 4) != cudaSuccess)
-        return KNNAG_ERR_CUDA;
-      items_smem[dev] = kPlanMaxBlocks * 4;
-    }
-  }
-  SearchParams ap = a;
-  if (!plan) ap.items = nullptr;  // one wave (or too many blocks to plan): the plain grid
-  profile_begin(st);  // the plan does the seed work of the search: timed with it
-  if (plan) {
-    search_plan_kernel<KMAX><<<dim3(nb, a.B), 32 * ((QPC + kPlanQPW - 1) / kPlanQPW), 0, st>>>(ap, QPC, nb);
-    search_items_kernel<<<1, kPlanItemsThreads, (size_t)nbt * 4, st>>>(ap, nb, QPC);
-    note_launches(2);
-  }
-  search_f32_kernel<KMAX, WPC, QPW><<<grid, 32 * WPC, smem, st>>>(ap);
-  profile_end(st);
-  note_launches(1);
-  return cudaGetLastError() == cudaSuccess ? KNNAG_OK : KNNAG_ERR_CUDA;
+// Launch shape of the one-warp-per-query search (see search_qpw): a unit of
+// four queries per warp, fewer when that would leave the chip's 24 warps per
+// SM without work.
+int choose_warp_shape(int B, int Q, int dev) {
+  const int64_t n = (int64_t)B * Q, slots = (int64_t)num_sms(dev) * 24;
+  return n <= slots ? 64 : n <= 2 * slots ? 32 : 4;
 }
 
-template <int KMAX, int WPC, int QPW>
-int launch_search_ragged_t(const SearchParams& a, int64_t cap_items, cudaStream_t st) {
-  const size_t smem = search_smem_bytes(WPC, QPW) + search_region_c_bytes(a.ntile);
-  if (smem > 227 * 1024) return KNNAG_ERR_TOO_LARGE;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  static int attr_set[64] = {0};
-  if (dev >= 0 && dev < 64 && attr_set[dev] < (int)smem) {
-    if (cudaFuncSetAttribute(search_ragged_kernel<KMAX, WPC, QPW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem) != cudaSuccess)
-      return KNNAG_ERR_CUDA;
-    attr_set[dev] = (int)smem;
-  }
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, search_ragged_kernel<KMAX, WPC, QPW>, 32 * WPC, smem) !=
-          cudaSuccess ||
-      per_sm < 1)
-    per_sm = 1;
-  int64_t grid = (int64_t)num_sms(dev) * per_sm;
-  if (grid > cap_items) grid = cap_items;
-  if (grid < 1) grid = 1;
-  profile_begin(st);
-  search_ragged_kernel<KMAX, WPC, QPW><<<(unsigned)grid, 32 * WPC, smem, st>>>(a);
-  profile_end(st);
-  note_launches(1);
-  return cudaGetLastError() == cudaSuccess ? KNNAG_OK : KNNAG_ERR_CUDA;
-}
-
-// launch-shape code s -> (warps per CTA, queries per warp)
-template <int KMAX>
-int launch_search_ragged_k(const SearchParams& a, int s, int64_t cap_items, cudaStream_t st) {
-  switch (s) {
-    case 1: return launch_search_ragged_t<KMAX, 4, 32>(a, cap_items, st);
-    case 2: return launch_search_ragged_t<KMAX, 2, 32>(a, cap_items, st);
-    case 8: return launch_search_ragged_t<KMAX, 2, 16>(a, cap_items, st);
-    case 16: return launch_search_ragged_t<KMAX, 4, 8>(a, cap_items, st);
-    case 32: return launch_search_ragged_t<KMAX, 1, 16>(a, cap_items, st);
-    case 64: return launch_search_ragged_t<KMAX, 1, 8>(a, cap_items, st);
-    default: return launch_search_ragged_t<KMAX, 1, 32>(a, cap_items, st);
-  }
-}
-
-template <int KMAX>
-int launch_search_k(const SearchParams& a, int s, cudaStream_t st) {
-  switch (s) {
-    case 1: return launch_search_t<KMAX, 4, 32>(a, st);
-    case 2: return launch_search_t<KMAX, 2, 32>(a, st);
-    case 8: return launch_search_t<KMAX, 2, 16>(a, st);
-    case 16: return launch_search_t<KMAX, 4, 8>(a, st);
-    case 32: return launch_search_t<KMAX, 1, 16>(a, st);
-    case 64: return launch_search_t<KMAX, 1, 8>(a, st);
-    default: return launch_search_t<KMAX, 1, 32>(a, st);
-  }
-}
-
-// Launch shape of the CUDA-core uniform search, by the warps the query set
-// gives at 32 queries per warp: many (large query sets) -> 128-query CTAs of
-// 4 warps; few -> fewer queries per warp, so that there are more warps to
-// hide the latency of each one's dependent work.
-int choose_cuda_core_splits(int B, int Q, int dev) {
-  const int64_t warps32 = ((int64_t)B * Q + 31) / 32;
-  const int64_t sms = num_sms(dev);
-  if (warps32 >= 16 * sms) return 1;
-  if (warps32 >= 4 * sms) return 8;
-  return 16;
-}
-
-// The process-wide setting when one is made; else the tensor-core filtered
-// search for grids of more than 8 waves of its 128-query CTAs (two per SM),
-// where it measured faster (B200, one cloud of 131072 points and 524288
-// queries: 2.80 against 2.95 ms), and the CUDA-core search below that (the
-// table workload, B = 2, Q = 12288, P = 4096: 0.148 against 0.113 ms).
-int choose_splits(int B, int Q, int dev) {
+// The process-wide setting when one is made, else by size.  While the test
+// hook of the bounded waits is armed the tensor-core search runs: it is the
+// one that waits (on its tile copies).
+int choose_splits(int B, int Q, int dev, bool stalled) {
   const int forced = search_splits_setting();
   if (search_setting_ok(forced)) return forced;
-  const int64_t ctas = (int64_t)B * ((Q + 127) / 128);
-  if (ctas > 16 * (int64_t)num_sms(dev)) return kShapeTensorFilter;
-  return choose_cuda_core_splits(B, Q, dev);
+  if (stalled) return kShapeTensorFilter;
+  return choose_warp_shape(B, Q, dev);
 }
 
 inline unsigned grid_for(int64_t n, int threads, int dev) {
@@ -1539,7 +690,7 @@ int launch_exact(const ExactParams<T>& a, cudaStream_t st) {
 template int launch_exact<float>(const ExactParams<float>&, cudaStream_t);
 template int launch_exact<double>(const ExactParams<double>&, cudaStream_t);
 
-FwdLayout fwd_layout(int B, int Q, int P, int K, int dtype, bool own_rec) {
+FwdLayout fwd_layout(int B, int Q, int P, int K, int dtype, bool own_rec, bool indexed) {
   FwdLayout L{};
   const size_t esz = dtype == KNNAG_F64 ? 8 : 4;
   size_t off = 0;
@@ -1551,13 +702,14 @@ FwdLayout fwd_layout(int B, int Q, int P, int K, int dtype, bool own_rec) {
   if (own_rec) off += align256((size_t)B * P * kRecLen * esz);
   L.P_pad = (int)round_up(P, kTilePoints);
   L.pairs = L.bounds = L.cell_count = L.cell_offset = L.perm_p = L.perm_q = L.tinfo = L.qseed = L.tau0 =
-      L.plan_est = L.items = L.tcops = L.tcinfo = off;
+      L.plan_est = L.items = L.tcops = L.tcinfo = L.tbox = L.sbox = L.gbox = L.pf = L.qf = off;
   L.bits = 0;
-  if (dtype == KNNAG_F32 && K <= 32) {
-    L.bits = spatial_bits(P);
+  if (indexed) {
+    L.bits = point_bits(P);
     const size_t cells = (size_t)1 << (3 * L.bits);
+    const size_t ntiles = (size_t)B * (L.P_pad / kTilePoints);
     L.pairs = off;
-    off += align256((size_t)B * L.P_pad * kRecLen * 4);
+    off += align256((size_t)B * L.P_pad * kRecLen * esz);
     L.bounds = off;  // per element kBoundParts partial boxes
     off += align256((size_t)B * kBoundParts * 8 * 4);
     // point and query cells of each batch element, sorted together
@@ -1569,34 +721,58 @@ FwdLayout fwd_layout(int B, int Q, int P, int K, int dtype, bool own_rec) {
     L.perm_q = off + (size_t)B * P * 4;
     off += align256((size_t)B * P * 4 + (size_t)B * Q * 4);
     L.tinfo = off;
-    off += align256((size_t)B * (L.P_pad / kTilePoints) * kTinfoBytes);
+    off += align256(ntiles * kTinfoBytes);
+    L.tbox = off;
+    off += align256(ntiles * 7 * 4);
+    L.sbox = off;
+    off += align256(ntiles * 8 * 16);
+    L.gbox = off;
+    off += align256((size_t)B * ((L.P_pad / kTilePoints + 31) / 32) * 7 * 4);
     L.qseed = off;
     off += align256((size_t)B * Q * 4);
-    // search plan: seed thresholds, per-block estimates, CTA items (for the
-    // smallest blocks, 8 queries)
-    const size_t nb_max = (size_t)B * ((Q + 7) / 8);
-    L.tau0 = off;
-    off += align256((size_t)B * Q * 4);
-    L.plan_est = off;
-    off += align256(nb_max * 4);
-    L.items = off;
-    off += align256(nb_max * 16);
-    // tensor-core filter: B operands and bound terms of every tile
-    const size_t ntiles = (size_t)B * (L.P_pad / kTilePoints);
-    L.tcops = off;
-    off += align256(ntiles * kTcOpsBytes);
-    L.tcinfo = off;
-    off += align256(ntiles * kTcInfoBytes);
+    if (dtype == KNNAG_F64) {
+      L.pf = off;
+      off += align256((size_t)B * P * 3 * 4);
+      L.qf = off;
+      off += align256((size_t)B * Q * 3 * 4);
+    } else if (K <= 32) {
+      // search plan of the tensor-core search: seed thresholds, per-block
+      // estimates, CTA items
+      const size_t nb_max = (size_t)B * ((Q + 7) / 8);
+      L.tau0 = off;
+      off += align256((size_t)B * Q * 4);
+      L.plan_est = off;
+      off += align256(nb_max * 4);
+      L.items = off;
+      off += align256(nb_max * 16);
+      // tensor-core filter: B operands and bound terms of every tile
+      L.tcops = off;
+      off += align256(ntiles * kTcOpsBytes);
+      L.tcinfo = off;
+      off += align256(ntiles * kTcInfoBytes);
+    }
   }
   L.total = off;
   return L;
 }
 
-int launch_pack_points_bounded(const float* p, const float* sigma, const float* R, int B, int P, float* rec,
-                               float* parts, cudaStream_t st, int* zero_words, int n_zero, int* zero_rows,
-                               int* zero_cells, int64_t n_cells) {
-  pack_points_bounded_kernel<<<dim3(kBoundParts, B), 256, 0, st>>>(p, sigma, R, P, rec, parts, zero_words, n_zero,
-                                                                   zero_rows, zero_cells, n_cells);
+FwdLayout fwd_layout_in(int B, int Q, int P, int K, int dtype, bool own_rec, size_t bytes, bool* indexed) {
+  *indexed = forward_indexed(B, P, K, dtype);
+  FwdLayout L = fwd_layout(B, Q, P, K, dtype, own_rec, *indexed);
+  if (*indexed && L.total > bytes && (dtype == KNNAG_F64 || K > 32)) {
+    *indexed = false;
+    L = fwd_layout(B, Q, P, K, dtype, own_rec, false);
+  }
+  return L;
+}
+
+template <typename T>
+int launch_pack_points_bounded(const T* p, const T* sigma, const T* R, const T* q, int B, int Q, int P, T* rec,
+                               float* parts, float* pf, float* qf, cudaStream_t st, int* zero_words, int n_zero,
+                               int* zero_rows, int* zero_cells, int64_t n_cells) {
+  pack_points_bounded_kernel<T><<<dim3(kBoundParts, B), 256, 0, st>>>(p, sigma, R, q, Q, P, rec, parts, pf, qf,
+                                                                      zero_words, n_zero, zero_rows, zero_cells,
+                                                                      n_cells);
   note_launches(1);
   return cudaGetLastError() == cudaSuccess ? KNNAG_OK : KNNAG_ERR_CUDA;
 }
@@ -1625,102 +801,149 @@ static int forward_exact_all(const T* q, const T* rec, const T* f, int B, int Q,
   return launch_exact<T>(e, st);
 }
 
-int forward_impl(const void* q, const void* p, const void* f, const void* sigma, const void* R, int B, int Q,
-                 int P, int F, int K, int dtype, void* f_out, void* w_out, void* dists, int64_t* idxs,
-                 void* points, void* workspace, cudaStream_t st, void* adjacency) {
-  NvtxRange range("knnag:forward");
-  int* adj_count = adjacency ? reinterpret_cast<int*>(static_cast<char*>(adjacency) + adj_layout(B, Q, P, K).cursor)
-                             : nullptr;
-  const bool own_rec = points == nullptr;
-  const FwdLayout L = fwd_layout(B, Q, P, K, dtype, own_rec);
-  char* ws = static_cast<char*>(workspace);
+// The forward through the spatial index: pack, sort, search, exact replay of
+// the flagged queries.
+template <typename T>
+static int forward_indexed_t(const T* q, const T* p, const T* f, const T* sigma, const T* R, int B, int Q, int P, int F,
+                             int K, T* f_out, T* w_out, T* dists, int64_t* idxs, T* rec, char* ws, const FwdLayout& L,
+                             int* adj_count, cudaStream_t st) {
   int* status = reinterpret_cast<int*>(ws + L.status);
   int* flag_count = status + 1;
   int* flag_list = reinterpret_cast<int*>(ws + L.flag_list);
-  void* rec = own_rec ? (void*)(ws + L.rec) : points;
+  float* pf = reinterpret_cast<float*>(ws + L.pf);
+  float* qf = reinterpret_cast<float*>(ws + L.qf);
+  const int ntile = L.P_pad / kTilePoints;
   int rc;
-  const bool search_path = dtype == KNNAG_F32 && K <= 32;
   {
     NvtxRange r("knnag:pack_points");
-    // also zeroes the status words and the adjacency's entry counts; on
-    // the search path also the cell counts, and it bounds the points
-    if (search_path)
-      // cell counts and offsets (the offsets are the scatter's cursors when
-      // the scan is folded into it) are zeroed, padding between them included
-      rc = launch_pack_points_bounded((const float*)p, (const float*)sigma, (const float*)R, B, P, (float*)rec,
-                                      reinterpret_cast<float*>(ws + L.bounds), st, status, 2, adj_count,
-                                      reinterpret_cast<int*>(ws + L.cell_count),
-                                      (int64_t)(L.cell_offset - L.cell_count) / 4 + (2 * (int64_t)B << (3 * L.bits)) + 1);
-    else
-      rc = launch_pack_points(p, sigma, R, B, P, dtype, rec, st, status, 2, adj_count);
+    // also zeroes the status words and the adjacency's entry counts, and
+    // bounds the points; cell counts and offsets (the offsets are the
+    // scatter's cursors when the scan is folded into it) are zeroed, padding
+    // between them included
+    rc = launch_pack_points_bounded<T>(p, sigma, R, q, B, Q, P, rec, reinterpret_cast<float*>(ws + L.bounds), pf, qf, st,
+                                       status, 2, adj_count, reinterpret_cast<int*>(ws + L.cell_count),
+                                       (int64_t)(L.cell_offset - L.cell_count) / 4 + (2 * (int64_t)B << (3 * L.bits)) + 1);
   }
   if (rc) return rc;
-  if (dtype == KNNAG_F64)
-    return forward_exact_all<double>((const double*)q, (const double*)rec, (const double*)f, B, Q, P, F, K,
-                                     (double*)f_out, (double*)w_out, (double*)dists, idxs, adj_count, st);
-  if (K > 32)
-    return forward_exact_all<float>((const float*)q, (const float*)rec, (const float*)f, B, Q, P, F, K,
-                                    (float*)f_out, (float*)w_out, (float*)dists, idxs, adj_count, st);
+  if (ntile > kSearchMaxTiles) return KNNAG_ERR_TOO_LARGE;
   int dev = 0;
   cudaGetDevice(&dev);
-  float* pairs = reinterpret_cast<float*>(ws + L.pairs);
-  int G = choose_splits(B, Q, dev);
-  if (G == kShapeTensorFilter && !search_tc_fits(L.P_pad / kTilePoints)) G = choose_cuda_core_splits(B, Q, dev);
+  SearchParams sp{};
+  apply_search_debug(sp);
+  int G = choose_warp_shape(B, Q, dev);
+  if (sizeof(T) == 4 && K <= 32) G = choose_splits(B, Q, dev, sp.stall_visit >= 0);
+  if (G == kShapeTensorFilter && !search_tc_fits(ntile)) G = choose_warp_shape(B, Q, dev);
   {
     NvtxRange r("knnag:spatial_index");
-    rc = launch_spatial_index((const float*)q, (const float*)rec, B, Q, P, L.P_pad, ws, L, st,
-                              G == kShapeTensorFilter);
+    rc = launch_spatial_index<T>(sizeof(T) == 4 ? reinterpret_cast<const float*>(q) : qf, pf, rec, B, Q, P, L.P_pad, ws,
+                                 L, st, G == kShapeTensorFilter);
   }
   if (rc) return rc;
-  SearchParams sp{};
-  sp.q = (const float*)q;
-  sp.perm_q = reinterpret_cast<const int*>(ws + L.perm_q);
-  sp.tinfo = reinterpret_cast<const float*>(ws + L.tinfo);
-  sp.ntile = L.P_pad / kTilePoints;
-  sp.pairs = pairs;
-  sp.rec = (const float*)rec;
-  sp.f = (const float*)f;
-  sp.B = B;
-  sp.Q = Q;
-  sp.P = P;
-  sp.P_pad = L.P_pad;
-  sp.F = F;
-  sp.K = K;
-  sp.vec4 = (F % 4 == 0) && ((uintptr_t)f % 16 == 0) && ((uintptr_t)f_out % 16 == 0);
-  sp.f_out = (float*)f_out;
-  sp.w_out = (float*)w_out;
-  sp.dists = (float*)dists;
-  sp.idxs = idxs;
-  sp.status = status;
-  sp.flag_count = flag_count;
-  sp.flag_list = flag_list;
-  sp.adj_count = adj_count;
-  sp.qseed = reinterpret_cast<const int*>(ws + L.qseed);
-  sp.tau0 = reinterpret_cast<float*>(ws + L.tau0);
-  sp.plan_est = reinterpret_cast<int*>(ws + L.plan_est);
-  sp.items = reinterpret_cast<int4*>(ws + L.items);
-  sp.tcops = reinterpret_cast<const float*>(ws + L.tcops);
-  sp.tcinfo = reinterpret_cast<const float*>(ws + L.tcinfo);
-  apply_search_debug(sp);
+  const int vec = F < (1 << 28) && (F % (16 / (int)sizeof(T)) == 0) && ((uintptr_t)f % 16 == 0) && ((uintptr_t)f_out % 16 == 0);
   if (G == kShapeTensorFilter) {
     NvtxRange r("knnag:search_tc");
+    sp.q = reinterpret_cast<const float*>(q);
+    sp.perm_q = reinterpret_cast<const int*>(ws + L.perm_q);
+    sp.tinfo = reinterpret_cast<const float*>(ws + L.tinfo);
+    sp.ntile = ntile;
+    sp.pairs = reinterpret_cast<const float*>(ws + L.pairs);
+    sp.rec = reinterpret_cast<const float*>(rec);
+    sp.f = reinterpret_cast<const float*>(f);
+    sp.B = B;
+    sp.Q = Q;
+    sp.P = P;
+    sp.P_pad = L.P_pad;
+    sp.F = F;
+    sp.K = K;
+    sp.vec4 = vec;
+    sp.f_out = reinterpret_cast<float*>(f_out);
+    sp.w_out = reinterpret_cast<float*>(w_out);
+    sp.dists = reinterpret_cast<float*>(dists);
+    sp.idxs = idxs;
+    sp.status = status;
+    sp.flag_count = flag_count;
+    sp.flag_list = flag_list;
+    sp.adj_count = adj_count;
+    sp.qseed = reinterpret_cast<const int*>(ws + L.qseed);
+    sp.tau0 = reinterpret_cast<float*>(ws + L.tau0);
+    sp.plan_est = reinterpret_cast<int*>(ws + L.plan_est);
+    sp.items = reinterpret_cast<int4*>(ws + L.items);
+    sp.tcops = reinterpret_cast<const float*>(ws + L.tcops);
+    sp.tcinfo = reinterpret_cast<const float*>(ws + L.tcinfo);
     rc = launch_search_tc(sp, st);
   } else {
     NvtxRange r("knnag:search");
-    if (K <= 8)
-      rc = launch_search_k<8>(sp, G, st);
-    else if (K <= 16)
-      rc = launch_search_k<16>(sp, G, st);
-    else
-      rc = launch_search_k<32>(sp, G, st);
+    WarpSearchParams<T> wp{};
+    wp.q = q;
+    wp.perm_q = reinterpret_cast<const int*>(ws + L.perm_q);
+    wp.qseed = reinterpret_cast<const int*>(ws + L.qseed);
+    wp.rec = rec;
+    wp.pairs = reinterpret_cast<const T*>(ws + L.pairs);
+    wp.tbox = reinterpret_cast<const float*>(ws + L.tbox);
+    wp.sbox = reinterpret_cast<const float4*>(ws + L.sbox);
+    wp.gbox = reinterpret_cast<const float*>(ws + L.gbox);
+    wp.ngroup = (ntile + 31) / 32;
+    wp.f = f;
+    wp.B = B;
+    wp.Q = Q;
+    wp.P = P;
+    wp.F = F;
+    wp.K = K;
+    wp.ntile = ntile;
+    wp.vec = vec;
+    wp.f_out = f_out;
+    wp.w_out = w_out;
+    wp.dists = dists;
+    wp.idxs = idxs;
+    wp.status = status;
+    wp.flag_count = flag_count;
+    wp.flag_list = flag_list;
+    wp.adj_count = adj_count;
+    rc = launch_search_warp<T>(wp, G, st);
   }
   if (rc) return rc;
   // Exact MinK replay of the flagged queries (count read on the device).
   NvtxRange r("knnag:replay_flagged");
-  ExactParams<float> e{(const float*)q, (const float*)rec, (const float*)f, nullptr, nullptr, 0, B, Q, P, F, K, 1,
-                       flag_list, flag_count, (float*)f_out, (float*)w_out, (float*)dists, idxs};
+  ExactParams<T> e{q, rec, f, nullptr, nullptr, 0, B, Q, P, F, K, 1, flag_list, flag_count, f_out, w_out, dists, idxs};
   e.adj_count = adj_count;
-  return launch_exact<float>(e, st);
+  return launch_exact<T>(e, st);
+}
+
+template <typename T>
+static int forward_t(const T* q, const T* p, const T* f, const T* sigma, const T* R, int B, int Q, int P, int F, int K,
+                     int dtype, T* f_out, T* w_out, T* dists, int64_t* idxs, void* points, char* ws, size_t ws_bytes,
+                     int* adj_count, cudaStream_t st) {
+  bool indexed = false;
+  const FwdLayout L = fwd_layout_in(B, Q, P, K, dtype, points == nullptr, ws_bytes, &indexed);
+  if (L.total > ws_bytes) return KNNAG_ERR_WORKSPACE;
+  T* rec = points ? static_cast<T*>(points) : reinterpret_cast<T*>(ws + L.rec);
+  if (indexed)
+    return forward_indexed_t<T>(q, p, f, sigma, R, B, Q, P, F, K, f_out, w_out, dists, idxs, rec, ws, L, adj_count, st);
+  // the exact kernel serves every query; the packing zeroes the status words
+  // and the adjacency's entry counts
+  int rc;
+  {
+    NvtxRange r("knnag:pack_points");
+    rc = launch_pack_points(p, sigma, R, B, P, dtype, rec, st, reinterpret_cast<int*>(ws + L.status), 2, adj_count);
+  }
+  if (rc) return rc;
+  return forward_exact_all<T>(q, rec, f, B, Q, P, F, K, f_out, w_out, dists, idxs, adj_count, st);
+}
+
+int forward_impl(const void* q, const void* p, const void* f, const void* sigma, const void* R, int B, int Q,
+                 int P, int F, int K, int dtype, void* f_out, void* w_out, void* dists, int64_t* idxs,
+                 void* points, void* workspace, size_t workspace_bytes, cudaStream_t st, void* adjacency) {
+  NvtxRange range("knnag:forward");
+  int* adj_count = adjacency ? reinterpret_cast<int*>(static_cast<char*>(adjacency) + adj_layout(B, Q, P, K).cursor)
+                             : nullptr;
+  char* ws = static_cast<char*>(workspace);
+  if (dtype == KNNAG_F64)
+    return forward_t<double>((const double*)q, (const double*)p, (const double*)f, (const double*)sigma,
+                             (const double*)R, B, Q, P, F, K, dtype, (double*)f_out, (double*)w_out, (double*)dists,
+                             idxs, points, ws, workspace_bytes, adj_count, st);
+  return forward_t<float>((const float*)q, (const float*)p, (const float*)f, (const float*)sigma, (const float*)R, B,
+                          Q, P, F, K, dtype, (float*)f_out, (float*)w_out, (float*)dists, idxs, points, ws,
+                          workspace_bytes, adj_count, st);
 }
 
 RaggedLayout ragged_layout(int cap_segs, int64_t cap_q) {
@@ -1764,33 +987,27 @@ int ragged_forward_impl(const char* cs, const void* segs, const float* q, const 
                           reinterpret_cast<int*>(ws + L.cell_offset), perm_q, status, st);
   if (rc) return rc;
   const int ks = max_k < 32 ? max_k : 32;
-  SearchParams sp{};
-  sp.q = q;
-  sp.perm_q = perm_q;
-  sp.ntile = ntile_cap;
-  sp.f = f;
-  sp.B = 1;
-  sp.F = F;
-  sp.K = ks;
-  sp.vec4 = (F % 4 == 0) && ((uintptr_t)f % 16 == 0) && ((uintptr_t)f_out % 16 == 0);
-  sp.f_out = f_out;
-  sp.w_out = w_out;
-  sp.dists = dists;
-  sp.idxs = idxs;
-  sp.status = status;
-  sp.flag_count = flag_count;
-  sp.flag_list = flag_list;
-  sp.cs = cs;
-  sp.segs = segs;
-  sp.item_counter = item_counter;
-  apply_search_debug(sp);
+  if (ntile_cap > kSearchMaxTiles) return KNNAG_ERR_TOO_LARGE;
+  WarpSearchParams<float> wp{};
+  wp.q = q;
+  wp.perm_q = perm_q;
+  wp.f = f;
+  wp.F = F;
+  wp.K = ks;
+  wp.ntile = ntile_cap;
+  wp.vec = F < (1 << 28) && (F % 4 == 0) && ((uintptr_t)f % 16 == 0) && ((uintptr_t)f_out % 16 == 0);
+  wp.f_out = f_out;
+  wp.w_out = w_out;
+  wp.dists = dists;
+  wp.idxs = idxs;
+  wp.status = status;
+  wp.flag_count = flag_count;
+  wp.flag_list = flag_list;
+  wp.cs = cs;
+  wp.segs = segs;
+  wp.item_counter = item_counter;
   const int64_t cap_items = cap_q / qpc + cap_segs;
-  if (ks <= 8)
-    rc = launch_search_ragged_k<8>(sp, G, cap_items, st);
-  else if (ks <= 16)
-    rc = launch_search_ragged_k<16>(sp, G, cap_items, st);
-  else
-    rc = launch_search_ragged_k<32>(sp, G, cap_items, st);
+  rc = launch_search_warp_ragged(wp, G, cap_items, st);
   if (rc) return rc;
   ExactParams<float> e{};
   e.q = q;

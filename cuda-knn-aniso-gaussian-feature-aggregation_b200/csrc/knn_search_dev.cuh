@@ -1,7 +1,6 @@
-// Device helpers shared by the search kernels (knn_search.cu: the CUDA-core
-// search and its plan; knn_search_tc.cu: the tensor-core filtered search):
-// the sorted candidate list, the candidate queues, the seed thresholds and
-// the tile lower bound.
+// Device helpers of the tensor-core filtered search (knn_search_tc.cu) and its
+// plan (knn_search.cu): the sorted candidate list, the seed thresholds and the
+// tile lower bound.
 #pragma once
 
 #include "knn_common.cuh"
@@ -31,35 +30,6 @@ __device__ __forceinline__ void list_insert(float (&keys)[L], int (&vals)[L], fl
   keys[0] = lt[0] ? k : keys[0];
   vals[0] = lt[0] ? i : vals[0];
   if (lt[L - 1] && out_i >= 0 && out_k == keys[L - 1]) tie_key = fminf(tie_key, out_k);
-}
-
-// Queue slot of entry e of query (lane) j: rows are rotated by j so that
-// appends (one query, consecutive entries) and drains (every lane its own
-// query, the same entry) are both free of bank conflicts.
-__device__ __forceinline__ int queue_slot(int j, int e) { return j * kQCap + ((e + j) & (kQCap - 1)); }
-
-// Lane `lane` folds its query's n queued candidates into its list and
-// refreshes its threshold; the caller resets the counts.
-template <int L>
-__device__ __forceinline__ void drain_queue(float (&keys)[L], int (&vals)[L], float& tie_key, float& tau, int n,
-                                            const float* qk, const int* qv, int lane) {
-  // the next entry is loaded while this one is folded in
-  float k = n > 0 ? qk[queue_slot(lane, 0)] : 0.f;
-  int i = n > 0 ? qv[queue_slot(lane, 0)] : -1;
-  for (int e = 0; e < n; ++e) {
-    const int s = queue_slot(lane, e + 1);
-    const float kn = e + 1 < n ? qk[s] : 0.f;
-    const int in = e + 1 < n ? qv[s] : -1;
-    const float top = keys[L - 1];
-    if (k < top) {
-      list_insert<L>(keys, vals, k, i, tie_key);
-    } else if (k == top) {
-      tie_key = fminf(tie_key, k);
-    }
-    k = kn;
-    i = in;
-  }
-  tau = fminf(tau, keys[L - 1]);
 }
 
 // Seed thresholds of a warp's NQ queries (NQ = 8, 16 or 32).  Any K+1
@@ -139,32 +109,6 @@ __device__ __forceinline__ void seed_warp(float4* tab, int my_seed, bool valid, 
     }
   }
 }
-
-// One search work item: up to WPC * QPW queries of one batch element or
-// segment, all against one cloud.  Pointers are offset to the group already.
-struct SearchItem {
-  const float* q;      // query rows (group-local index)
-  const int* perm_q;   // sorted position -> group-local query index
-  const float* rec;    // the cloud's records
-  const float* pairs;  // the cloud's search tiles
-  const float* tinfo;  // the cloud's tile infos (kTinfoFloats per tile)
-  const float* f;      // the cloud's feature rows
-  float* f_out;        // rows of the group's queries
-  float* w_out;        // entries of the group's queries (K per query)
-  float* dists;
-  int64_t* idxs;
-  int64_t row0;        // global query row of group-local query 0
-  int* adj_count;      // the group's per-point entry counts (optional)
-  const int* qseed;    // seed positions of the group's sorted queries (optional)
-  const float* tau0;   // or their seed thresholds, from the plan kernel (optional)
-  // or seeds from the query's cell: the scanned point counts of the
-  // cloud's grid cells (global positions, cell 0 first), its box and grid
-  const int* cell_start;
-  const float* cbox;
-  int cbits;
-  int Q, P, K, ntile;
-  int q0, q1;          // the item's queries: sorted positions [q0, q1), at most WPC * QPW
-};
 
 // Lower bound on the key of any query in box [bmin, bmax] against any point
 // of a tile (its box ti[0..5], bound factor mu = ti[6]): mu * dist(box,

@@ -35,6 +35,17 @@
 namespace knnag {
 namespace {
 
+constexpr size_t kSearchTileBytes = 8192;  // 128 points x 16 floats
+// Tiles per cloud rounded up to a power of two (the visit-order sort), and
+// the bytes of the order: bounds, tiles, counter.
+__host__ __device__ inline int search_tiles_pow2(int ntile) {
+  int n = 1;
+  while (n < ntile) n <<= 1;
+  return n;
+}
+__host__ __device__ inline size_t search_region_c_bytes(int ntile) { return (size_t)search_tiles_pow2(ntile) * 8 + 16; }
+
+
 constexpr int kTcQ = 128;           // queries per CTA = MMA M = TMEM lanes
 constexpr int kTcThreads = 256;     // two threads per query
 constexpr uint32_t kTcCols = 128;   // TMEM columns: one 128 x 128 FP32 accumulator

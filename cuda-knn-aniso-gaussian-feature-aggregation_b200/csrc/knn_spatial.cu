@@ -389,42 +389,60 @@ __device__ void tc_tile_operand(const float* tile, float (*red)[8], int k, bool 
 // for padding, whose sigma is NaN so its key is never a candidate) and
 // writes tinfo[tile * kTinfoFloats]: the tile's {min xyz, max xyz, mu, 0},
 // then one such box per warp's 32 points (the sub-boxes).
-__global__ void __launch_bounds__(kTilePoints) tile_info_kernel(const float* __restrict__ rec,
+// It also writes the same boxes where the one-warp-per-query search reads
+// them: the tile's by plane (plane m at tbox[m * tplane + tile], lanes over
+// tiles read each plane coalesced) and the sub-boxes as 8 float4 per tile
+// (4 x (min, mu), then 4 x (max, 0): the four lanes of a tile read 64
+// contiguous bytes).  FP64 records keep FP64 tiles; the boxes are rounded
+// outwards to FP32.
+template <typename T>
+__device__ __forceinline__ T index_bits(int idx);
+template <>
+__device__ __forceinline__ float index_bits<float>(int idx) { return __int_as_float(idx); }
+template <>
+__device__ __forceinline__ double index_bits<double>(int idx) { return (double)idx; }
+__device__ __forceinline__ float round_down(float v) { return v; }
+__device__ __forceinline__ float round_up_f(float v) { return v; }
+__device__ __forceinline__ float round_down(double v) { return __double2float_rd(v); }
+__device__ __forceinline__ float round_up_f(double v) { return __double2float_ru(v); }
+
+template <typename T>
+__global__ void __launch_bounds__(kTilePoints) tile_info_kernel(const T* __restrict__ rec,
                                                                 const int* __restrict__ perm,
                                                                 const CloudDesc* __restrict__ cd, int P, int ntile,
-                                                                float* __restrict__ pairs,
-                                                                float* __restrict__ tinfo,
-                                                                float* __restrict__ tcops,
+                                                                T* __restrict__ pairs, float* __restrict__ tinfo,
+                                                                float* __restrict__ tbox, int64_t tplane,
+                                                                float4* __restrict__ sbox, float* __restrict__ tcops,
                                                                 float* __restrict__ tcinfo) {
   const TileGroup g = tile_group(cd, blockIdx.y, P, ntile);
   const int t = blockIdx.x;
   if (t >= g.ntile) return;
   __shared__ float red[kTilePoints / 32][8];
-  __shared__ __align__(16) float tile[kTilePoints * kRecLen];
+  __shared__ __align__(16) T tile[kTilePoints * kRecLen];
   const int k = threadIdx.x, lane = k & 31, warp = k >> 5;
   float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
   float mu = INFINITY;
   bool bad = false;
   const int pos = t * kTilePoints + k;
-  float* slot = tile + k;  // field f of point k at slot[f * kTilePoints]
+  T* slot = tile + k;  // field f of point k at slot[f * kTilePoints]
   if (pos >= g.P) {
 #pragma unroll
     for (int m = 0; m < kRecLen; ++m)
-      slot[m * kTilePoints] = m == kRecPad ? __int_as_float(-1)
-                                           : ((m == kS0 || m == kS1 || m == kS2) ? __int_as_float(0x7fc00000) : 0.0f);
+      slot[m * kTilePoints] = m == kRecPad ? index_bits<T>(-1)
+                                           : ((m == kS0 || m == kS1 || m == kS2) ? T(__int_as_float(0x7fc00000)) : T(0));
   } else {
     const int idx = perm[g.p0 + pos];
-    const float* r = rec + (g.p0 + idx) * kRecLen;
-    float v[kRecLen];
+    const T* r = rec + (g.p0 + idx) * kRecLen;
+    T v[kRecLen];
     load_rec(r, v);
 #pragma unroll
-    for (int m = 0; m < kRecLen; ++m) slot[m * kTilePoints] = m == kRecPad ? __int_as_float(idx) : v[m];
+    for (int m = 0; m < kRecLen; ++m) slot[m * kTilePoints] = m == kRecPad ? index_bits<T>(idx) : v[m];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      const float c = -v[kNPX + a];
-      mn[a] = fminf(mn[a], c);
-      mx[a] = fmaxf(mx[a], c);
-      if (!isfinite(c)) bad = true;
+      const T c = -v[kNPX + a];
+      mn[a] = fminf(mn[a], round_down(c));
+      mx[a] = fmaxf(mx[a], round_up_f(c));
+      if (!isfinite(mn[a]) || !isfinite(mx[a])) bad = true;
     }
     double M[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
     double err = 0.0;
@@ -472,14 +490,17 @@ __global__ void __launch_bounds__(kTilePoints) tile_info_kernel(const float* __r
     }
     o[6] = bad ? -1.0f : mu;  // +inf: no points (the box is empty)
     o[7] = 0.0f;
+    sbox[(g.t0 + t) * 8 + warp] = make_float4(mn[0], mn[1], mn[2], o[6]);
+    sbox[(g.t0 + t) * 8 + 4 + warp] = make_float4(mx[0], mx[1], mx[2], 0.f);
   }
   __syncthreads();
   {
     const float4* src = reinterpret_cast<const float4*>(tile);
     float4* dst = reinterpret_cast<float4*>(pairs + (g.t0 + t) * kTilePoints * kRecLen);
-    for (int i = k; i < kTilePoints * kRecLen / 4; i += kTilePoints) dst[i] = src[i];
+    for (int i = k; i < (int)(kTilePoints * kRecLen * sizeof(T) / 16); i += kTilePoints) dst[i] = src[i];
   }
-  if (tcops) tc_tile_operand(tile, red, k, pos < g.P, tcops + (g.t0 + t) * kTcOpsFloats, tcinfo + (g.t0 + t) * kTcInfoFloats);
+  if constexpr (sizeof(T) == 4)
+    if (tcops) tc_tile_operand(tile, red, k, pos < g.P, tcops + (g.t0 + t) * kTcOpsFloats, tcinfo + (g.t0 + t) * kTcInfoFloats);
   if (k == 0) {
     for (int w = 1; w < kTilePoints / 32; ++w) {
       for (int a = 0; a < 3; ++a) {
@@ -496,7 +517,43 @@ __global__ void __launch_bounds__(kTilePoints) tile_info_kernel(const float* __r
     }
     o[6] = bad ? -1.0f : (mu < INFINITY ? mu : 0.0f);  // -1: the tile has no key bound
     o[7] = 0.0f;
+    for (int m = 0; m < 7; ++m) tbox[m * tplane + g.t0 + t] = o[m];
   }
+}
+
+// Boxes of groups of 32 tiles (warp blockIdx.x of batch element or cloud
+// blockIdx.y): the search tests a group before its tiles.  mu is the least of
+// the group's tiles, -1 where one has no bound.
+__global__ void __launch_bounds__(32) group_box_kernel(const CloudDesc* __restrict__ cd, int ntile, int ngroup,
+                                                       const float* __restrict__ tbox, int64_t tplane,
+                                                       float* __restrict__ gbox, int64_t gplane) {
+  const int b = blockIdx.y, gi = blockIdx.x, lane = threadIdx.x;
+  const int64_t t0 = cd ? cd[b].tile_off : (int64_t)b * ntile;
+  const int nt = cd ? cd[b].ntile : ntile;
+  if (gi * 32 >= nt) return;
+  const int t = gi * 32 + lane;
+  float v[7];
+#pragma unroll
+  for (int m = 0; m < 7; ++m) v[m] = t < nt ? tbox[m * tplane + t0 + t] : (m >= 3 && m < 6 ? -INFINITY : INFINITY);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int m = 0; m < 7; ++m) {
+      const float w = __shfl_xor_sync(0xffffffffu, v[m], o);
+      v[m] = m >= 3 && m < 6 ? fmaxf(v[m], w) : fminf(v[m], w);
+    }
+  if (lane == 0) {
+    const int64_t g0 = (cd ? first_group(t0, b) : (int64_t)b * ngroup) + gi;
+#pragma unroll
+    for (int m = 0; m < 7; ++m) gbox[m * gplane + g0] = v[m];
+  }
+}
+
+int point_bits(int P) {
+  int bits = spatial_bits(P);
+  if (P > 4096)
+    while (bits < 10 && (int64_t(1) << (3 * bits)) < P) ++bits;
+  return bits;
 }
 
 int spatial_bits(int P) {
@@ -512,8 +569,11 @@ unsigned grid_x(int64_t n, int sms, int groups) {
 }
 }  // namespace
 
-int launch_spatial_index(const float* q, const float* rec, int B, int Q, int P, int P_pad, char* ws, const FwdLayout& L,
-                         cudaStream_t st, bool tc_ops) {
+// qf, pf: the coordinates the cells are taken from (FP32): the queries, and
+// for FP64 the rounded points (FP32 points are read from the records).
+template <typename T>
+int launch_spatial_index(const float* qf, const float* pf, const T* rec, int B, int Q, int P, int P_pad, char* ws,
+                         const FwdLayout& L, cudaStream_t st, bool tc_ops) {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -522,7 +582,7 @@ int launch_spatial_index(const float* q, const float* rec, int B, int Q, int P, 
   int* cnt = reinterpret_cast<int*>(ws + L.cell_count);
   int* off = reinterpret_cast<int*>(ws + L.cell_offset);
   int* perm = reinterpret_cast<int*>(ws + L.perm_p);  // perm_q follows perm_p directly
-  float* pairs = reinterpret_cast<float*>(ws + L.pairs);
+  T* pairs = reinterpret_cast<T*>(ws + L.pairs);
   float* tinfo = reinterpret_cast<float*>(ws + L.tinfo);
   const int ntile = P_pad / kTilePoints;
   GroupMap pm{P, bits, nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -532,8 +592,9 @@ int launch_spatial_index(const float* q, const float* rec, int B, int Q, int P, 
   // one counting sort: their cells are scanned together, so the queries'
   // positions start after all points' and land in perm_q, which follows perm_p
   const int64_t nc = 2 * (int64_t)B * cells;
-  const CellJob jp{rec + kNPX, kRecLen, 1, pm, 0, kBoundParts};
-  const CellJob jq{q, 3, 0, qm, B * cells, kBoundParts, reinterpret_cast<int*>(ws + L.qseed), (int64_t)B * P};
+  const CellJob jp = sizeof(T) == 4 ? CellJob{reinterpret_cast<const float*>(rec) + kNPX, kRecLen, 1, pm, 0, kBoundParts}
+                                    : CellJob{pf, 3, 0, pm, 0, kBoundParts};
+  const CellJob jq{qf, 3, 0, qm, B * cells, kBoundParts, reinterpret_cast<int*>(ws + L.qseed), (int64_t)B * P};
   const dim3 grid(grid_x(P > Q ? P : Q, sms, B), B, 2);
   cell_count_kernel<<<grid, 256, 0, st>>>(jp, jq, bnd, cnt);
   if (nc <= kScatterScanMax) {
@@ -545,12 +606,26 @@ int launch_spatial_index(const float* q, const float* rec, int B, int Q, int P, 
     if (rc) return rc;
     cell_scatter_kernel<<<grid, 256, 0, st>>>(jp, jq, bnd, off, cnt, perm);
   }
-  tile_info_kernel<<<dim3(ntile, B), kTilePoints, 0, st>>>(rec, perm, nullptr, P, ntile, pairs, tinfo,
+  tile_info_kernel<T><<<dim3(ntile, B), kTilePoints, 0, st>>>(rec, perm, nullptr, P, ntile, pairs, tinfo,
+                                                            reinterpret_cast<float*>(ws + L.tbox), (int64_t)B * ntile,
+                                                            reinterpret_cast<float4*>(ws + L.sbox),
                                                             tc_ops ? reinterpret_cast<float*>(ws + L.tcops) : nullptr,
                                                             tc_ops ? reinterpret_cast<float*>(ws + L.tcinfo) : nullptr);
   note_launches(3);  // + 1 scan, counted by launch_exclusive_scan
+  const int ngroup = (ntile + 31) / 32;
+  if (ngroup > 2 && !tc_ops) {  // with one or two groups the search takes them all
+    group_box_kernel<<<dim3(ngroup, B), 32, 0, st>>>(nullptr, ntile, ngroup, reinterpret_cast<const float*>(ws + L.tbox),
+                                                     (int64_t)B * ntile, reinterpret_cast<float*>(ws + L.gbox),
+                                                     (int64_t)B * ngroup);
+    note_launches(1);
+  }
   return cudaGetLastError() == cudaSuccess ? KNNAG_OK : KNNAG_ERR_CUDA;
 }
+
+template int launch_spatial_index<float>(const float*, const float*, const float*, int, int, int, int, char*,
+                                         const FwdLayout&, cudaStream_t, bool);
+template int launch_spatial_index<double>(const float*, const float*, const double*, int, int, int, int, char*,
+                                          const FwdLayout&, cudaStream_t, bool);
 
 // Cloud-set index: bounds, Hilbert order, sorted tiles and tile boxes of
 // every cloud (records already packed); the cell offsets stay in the cloud
@@ -575,9 +650,13 @@ int launch_cloudset_index(char* cs, const CloudSetHeader& h, const CloudDesc* cd
   int rc = launch_exclusive_scan(cnt, h.total_cells, off, st);
   if (rc) return rc;
   cell_scatter_kernel<<<grid, 256, 0, st>>>(jp, jp, bnd, off, cnt, perm_p);
-  tile_info_kernel<<<dim3(max_ntile, C), kTilePoints, 0, st>>>(rec, perm_p, cd_dev, 0, 0, pairs, tinfo, nullptr,
-                                                                nullptr);
-  note_launches(4);  // + 1 scan
+  tile_info_kernel<float><<<dim3(max_ntile, C), kTilePoints, 0, st>>>(
+      rec, perm_p, cd_dev, 0, 0, pairs, tinfo, reinterpret_cast<float*>(cs + h.tbox_off), h.total_tiles,
+      reinterpret_cast<float4*>(cs + h.sbox_off), nullptr, nullptr);
+  group_box_kernel<<<dim3((max_ntile + 31) / 32, C), 32, 0, st>>>(
+      cd_dev, 0, 0, reinterpret_cast<const float*>(cs + h.tbox_off), h.total_tiles,
+      reinterpret_cast<float*>(cs + h.gbox_off), tile_groups(h.total_tiles, C));
+  note_launches(5);  // + 1 scan
   return cudaGetLastError() == cudaSuccess ? KNNAG_OK : KNNAG_ERR_CUDA;
 }
 

@@ -1,0 +1,108 @@
+"""The one-warp-per-query search at the sizes where it can go wrong: list
+lengths around 32, 64 and 128, FP64, clouds of one point around a tile, a
+group of tiles and the finer grid, queries that fill no unit, tied, negative
+and non-finite keys.
+
+Two oracles, both exact (every output must be equal bit for bit, so there is
+no tolerance): the CPU oracle for FP32 indices and keys, and the exact MinK
+kernel, which serves FP64 and K > 32 when the workspace has no room for the
+search index."""
+import numpy as np
+import pytest
+import torch
+
+import oracle as O
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda:0")
+
+
+def _inputs(kind, B, Q, P, F, dtype, seed):
+    g = torch.Generator().manual_seed(seed)
+    q = torch.rand(B, Q, 3, generator=g, dtype=torch.float64)
+    p = torch.rand(B, P, 3, generator=g, dtype=torch.float64)
+    f = torch.rand(B, P, F, generator=g, dtype=torch.float64)
+    sigma = torch.rand(B, P, 3, generator=g, dtype=torch.float64)
+    R = torch.rand(B, P, 3, 3, generator=g, dtype=torch.float64)
+    if kind == "ties":  # a coarse lattice, unit Gaussians: most keys are shared
+        p, q = (p * 5).round() / 4, (q * 9).round() / 8
+        sigma, R = torch.ones_like(sigma), torch.eye(3, dtype=torch.float64).expand(B, P, 3, 3).clone()
+    elif kind == "negative":
+        sigma = sigma - 0.5
+    elif kind == "nan":
+        p[:, 1::97] = float("nan")
+        sigma[:, 3::89] = float("inf")
+    elif kind == "far":  # queries outside the points' box, where windows tell little
+        q = q * 6 - 3
+    return [t.to(dtype).contiguous().to(DEV) for t in (q, p, f, sigma, R)]
+
+
+def _call(x, K, ws_bytes):
+    from cuda_knn_aggregate import capi
+
+    q, p, f, sigma, R = x
+    B, Q, P, F = q.shape[0], q.shape[1], p.shape[1], f.shape[2]
+    o = dict(dtype=q.dtype, device=DEV)
+    out = [torch.full((B, Q, F), -7.0, **o), torch.full((B, Q, K), -7.0, **o), torch.full((B, Q, K), -7.0, **o),
+           torch.full((B, Q, K), -7, dtype=torch.int64, device=DEV)]
+    ws = torch.empty(ws_bytes, dtype=torch.uint8, device=DEV)
+    code = capi.F64 if q.dtype == torch.float64 else capi.F32
+    rc = capi.lib().knnag_forward(*[capi._p(t) for t in x], B, Q, P, F, K, code, *[capi._p(t) for t in out], None,
+                                  capi._p(ws), ws_bytes, capi._stream(DEV))
+    assert rc == 0 and capi.read_device_status(ws, DEV) == 0
+    return out
+
+
+def _bits(t):
+    return t.view(torch.int32) if t.dtype == torch.float32 else t.view(torch.int64)
+
+
+@pytest.mark.parametrize("kind,dtype,B,Q,P,F,K", [
+    ("rand", torch.float64, 2, 131, 128, 6, 1),       # one tile; units of 4 with 3 left over
+    ("rand", torch.float64, 1, 257, 4097, 5, 32),     # full list; past a group of tiles, finer grid, odd F
+    ("rand", torch.float64, 1, 60, 700, 4, 33),       # second list register
+    ("rand", torch.float64, 1, 30, 700, 4, 128),      # fourth
+    ("rand", torch.float32, 2, 101, 129, 8, 33),
+    ("rand", torch.float32, 1, 203, 8193, 12, 64),    # full two-register list; three groups of tiles
+    ("rand", torch.float32, 1, 45, 1000, 4, 65),
+    ("rand", torch.float32, 1, 33, 128, 4, 128),      # K == P
+    ("ties", torch.float64, 1, 90, 600, 4, 9),
+    ("ties", torch.float32, 1, 90, 600, 4, 64),
+    ("negative", torch.float64, 1, 70, 900, 4, 12),
+    ("negative", torch.float32, 1, 70, 900, 4, 40),
+    ("nan", torch.float64, 1, 70, 900, 4, 12),
+    ("nan", torch.float32, 1, 70, 900, 4, 40),
+    ("far", torch.float64, 1, 300, 9000, 4, 16),
+    ("far", torch.float32, 1, 300, 9000, 4, 48),
+])
+def test_indexed_calls_equal_the_exact_kernel(kind, dtype, B, Q, P, F, K):
+    from cuda_knn_aggregate import capi
+
+    x = _inputs(kind, B, Q, P, F, dtype, seed=P + K)
+    size = 8 if dtype == torch.float64 else 4
+    r256 = lambda n: (n + 255) // 256 * 256  # noqa: E731
+    lean = 256 + r256(B * Q * 4) + r256(B * P * 16 * size)
+    full = capi.lib().knnag_forward_workspace_bytes(B, Q, P, F, K, capi.F64 if size == 8 else capi.F32)
+    assert full > lean
+    got, want = _call(x, K, full), _call(x, K, lean)
+    for a, b in zip(got, want):
+        assert torch.equal(_bits(a), _bits(b))
+
+
+@pytest.mark.parametrize("kind,B,Q,P,K", [
+    ("rand", 1, 1, 1, 1), ("rand", 3, 5, 31, 31), ("rand", 1, 6, 64, 32), ("rand", 1, 9, 65, 32),
+    ("rand", 1, 4750, 127, 7),     # two queries a warp
+    ("rand", 1, 9501, 300, 3),     # four a warp, one left over
+    ("far", 1, 700, 4096, 16), ("far", 1, 700, 4097, 32), ("far", 2, 300, 12500, 8),
+    ("ties", 1, 500, 4200, 32), ("negative", 1, 200, 5000, 32), ("nan", 1, 200, 5000, 32),
+])
+def test_forward_matches_the_cpu_oracle(kind, B, Q, P, K):
+    from cuda_knn_aggregate import capi
+
+    x = _inputs(kind, B, Q, P, 4, torch.float32, seed=Q + P)
+    out = _call(x, K, capi.lib().knnag_forward_workspace_bytes(B, Q, P, 4, K, capi.F32))
+    _, _, d_ref, i_ref = O.forward_f32(*[t.cpu() for t in x], K, with_features=False)
+    assert np.array_equal(out[3].cpu().numpy(), i_ref)
+    d = out[2].cpu().numpy()
+    assert np.array_equal(np.isnan(d), np.isnan(d_ref))  # the GPU's and the CPU's NaN differ in their payload
+    assert np.array_equal(d.view(np.int32)[~np.isnan(d)], d_ref.view(np.int32)[~np.isnan(d)])
