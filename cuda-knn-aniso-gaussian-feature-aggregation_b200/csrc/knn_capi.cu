@@ -325,12 +325,12 @@ int knnag_forward_isotropic(const void* q, const void* p, const void* f, const v
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (dtype == KNNAG_F64) {
     ExactParams<double> e{(const double*)q, nullptr, (const double*)f, (const double*)p, (const double*)sigma,
-                          sigma_cols, B, Q, P, F, K, 0, nullptr, nullptr, (double*)f_out, (double*)w_sum,
+                          sigma_cols, B, Q, P, F, K, nullptr, nullptr, (double*)f_out, (double*)w_sum,
                           (double*)dists, idxs};
     return launch_exact<double>(e, st);
   }
   ExactParams<float> e{(const float*)q, nullptr, (const float*)f, (const float*)p, (const float*)sigma, sigma_cols,
-                       B, Q, P, F, K, 0, nullptr, nullptr, (float*)f_out, (float*)w_sum, (float*)dists, idxs};
+                       B, Q, P, F, K, nullptr, nullptr, (float*)f_out, (float*)w_sum, (float*)dists, idxs};
   return launch_exact<float>(e, st);
 }
 

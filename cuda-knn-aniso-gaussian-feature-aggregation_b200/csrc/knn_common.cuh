@@ -142,6 +142,22 @@ __device__ __forceinline__ float2 key_pair(float2 qx2, float2 qy2, float2 qz2, c
                     __ffma2_rn(__fmul2_rn(j, j), pr[kS0], __fmul2_rn(__fmul2_rn(k, k), pr[kS1])));
 }
 
+// MinK's final sort (csrc/mink.cuh:99-112): a bubble sort with a strict '<'
+// swap.
+template <typename T>
+__device__ void bubble_sort_slots(T* sk, int* sv, int size) {
+  for (int x = 0; x < size - 1; ++x)
+    for (int y = 0; y < size - x - 1; ++y)
+      if (sk[y + 1] < sk[y]) {
+        const T tk = sk[y];
+        const int tv = sv[y];
+        sk[y] = sk[y + 1];
+        sv[y] = sv[y + 1];
+        sk[y + 1] = tk;
+        sv[y + 1] = tv;
+      }
+}
+
 // The TF32 part of x (low 13 mantissa bits cleared); x - tf32_hi(x) is exact.
 __device__ __forceinline__ float tf32_hi(float x) { return __int_as_float(__float_as_int(x) & 0xffffe000); }
 

@@ -34,18 +34,15 @@ struct ExactParams {
   const T* iso_sigma;
   int iso_stride;
   int B, Q, P, F, K;
-  int use_list;            // 1: process list[0 .. *list_count), 0: every query
-  const int* list;
+  const int* list;         // replay: the flagged queries' rows, list[0 .. *list_count)
   const int* list_count;
   T* f_out;
   T* w_out;
   T* dists;
   int64_t* idxs;
   // ragged calls (FP32): per-query sizes and offsets from the segment table,
-  // records from the cloud set.  List items are global query rows; without a
-  // list the kernel serves the queries of segments with K > 32.  Nothing is
-  // done when *status is nonzero (a table that failed validation); a list
-  // row out of range latches kStatusBadIndex there.
+  // records from the cloud set.  Nothing is done when *status is nonzero (a
+  // table that failed validation).
   const char* cs;
   const void* segs;
   int* status;
@@ -227,8 +224,13 @@ int ragged_grad_q_impl(const char* cs, const void* segs, const float* q, const f
                        const float* f_row_sums, const int64_t* idxs, int64_t cap_q, float* dq, const int* status,
                        cudaStream_t st);
 int launch_row_sums(const void* f, int64_t rows, int F, int dtype, void* out, cudaStream_t st);
+// Every query (of segments with K > 32: ragged calls) by the exact kernel.
 template <typename T>
 int launch_exact(const ExactParams<T>& a, cudaStream_t st);
+// The queries of a.list (knn_replay.cu), K <= kWarpSearchMaxK; max_points: the
+// most points of any of their clouds.
+template <typename T>
+int launch_replay_list(const ExactParams<T>& a, int max_points, cudaStream_t st);
 int variants_precomputed(const void* q, const void* f, const void* rec, const int64_t* idxs, int B, int Q, int P,
                          int F, int K, int dtype, void* f_out, void* w_out, void* dists, cudaStream_t st);
 int variants_lookup(const void* q, const void* p, const void* f, const void* rec, const int64_t* table, int tstride, int B, int Q,

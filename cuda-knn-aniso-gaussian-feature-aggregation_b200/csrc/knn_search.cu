@@ -149,21 +149,8 @@ __device__ __forceinline__ T warp_max(T v) {
 }
 
 template <typename T>
-__device__ void bubble_sort_slots(T* sk, int* sv, int size) {
-  for (int x = 0; x < size - 1; ++x)
-    for (int y = 0; y < size - x - 1; ++y)
-      if (sk[y + 1] < sk[y]) {
-        const T tk = sk[y];
-        const int tv = sv[y];
-        sk[y] = sk[y + 1];
-        sv[y] = sv[y + 1];
-        sk[y + 1] = tk;
-        sv[y + 1] = tv;
-      }
-}
-
-template <typename T, int NTH>
-__global__ void __launch_bounds__(NTH) mink_replay_kernel(ExactParams<T> a) {
+__global__ void __launch_bounds__(kReplayThreads) mink_replay_kernel(ExactParams<T> a) {
+  constexpr int NTH = kReplayThreads;
   constexpr int CH = replay_chunk<T>();
   constexpr int HC = CH / 2;  // keys per chunk: two chunk buffers
   constexpr unsigned FULL = 0xffffffffu;
@@ -175,8 +162,7 @@ __global__ void __launch_bounds__(NTH) mink_replay_kernel(ExactParams<T> a) {
   const int F = a.F;
   const SegHeader* sh = static_cast<const SegHeader*>(a.segs);
   if (sh && *a.status) return;
-  const int64_t n_items = a.use_list ? (int64_t)(*a.list_count)
-                                     : (sh ? sh->bigk_q : (int64_t)a.B * a.Q);
+  const int64_t n_items = sh ? sh->bigk_q : (int64_t)a.B * a.Q;
 
   for (int64_t item = blockIdx.x; item < n_items; item += gridDim.x) {
     // bq: the query's global row; e0: its first entry; b: batch element
@@ -187,18 +173,8 @@ __global__ void __launch_bounds__(NTH) mink_replay_kernel(ExactParams<T> a) {
     const T* fb;
     if (sh) {
       const SegDesc* sd = seg_descs(a.segs);
-      int s;
-      if (a.use_list) {
-        bq = a.list[item];
-        if (bq < 0 || bq >= sh->total_q) {  // the search lists its own rows: never taken
-          if (tid == 0) atomicOr(a.status, kStatusBadIndex);
-          continue;
-        }
-        s = seg_of_row(sd, sh->nseg, bq);
-      } else {
-        s = seg_of_bigk(sd, sh->nseg, item);
-        bq = sd[s].q_off + (item - sd[s].bigk_off);
-      }
+      const int s = seg_of_bigk(sd, sh->nseg, item);
+      bq = sd[s].q_off + (item - sd[s].bigk_off);
       const SegDesc g = sd[s];
       const CloudDesc c = cloud_descs(a.cs)[g.cloud];
       K = g.K;
@@ -209,8 +185,7 @@ __global__ void __launch_bounds__(NTH) mink_replay_kernel(ExactParams<T> a) {
       fb = a.f + c.p_off * F;
       if (K > a.K || K > P) continue;  // the host checked the table; never reached
     } else {
-      bq = a.use_list ? (int64_t)a.list[item] : item;
-      if (bq < 0 || bq >= (int64_t)a.B * a.Q) continue;  // the search lists its own rows: never taken
+      bq = item;
       b = bq / a.Q;
       K = a.K;
       P = a.P;
@@ -661,28 +636,19 @@ template <typename T>
 int launch_exact(const ExactParams<T>& a, cudaStream_t st) {
   const size_t smem = (size_t)replay_chunk<T>() * sizeof(T) + (size_t)a.K * (sizeof(T) + sizeof(int));
   if (smem > 200 * 1024) return KNNAG_ERR_TOO_LARGE;
-  // A list of flagged queries is short: 512 threads per CTA, fifteen warps
-  // computing keys beside the warp that runs MinK.  Every query of a call:
-  // 256 threads, more queries per SM at once.
-  auto kernel = a.use_list ? mink_replay_kernel<T, 2 * kReplayThreads> : mink_replay_kernel<T, kReplayThreads>;
-  const int threads = a.use_list ? 2 * kReplayThreads : kReplayThreads;
+  auto kernel = mink_replay_kernel<T>;
   if (smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
                               cudaSuccess)
     return KNNAG_ERR_CUDA;
   int dev = 0;
   cudaGetDevice(&dev);
-  int64_t blocks;
-  if (a.use_list) {
-    blocks = (int64_t)num_sms(dev) * 2;  // flagged queries are few; each CTA loops over them
-  } else {
-    blocks = (int64_t)a.B * a.Q;
-    const int64_t cap = (int64_t)num_sms(dev) * 8;
-    if (blocks > cap) blocks = cap;
-  }
+  int64_t blocks = (int64_t)a.B * a.Q;
+  const int64_t cap = (int64_t)num_sms(dev) * 8;
+  if (blocks > cap) blocks = cap;
   if (blocks < 1) blocks = 1;
-  if (!a.use_list) profile_begin(st);
-  kernel<<<(unsigned)blocks, threads, smem, st>>>(a);
-  if (!a.use_list) profile_end(st);
+  profile_begin(st);
+  kernel<<<(unsigned)blocks, kReplayThreads, smem, st>>>(a);
+  profile_end(st);
   note_launches(1);
   return cudaGetLastError() == cudaSuccess ? KNNAG_OK : KNNAG_ERR_CUDA;
 }
@@ -796,7 +762,7 @@ int launch_pack_points(const void* p, const void* sigma, const void* R, int B, i
 template <typename T>
 static int forward_exact_all(const T* q, const T* rec, const T* f, int B, int Q, int P, int F, int K, T* f_out,
                              T* w_out, T* dists, int64_t* idxs, int* adj_count, cudaStream_t st) {
-  ExactParams<T> e{q, rec, f, nullptr, nullptr, 0, B, Q, P, F, K, 0, nullptr, nullptr, f_out, w_out, dists, idxs};
+  ExactParams<T> e{q, rec, f, nullptr, nullptr, 0, B, Q, P, F, K, nullptr, nullptr, f_out, w_out, dists, idxs};
   e.adj_count = adj_count;
   return launch_exact<T>(e, st);
 }
@@ -904,9 +870,9 @@ static int forward_indexed_t(const T* q, const T* p, const T* f, const T* sigma,
   if (rc) return rc;
   // Exact MinK replay of the flagged queries (count read on the device).
   NvtxRange r("knnag:replay_flagged");
-  ExactParams<T> e{q, rec, f, nullptr, nullptr, 0, B, Q, P, F, K, 1, flag_list, flag_count, f_out, w_out, dists, idxs};
+  ExactParams<T> e{q, rec, f, nullptr, nullptr, 0, B, Q, P, F, K, flag_list, flag_count, f_out, w_out, dists, idxs};
   e.adj_count = adj_count;
-  return launch_exact<T>(e, st);
+  return launch_replay_list<T>(e, P, st);
 }
 
 template <typename T>
@@ -1016,7 +982,6 @@ int ragged_forward_impl(const char* cs, const void* segs, const float* q, const 
   e.Q = (int)(cap_q < (1 << 30) ? cap_q : (1 << 30));
   e.F = F;
   e.K = ks;
-  e.use_list = 1;
   e.list = flag_list;
   e.list_count = flag_count;
   e.f_out = f_out;
@@ -1026,10 +991,9 @@ int ragged_forward_impl(const char* cs, const void* segs, const float* q, const 
   e.cs = cs;
   e.segs = segs;
   e.status = status;
-  rc = launch_exact<float>(e, st);
+  rc = launch_replay_list<float>(e, ntile_cap * kTilePoints, st);
   if (rc || max_k <= 32) return rc;
   e.K = max_k;
-  e.use_list = 0;
   return launch_exact<float>(e, st);
 }
 

@@ -106,3 +106,30 @@ def test_forward_matches_the_cpu_oracle(kind, B, Q, P, K):
     d = out[2].cpu().numpy()
     assert np.array_equal(np.isnan(d), np.isnan(d_ref))  # the GPU's and the CPU's NaN differ in their payload
     assert np.array_equal(d.view(np.int32)[~np.isnan(d)], d_ref.view(np.int32)[~np.isnan(d)])
+
+
+@pytest.mark.parametrize("P,K,order", [
+    (700, 12, "lattice"),       # one CTA per query, first ranges only
+    (9000, 32, "lattice"),      # two CTAs, two ranges per warp
+    (70000, 16, "lattice"),     # eight CTAs
+    (70000, 24, "descending"),  # every key is below all before it: more points kept than are merged at a time
+])
+def test_flagged_queries_replay_as_the_cpu_oracle(P, K, order):
+    """Tied keys everywhere (every query is replayed): MinK's order of equal
+    keys depends on the whole history of its slots."""
+    from cuda_knn_aggregate import capi
+
+    g = torch.Generator().manual_seed(P)
+    Q = 23
+    q = (torch.rand(1, Q, 3, generator=g) * 8).round() / 8
+    p = (torch.rand(1, P, 3, generator=g) * 12).round() / 8
+    if order == "descending":
+        p = 2 + (torch.arange(P, 0, -1, dtype=torch.float64) / P).to(torch.float32)[None, :, None].expand(1, P, 3)
+        p = torch.cat([p, p[:, -K:]], 1).contiguous()  # the nearest ones twice
+    P = p.shape[1]
+    x = [t.contiguous() for t in (q, p, torch.rand(1, P, 4, generator=g), torch.ones(1, P, 3),
+                                  torch.eye(3).expand(1, P, 3, 3))]
+    out = _call([t.to(DEV) for t in x], K, capi.lib().knnag_forward_workspace_bytes(1, Q, P, 4, K, capi.F32))
+    _, _, d_ref, i_ref = O.forward_f32(*x, K, with_features=False)
+    assert np.array_equal(out[3].cpu().numpy(), i_ref)
+    assert np.array_equal(out[2].cpu().numpy().view(np.int32), d_ref.view(np.int32))
