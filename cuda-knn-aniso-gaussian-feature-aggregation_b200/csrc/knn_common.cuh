@@ -142,6 +142,30 @@ __device__ __forceinline__ float2 key_pair(float2 qx2, float2 qy2, float2 qz2, c
                     __ffma2_rn(__fmul2_rn(j, j), pr[kS0], __fmul2_rn(__fmul2_rn(k, k), pr[kS1])));
 }
 
+// 16-byte groups of feature columns.
+template <typename T>
+struct Group16;
+template <>
+struct Group16<float> {
+  using type = float4;
+};
+template <>
+struct Group16<double> {
+  using type = double2;
+};
+__device__ __forceinline__ void fma_group(const float4& v, float w, float (&acc)[4]) {
+  acc[0] = __fmaf_rn(v.x, w, acc[0]);
+  acc[1] = __fmaf_rn(v.y, w, acc[1]);
+  acc[2] = __fmaf_rn(v.z, w, acc[2]);
+  acc[3] = __fmaf_rn(v.w, w, acc[3]);
+}
+__device__ __forceinline__ void fma_group(const double2& v, double w, double (&acc)[2]) {
+  acc[0] = __fma_rn(v.x, w, acc[0]);
+  acc[1] = __fma_rn(v.y, w, acc[1]);
+}
+__device__ __forceinline__ float4 group_of(const float (&a)[4]) { return make_float4(a[0], a[1], a[2], a[3]); }
+__device__ __forceinline__ double2 group_of(const double (&a)[2]) { return make_double2(a[0], a[1]); }
+
 // MinK's final sort (csrc/mink.cuh:99-112): a bubble sort with a strict '<'
 // swap.
 template <typename T>

@@ -203,30 +203,6 @@ __device__ __forceinline__ float box_bound(const float (&mn)[3], const float (&m
   return mu >= 0.f ? (lb >= 0.f ? lb : 0.f) : -INFINITY;
 }
 
-// 16-byte groups of feature columns.
-template <typename T>
-struct Vec16;
-template <>
-struct Vec16<float> {
-  using type = float4;
-};
-template <>
-struct Vec16<double> {
-  using type = double2;
-};
-__device__ __forceinline__ void fma_group(const float4& v, float w, float (&acc)[4]) {
-  acc[0] = __fmaf_rn(v.x, w, acc[0]);
-  acc[1] = __fmaf_rn(v.y, w, acc[1]);
-  acc[2] = __fmaf_rn(v.z, w, acc[2]);
-  acc[3] = __fmaf_rn(v.w, w, acc[3]);
-}
-__device__ __forceinline__ void fma_group(const double2& v, double w, double (&acc)[2]) {
-  acc[0] = __fma_rn(v.x, w, acc[0]);
-  acc[1] = __fma_rn(v.y, w, acc[1]);
-}
-__device__ __forceinline__ float4 group_of(const float (&a)[4]) { return make_float4(a[0], a[1], a[2], a[3]); }
-__device__ __forceinline__ double2 group_of(const double (&a)[2]) { return make_double2(a[0], a[1]); }
-
 // What a unit of queries is searched against, and where its results go.
 // Pointers are offset to the unit's batch element or segment and cloud.
 template <typename T>
@@ -665,7 +641,7 @@ __device__ __forceinline__ void search_unit(const WarpSearchParams<T>& a, const 
   // 16 bytes a lane, take the unit's queries side by side, a slice of columns
   // at a time: the queries share most of their neighbours, so a slice of a
   // row one of them has loaded is still in L1 when the next one asks for it.
-  using V16 = typename Vec16<T>::type;
+  using V16 = typename Group16<T>::type;
   const int cols = a.vec ? a.F / (int)(16 / sizeof(T)) : a.F;
   int g = 0;
   while (g < 5 && (1 << g) < cols && (n << g) < 32) ++g;

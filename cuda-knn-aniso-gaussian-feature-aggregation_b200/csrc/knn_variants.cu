@@ -15,119 +15,257 @@
 
 namespace knnag {
 
-// One warp per query.  Lane k (and k+32, ...) takes neighbour k: key from the
-// packed record, w = exp(-key) (-> dists, w_out); the warp then sums
-// f_out = sum_k w_k f[idx_k] in k order with lanes spanning columns.  The
-// neighbour index comes from `idxs` [B,Q,K] or, for the lookup, from
-// `table` [P,K] at row nearest[b*Q+q] (and is written to idxs_out).  An
-// index outside [0, P) contributes nothing (w = 0, dist = +inf).
+// A warp takes four queries.  The K (query, neighbour) pairs of all four first:
+// key from the packed record, w = exp(-key) (-> dists, w_out); then
+// f_out = sum_k w_k f[idx_k] in k order, 8 lanes per query side by side (16
+// bytes a lane where the rows allow), eight rows in flight.  The neighbour
+// index comes from `idxs` [B,Q,K] or, for the lookup, from `table` [P,K] at
+// row nearest[b*Q+q] (and is written to idxs_out).  An index outside [0, P)
+// contributes nothing (w = 0, dist = +inf).
+//
+// Bound by the gathered rows, which L2 serves (K * 4 F bytes per query): with a
+// warp per query and scalar loads 28 us at B = 2, Q = 12288, K = 16, F = 64,
+// now 24 us.
+constexpr int kGatherQueries = 4;
+
 template <typename T>
 __global__ void __launch_bounds__(256) gather_aggregate_kernel(const T* __restrict__ q, const T* __restrict__ f,
                                                               const T* __restrict__ rec,
                                                               const int64_t* __restrict__ idxs,
                                                               const int64_t* __restrict__ table,
                                                               const int* __restrict__ nearest, int tstride, int B,
-                                                              int Q, int P, int F, int K, T* __restrict__ f_out,
-                                                              T* __restrict__ w_out, T* __restrict__ dists,
-                                                              int64_t* __restrict__ idxs_out) {
+                                                              int Q, int P, int F, int K, int vec,
+                                                              T* __restrict__ f_out, T* __restrict__ w_out,
+                                                              T* __restrict__ dists, int64_t* __restrict__ idxs_out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  T* sw = reinterpret_cast<T*>(smem_raw) + (size_t)warp * K;
-  int* si = reinterpret_cast<int*>(reinterpret_cast<T*>(smem_raw) + (size_t)8 * K) + (size_t)warp * K;
-  const int BQ = B * Q;
-  const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nw = (gridDim.x * blockDim.x) >> 5;
-  for (int bq = gw; bq < BQ; bq += nw) {
-    const int b = bq / Q;
-    const T qx = q[(int64_t)bq * 3 + 0], qy = q[(int64_t)bq * 3 + 1], qz = q[(int64_t)bq * 3 + 2];
-    const int64_t row = table ? (int64_t)nearest[bq] : 0;
-    for (int k = lane; k < K; k += 32) {
-      const int64_t e = (int64_t)bq * K + k;
-      const int64_t idx = table ? table[row * tstride + k] : idxs[e];
-      T key = T(INFINITY), w = T(0);
-      if (idx >= 0 && idx < P) {
-        key = key_rec<T>(qx, qy, qz, rec + ((int64_t)b * P + idx) * kRecLen);
-        w = weight_of(key);
+  constexpr int N = kGatherQueries, G = 32 / N;  // queries of the warp, lanes per query
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane / G, gl = lane % G;
+  T* sw = reinterpret_cast<T*>(smem_raw) + (size_t)(warp * N + sub) * K;
+  int* si = reinterpret_cast<int*>(reinterpret_cast<T*>(smem_raw) + (size_t)(blockDim.x >> 5) * N * K) +
+            (size_t)(warp * N + sub) * K;
+  const int64_t BQ = (int64_t)B * Q;
+  const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nw = (gridDim.x * (int64_t)blockDim.x) >> 5;
+  for (int64_t base = gw * N; base < BQ; base += nw * N) {
+    const int64_t bq = base + sub;
+    const int64_t b = bq / Q;
+    if (bq < BQ) {
+      const T qx = q[bq * 3 + 0], qy = q[bq * 3 + 1], qz = q[bq * 3 + 2];
+      const int64_t row = table ? (int64_t)nearest[bq] : 0;
+      for (int k = gl; k < K; k += G) {
+        const int64_t e = bq * K + k;
+        const int64_t idx = table ? table[row * tstride + k] : idxs[e];
+        T key = T(INFINITY), w = T(0);
+        if (idx >= 0 && idx < P) {
+          key = key_rec<T>(qx, qy, qz, rec + (b * P + idx) * kRecLen);
+          w = weight_of(key);
+        }
+        dists[e] = key;
+        w_out[e] = w;
+        if (idxs_out) idxs_out[e] = idx;
+        sw[k] = w;
+        si[k] = (idx >= 0 && idx < P) ? (int)idx : -1;
       }
-      dists[e] = key;
-      w_out[e] = w;
-      if (idxs_out) idxs_out[e] = idx;
-      sw[k] = w;
-      si[k] = (idx >= 0 && idx < P) ? (int)idx : -1;
     }
     __syncwarp();
-    const T* fb = f + (int64_t)b * P * F;
-    for (int c0 = 0; c0 < F; c0 += 32) {
-      const int c = c0 + lane;
-      if (c < F) {
-        T acc = T(0);
-        for (int k = 0; k < K; ++k)
-          if (si[k] >= 0) acc = fma_rn(fb[(int64_t)si[k] * F + c], sw[k], acc);
-        f_out[(int64_t)bq * F + c] = acc;
+    if (bq < BQ) {
+      const T* fb = f + b * P * F;
+      constexpr int RB = 8, C = 16 / sizeof(T);
+      if (vec) {
+        using V = typename Group16<T>::type;
+        const int cols = F / C;
+        for (int c = gl; c < cols; c += G) {
+          T acc[C];
+#pragma unroll
+          for (int u = 0; u < C; ++u) acc[u] = T(0);
+          for (int k0 = 0; k0 < K; k0 += RB) {
+            V v[RB];
+#pragma unroll
+            for (int u = 0; u < RB; ++u)
+              if (k0 + u < K && si[k0 + u] >= 0) v[u] = __ldg(reinterpret_cast<const V*>(fb + (int64_t)si[k0 + u] * F) + c);
+#pragma unroll
+            for (int u = 0; u < RB; ++u)
+              if (k0 + u < K && si[k0 + u] >= 0) fma_group(v[u], sw[k0 + u], acc);
+          }
+          reinterpret_cast<V*>(f_out + bq * F)[c] = group_of(acc);
+        }
+      } else {
+        for (int c = gl; c < F; c += G) {
+          T acc = T(0);
+#pragma unroll 8
+          for (int k = 0; k < K; ++k)
+            if (si[k] >= 0) acc = fma_rn(__ldg(fb + (int64_t)si[k] * F + c), sw[k], acc);
+          f_out[bq * F + c] = acc;
+        }
       }
     }
     __syncwarp();
   }
 }
 
-// Euclidean nearest point of every query: strict '<' scan in index order
-// from 1e10 (the first index wins ties; 0 when no distance is below 1e10),
-// d = fma(z,z, fma(x,x, y*y)) for x*x + y*y + z*z (csrc/forward.cu:141-160).
-// One thread per query, 256 queries per CTA, points staged 1024 at a time.
-template <typename T>
-__global__ void __launch_bounds__(256) nearest_point_kernel(const T* __restrict__ q, const T* __restrict__ p, int B,
-                                                           int Q, int P, int* __restrict__ nearest) {
-  constexpr int CH = 1024;
-  __shared__ T sp[CH * 3];
-  const int b = blockIdx.y;
-  const int qi = blockIdx.x * 256 + threadIdx.x;
-  const bool valid = qi < Q;
-  const int64_t bq = (int64_t)b * Q + (valid ? qi : 0);
-  const T qx = q[bq * 3 + 0], qy = q[bq * 3 + 1], qz = q[bq * 3 + 2];
-  T best = T(1e10);
-  int arg = 0;
-  const T* pb = p + (int64_t)b * P * 3;
-  for (int c0 = 0; c0 < P; c0 += CH) {
-    const int n = min(CH, P - c0);
+// Euclidean nearest point of every query: the smallest
+// d = fma(z,z, fma(x,x, y*y)) for x*x + y*y + z*z below 1e10, of equal ones the
+// lowest index; 0 when there is none (the reference's strict '<' scan in index
+// order from 1e10, csrc/forward.cu:141-160).
+//
+// A CTA serves 32 queries per lane slot (N slots); its 8 warps share the
+// points, four consecutive ones a step, staged in shared memory and broadcast
+// to the N queries of a lane.  A step keeps the least of its four distances
+// and, when that is below the best so far, its place; which of the four it was
+// is found out once at the end, from the same arithmetic.  The broadcasts bound
+// it at N = 1, FP32 issue at N = 2 (5 instructions per pair).  One thread per
+// query with the whole scan left the chip idle: 96 CTAs at B = 2, Q = 12288,
+// P = 4096, 83 us; N = 1 takes 52 us, N = 2 43 us.
+constexpr int kNearestChunk = 1024;  // points staged at a time
+constexpr int kNearestWarps = 8;
+
+// Squared distances to four points, staged negated: x[4], y[4], z[4].
+__device__ __forceinline__ void dist4(float qx, float qy, float qz, const float* s, float (&d)[4]) {
+  const float4 px = *reinterpret_cast<const float4*>(s), py = *reinterpret_cast<const float4*>(s + 4),
+               pz = *reinterpret_cast<const float4*>(s + 8);
+  const float2 X = make_float2(qx, qx), Y = make_float2(qy, qy), Z = make_float2(qz, qz);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const float2 x = __fadd2_rn(X, h ? make_float2(px.z, px.w) : make_float2(px.x, px.y));
+    const float2 y = __fadd2_rn(Y, h ? make_float2(py.z, py.w) : make_float2(py.x, py.y));
+    const float2 z = __fadd2_rn(Z, h ? make_float2(pz.z, pz.w) : make_float2(pz.x, pz.y));
+    const float2 r = __ffma2_rn(z, z, __ffma2_rn(x, x, __fmul2_rn(y, y)));
+    d[2 * h] = r.x;
+    d[2 * h + 1] = r.y;
+  }
+}
+__device__ __forceinline__ void dist4(double qx, double qy, double qz, const double* s, double (&d)[4]) {
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const double x = qx + s[u], y = qy + s[4 + u], z = qz + s[8 + u];
+    d[u] = fma_rn(z, z, fma_rn(x, x, mul_rn(y, y)));
+  }
+}
+
+template <typename T, int N>
+__global__ void __launch_bounds__(32 * kNearestWarps) nearest_point_kernel(const T* __restrict__ q,
+                                                                           const T* __restrict__ p, int Q, int P,
+                                                                           int* __restrict__ nearest) {
+  __shared__ __align__(16) T sp[kNearestChunk * 3];  // steps of four points: x[4] y[4] z[4], negated
+  __shared__ T sbest[kNearestWarps][32 * N];
+  __shared__ int sarg[kNearestWarps][32 * N];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t blocks = (Q + 32 * N - 1) / (32 * N), b = blockIdx.x / blocks;
+  const int q0 = (int)(blockIdx.x - b * blocks) * 32 * N + lane;  // queries q0 + 32 u
+  const T* pb = p + b * P * 3;
+  T qx[N], qy[N], qz[N], best[N];
+  int step[N];  // first point of the best step
+#pragma unroll
+  for (int u = 0; u < N; ++u) {
+    const int64_t bq = b * Q + min(q0 + 32 * u, Q - 1);
+    qx[u] = q[bq * 3 + 0];
+    qy[u] = q[bq * 3 + 1];
+    qz[u] = q[bq * 3 + 2];
+    best[u] = T(1e10);
+    step[u] = -1;
+  }
+  // four points of step s (of the whole cloud), NaN past the last point: never
+  // the nearest
+  auto load = [&](int s, T* dst) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int a = 0; a < 3; ++a) dst[4 * a + u] = 4 * s + u < P ? -pb[(int64_t)(4 * s + u) * 3 + a] : T(NAN);
+  };
+  for (int c0 = 0; c0 < P; c0 += kNearestChunk) {
+    const int steps = (min(kNearestChunk, P - c0) + 3) / 4;
     __syncthreads();
-    for (int i = threadIdx.x; i < n * 3; i += 256) sp[i] = pb[(int64_t)c0 * 3 + i];
+    for (int s = tid; s < steps; s += 32 * kNearestWarps) load(c0 / 4 + s, sp + 12 * s);
     __syncthreads();
-    for (int i = 0; i < n; ++i) {
-      const T x = qx - sp[3 * i], y = qy - sp[3 * i + 1], z = qz - sp[3 * i + 2];
-      const T d = fma_rn(z, z, fma_rn(x, x, mul_rn(y, y)));
-      if (d < best) {
-        best = d;
-        arg = c0 + i;
+#pragma unroll 2
+    for (int s = warp; s < steps; s += kNearestWarps) {
+#pragma unroll
+      for (int u = 0; u < N; ++u) {
+        T d[4];
+        dist4(qx[u], qy[u], qz[u], sp + 12 * s, d);
+        const T m = fmin(fmin(d[0], d[1]), fmin(d[2], d[3]));  // NaN only if all are
+        if (m < best[u]) {
+          best[u] = m;
+          step[u] = c0 + 4 * s;
+        }
       }
     }
   }
-  if (valid) nearest[bq] = arg;
+#pragma unroll
+  for (int u = 0; u < N; ++u) {
+    int arg = 0x7fffffff;
+    if (step[u] >= 0) {
+      __align__(16) T s[12];
+      T d[4];
+      load(step[u] / 4, s);
+      dist4(qx[u], qy[u], qz[u], s, d);
+#pragma unroll
+      for (int v = 3; v >= 0; --v)
+        if (d[v] == best[u]) arg = step[u] + v;
+    }
+    sbest[warp][lane + 32 * u] = best[u];
+    sarg[warp][lane + 32 * u] = arg;
+  }
+  __syncthreads();
+  if (tid < 32 * N && q0 - lane + tid < Q) {
+    T d = sbest[0][tid];
+    int arg = sarg[0][tid];
+    for (int w = 1; w < kNearestWarps; ++w) {
+      const T dw = sbest[w][tid];
+      const int i = sarg[w][tid];
+      if (dw < d || (dw == d && i < arg)) {
+        d = dw;
+        arg = i;
+      }
+    }
+    nearest[b * Q + q0 - lane + tid] = arg == 0x7fffffff ? 0 : arg;
+  }
 }
 
 namespace {
-int variant_blocks(int64_t warps) {
-  int dev = 0, sms = 148;
+int variant_blocks(int64_t warps, int cta_warps) {
+  int dev = 0;
   cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  int64_t b = (warps * 32 + 255) / 256;
-  const int64_t cap = (int64_t)sms * 16;
+  int64_t b = (warps + cta_warps - 1) / cta_warps;
+  const int64_t cap = (int64_t)num_sms(dev) * 16;
   if (b > cap) b = cap;
   return (int)(b < 1 ? 1 : b);
+}
+
+// Two queries per lane where that leaves a CTA of 64 queries for every SM.
+template <typename T>
+int launch_nearest(const T* q, const T* p, int B, int Q, int P, int* nearest, cudaStream_t st) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const bool two = (int64_t)B * Q >= (int64_t)num_sms(dev) * 64;
+  const int per = two ? 64 : 32;
+  const int64_t blocks = (int64_t)((Q + per - 1) / per) * B;
+  if (blocks > 0x7fffffff) return KNNAG_ERR_TOO_LARGE;
+  if (two)
+    nearest_point_kernel<T, 2><<<(unsigned)blocks, 32 * kNearestWarps, 0, st>>>(q, p, Q, P, nearest);
+  else
+    nearest_point_kernel<T, 1><<<(unsigned)blocks, 32 * kNearestWarps, 0, st>>>(q, p, Q, P, nearest);
+  note_launches(1);
+  return cudaGetLastError() == cudaSuccess ? KNNAG_OK : KNNAG_ERR_CUDA;
 }
 
 template <typename T>
 int launch_gather(const T* q, const T* f, const T* rec, const int64_t* idxs, const int64_t* table, const int* nearest,
                   int tstride, int B, int Q, int P, int F, int K, T* f_out, T* w_out, T* dists, int64_t* idxs_out,
                   cudaStream_t st) {
-  const size_t smem = (size_t)8 * K * (sizeof(T) + sizeof(int));
-  if (smem > 200 * 1024) return KNNAG_ERR_TOO_LARGE;
+  const size_t per_query = (size_t)K * (sizeof(T) + sizeof(int));
+  if (8 * per_query > 200 * 1024) return KNNAG_ERR_TOO_LARGE;
+  int cta_warps = 8;  // fewer where the neighbours of 8 x 4 queries do not fit
+  while (cta_warps > 1 && cta_warps * kGatherQueries * per_query > 100 * 1024) cta_warps /= 2;
+  const size_t smem = cta_warps * kGatherQueries * per_query;
   if (smem > 48 * 1024 &&
       cudaFuncSetAttribute(gather_aggregate_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
           cudaSuccess)
     return KNNAG_ERR_CUDA;
-  gather_aggregate_kernel<T><<<variant_blocks((int64_t)B * Q), 256, smem, st>>>(q, f, rec, idxs, table, nearest, tstride,
-                                                                                 B, Q, P, F, K, f_out, w_out, dists,
-                                                                                 idxs_out);
+  const int vec = F % (int)(16 / sizeof(T)) == 0 && (uintptr_t)f % 16 == 0 && (uintptr_t)f_out % 16 == 0;
+  const int64_t warps = ((int64_t)B * Q + kGatherQueries - 1) / kGatherQueries;
+  gather_aggregate_kernel<T><<<variant_blocks(warps, cta_warps), 32 * cta_warps, smem, st>>>(q, f, rec, idxs, table, nearest, tstride, B, Q, P,
+                                                                       F, K, vec, f_out, w_out, dists, idxs_out);
   note_launches(1);
   return cudaGetLastError() == cudaSuccess ? KNNAG_OK : KNNAG_ERR_CUDA;
 }
@@ -145,13 +283,9 @@ int variants_precomputed(const void* q, const void* f, const void* rec, const in
 int variants_lookup(const void* q, const void* p, const void* f, const void* rec, const int64_t* table, int tstride, int B, int Q,
                     int P, int F, int K, int dtype, int* nearest, void* f_out, void* w_out, void* dists,
                     int64_t* idxs, cudaStream_t st) {
-  dim3 grid((Q + 255) / 256, B);
-  if (dtype == KNNAG_F64)
-    nearest_point_kernel<double><<<grid, 256, 0, st>>>((const double*)q, (const double*)p, B, Q, P, nearest);
-  else
-    nearest_point_kernel<float><<<grid, 256, 0, st>>>((const float*)q, (const float*)p, B, Q, P, nearest);
-  note_launches(1);
-  if (cudaGetLastError() != cudaSuccess) return KNNAG_ERR_CUDA;
+  const int rc = dtype == KNNAG_F64 ? launch_nearest<double>((const double*)q, (const double*)p, B, Q, P, nearest, st)
+                                    : launch_nearest<float>((const float*)q, (const float*)p, B, Q, P, nearest, st);
+  if (rc) return rc;
   if (dtype == KNNAG_F64)
     return launch_gather<double>((const double*)q, (const double*)f, (const double*)rec, nullptr, table, nearest,
                                  tstride, B, Q, P, F, K, (double*)f_out, (double*)w_out, (double*)dists, idxs, st);

@@ -261,3 +261,42 @@ def test_variant_gradients(variant):
         assert rel_err(a.detach().cpu().numpy(), b.numpy()) < GRAD_TOL, n
     for n, t, b in zip(("dq", "dp", "df", "dsigma", "dR"), dev, second[1:]):
         assert rel_err(t.grad.cpu().numpy(), b.numpy()) < GRAD_TOL, n
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("B,Q,P", [(1, 1, 1), (2, 33, 3), (1, 70, 1025), (3, 257, 1024), (1, 40, 2050),
+                                   (1, 9500, 131)])  # two queries a lane
+def test_lookup_nearest_point_rules(dtype, B, Q, P):
+    """The nearest point is the lowest index among equal distances; a NaN or a
+    distance of 1e10 or more is never taken, and 0 when nothing is.  Lattice
+    coordinates: every distance is exact, so the comparison has no tolerance.
+    The table is the identity, so idxs[..., 0] is the nearest point."""
+    import cuda_knn_aggregate as C
+
+    g = torch.Generator().manual_seed(Q * P)
+    q = (torch.rand(B, Q, 3, generator=g) * 8).round()
+    p = (torch.rand(B, P, 3, generator=g) * 8).round()
+    p[:, ::7, 1] = float("nan")
+    q[:, ::11] = 3e5  # every squared distance is above 1e10
+    d = ((q[:, :, None].double() - p[:, None].double()) ** 2).sum(-1)
+    d = torch.where(d.isnan() | (d >= 1e10), torch.inf, d)
+    want = torch.where(d.amin(-1).isinf(), 0, d.argmin(-1))  # argmin: the first of equal ones
+    x = [t.to(dtype).cuda() for t in (q, p, torch.rand(B, P, 4), torch.ones(B, P, 3), torch.eye(3).expand(B, P, 3, 3))]
+    table = torch.arange(P)[:, None].cuda()
+    out = C._C.knn_lookup_aggregate_aniso_forward(*[t.contiguous() for t in x], table, 1)
+    assert torch.equal(out[3][..., 0].cpu(), want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,Q,F,K", [(1, 1, 64, 16), (1, 5, 3, 9), (2, 67, 40, 33), (1, 9, 4, 900)])
+def test_precomputed_is_the_fused_ops_sum(B, Q, F, K):
+    """At the fused op's own indices the gather gives its outputs bit for bit
+    (the same keys, weights and order of sums)."""
+    import cuda_knn_aggregate as C
+
+    q, p, f, s, R = [t.cuda() for t in _cloud(B, Q, 1000, F, seed=F + K)]
+    fo, w, d, idx = C.knn_aggregate_aniso(q, p, f, s, R, K)
+    got = C._C.knn_precomputed_aggregate_aniso_forward(q, p, f, s, R, idx, K)
+    for a, b in zip(got, (fo, w, d)):
+        assert torch.equal(a, b)
