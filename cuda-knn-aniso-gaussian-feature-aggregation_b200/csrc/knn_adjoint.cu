@@ -499,9 +499,53 @@ __global__ void __launch_bounds__(256) row_sum_kernel(const T* __restrict__ f, i
   }
 }
 
+// A query row's sizes, first entry, and its cloud's records, features and
+// first point.
+template <typename T>
+struct QueryRow {
+  int K, P;
+  int64_t e0, pbase;
+  const T* recb;
+  const T* fb;
+};
+template <typename T>
+__device__ __forceinline__ QueryRow<T> uniform_row(const QueryParams<T>& a, int64_t bq) {
+  const int64_t b = bq / a.Q;
+  return QueryRow<T>{a.K, a.P, bq * a.K, b * a.P, a.rec + b * a.P * kRecLen, a.f + b * a.P * a.F};
+}
+// Row bq of segment s of a ragged call.
+template <typename T>
+__device__ __forceinline__ QueryRow<T> segment_row(const QueryParams<T>& a, const SegDesc* sd, int s, int64_t bq) {
+  const SegDesc g = sd[s];
+  const CloudDesc c = cloud_descs(a.cs)[g.cloud];
+  const T* rec = reinterpret_cast<const T*>(a.cs + reinterpret_cast<const CloudSetHeader*>(a.cs)->rec_off);
+  return QueryRow<T>{g.K, c.P, g.e_off + (bq - g.q_off) * g.K, c.p_off, rec + c.p_off * kRecLen, a.f + c.p_off * a.F};
+}
+
+// One neighbour's share of dq: -2 c w v.
+template <typename T>
+__device__ __forceinline__ void add_dq(const QueryParams<T>& a, const T* rec_g, T qx, T qy, T qz, int64_t e, T c,
+                                       T (&acc)[3]) {
+  T rec[kRecLen];
+  load_rec(rec_g, rec);
+  Geo<T> geo;
+  geometry(qx, qy, qz, rec, geo);
+  const T w = a.w_in ? a.w_in[e] : geo.w;
+  const T sg[3] = {rec[kS0], rec[kS1], rec[kS2]};
+  T v[3];
+  rot_back(rec + kR00, sg, geo.u, v);
+  const T t = T(-2) * c * w;
+#pragma unroll
+  for (int m = 0; m < 3; ++m) acc[m] += t * v[m];
+}
+
 // First-order query side with a broadcast grad_f_out s: c_k = s *
 // rowsum(f)[idx_k] needs no F-wide dot product, so each lane takes one
-// neighbour, and a warp serves two queries when K <= 16 (uniform calls).
+// neighbour, and a warp serves two queries when K <= 16.  A warp of a ragged
+// call takes kRowBlock consecutive rows, so that the segment is looked up once
+// for them and not by a chain of dependent loads per row.
+constexpr int kRowBlock = 8;
+
 template <typename T>
 __device__ __forceinline__ void query_order1_scalar(const QueryParams<T>& a, const SegHeader* sh, int64_t BQ) {
   const int lane = threadIdx.x & 31;
@@ -510,75 +554,93 @@ __device__ __forceinline__ void query_order1_scalar(const QueryParams<T>& a, con
   const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = (gridDim.x * (int64_t)blockDim.x) >> 5;
   const T sg0 = a.gfo ? a.gfo[0] : T(1);  // ragged calls: no grad_f_out means all ones
-  for (int64_t base = gw * qpw; base < BQ; base += nw * qpw) {
-    const int64_t bq = base + sub;
-    T acc[3] = {T(0), T(0), T(0)};
-    if (bq < BQ) {
-      int K, P;
-      int64_t e0, pbase;
-      const T* recb;
-      if (sh) {
-        const SegDesc* sd = seg_descs(a.segs);
-        const SegDesc g = sd[seg_of_row(sd, sh->nseg, bq)];
-        const CloudDesc c = cloud_descs(a.cs)[g.cloud];
-        K = g.K;
-        P = c.P;
-        e0 = g.e_off + (bq - g.q_off) * K;
-        pbase = c.p_off;
-        recb = reinterpret_cast<const T*>(a.cs + reinterpret_cast<const CloudSetHeader*>(a.cs)->rec_off) +
-               c.p_off * kRecLen;
-      } else {
-        const int64_t b = bq / a.Q;
-        K = a.K;
-        P = a.P;
-        e0 = bq * K;
-        pbase = b * a.P;
-        recb = a.rec + b * a.P * kRecLen;
-      }
-      const T qx = a.q[bq * 3 + 0], qy = a.q[bq * 3 + 1], qz = a.q[bq * 3 + 2];
-      for (int k = kl; k < K; k += lpq) {
-        const int64_t e = e0 + k;
-        const int64_t idx = a.idxs[e];
-        T c = T(0);
-        if (idx >= 0 && idx < P) {
-          c = sg0 * a.frowsum[pbase + idx];
-          T rr[kRecLen];
-          load_rec(recb + idx * kRecLen, rr);
-          const T* rec = rr;
-          Geo<T> geo;
-          geometry(qx, qy, qz, rec, geo);
-          const T w = a.w_in ? a.w_in[e] : geo.w;
-          const T sg[3] = {rec[kS0], rec[kS1], rec[kS2]};
-          T v[3];
-          rot_back(rec + kR00, sg, geo.u, v);
-          const T t = T(-2) * c * w;
-#pragma unroll
-          for (int mm = 0; mm < 3; ++mm) acc[mm] += t * v[mm];
+  const SegDesc* sd = sh ? seg_descs(a.segs) : nullptr;
+  const int rows = sh ? kRowBlock : qpw;  // of a warp's turn
+  for (int64_t turn = gw * rows; turn < BQ; turn += nw * rows) {
+    int s = sh ? seg_of_row(sd, sh->nseg, turn) : 0;
+    for (int64_t base = turn; base < BQ && base < turn + rows; base += qpw) {
+      const int64_t bq = base + sub;
+      T acc[3] = {T(0), T(0), T(0)};
+      if (sh)
+        while (s + 1 < sh->nseg && sd[s + 1].q_off <= bq) ++s;
+      if (bq < BQ) {
+        const QueryRow<T> r = sh ? segment_row(a, sd, s, bq) : uniform_row(a, bq);
+        const T qx = a.q[bq * 3 + 0], qy = a.q[bq * 3 + 1], qz = a.q[bq * 3 + 2];
+        for (int k = kl; k < r.K; k += lpq) {
+          const int64_t e = r.e0 + k;
+          const int64_t idx = a.idxs[e];
+          T c = T(0);
+          if (idx >= 0 && idx < r.P) {
+            c = sg0 * a.frowsum[r.pbase + idx];
+            add_dq(a, r.recb + idx * kRecLen, qx, qy, qz, e, c, acc);
+          }
+          if (a.coef_out) a.coef_out[e] = c;
         }
-        if (a.coef_out) a.coef_out[e] = c;
       }
-    }
 #pragma unroll
-    for (int mm = 0; mm < 3; ++mm)
-      for (int o = lpq >> 1; o >= 1; o >>= 1) acc[mm] += __shfl_xor_sync(0xffffffffu, acc[mm], o);
-    if (bq < BQ && kl == 0 && a.dq) {
-      a.dq[bq * 3 + 0] = acc[0];
-      a.dq[bq * 3 + 1] = acc[1];
-      a.dq[bq * 3 + 2] = acc[2];
+      for (int mm = 0; mm < 3; ++mm)
+        for (int o = lpq >> 1; o >= 1; o >>= 1) acc[mm] += __shfl_xor_sync(0xffffffffu, acc[mm], o);
+      if (bq < BQ && kl == 0 && a.dq) {
+        a.dq[bq * 3 + 0] = acc[0];
+        a.dq[bq * 3 + 1] = acc[1];
+        a.dq[bq * 3 + 2] = acc[2];
+      }
     }
   }
 }
 
-// First-order query side: one warp per query.  For each group of 8
-// neighbours the lanes sweep the feature columns (coalesced rows of f, all
-// 8 rows in flight), then a reduce-scatter leaves c_k = gfo[q] . f[idx_k] of
-// neighbour k0 + (lane >> 2) in lanes 4m..4m+3; the first lane of each quad
-// does that neighbour's geometry.  dq = sum_k -2 c_k w_k v_k.
+// 16-byte column groups of f and grad_f_out rows (C values), or single values.
+template <typename T, bool VEC>
+struct ColGroup {
+  using type = typename Group16<T>::type;
+  static constexpr int C = 16 / sizeof(T);
+};
 template <typename T>
-__global__ void __launch_bounds__(256, 3) query_order1_kernel(QueryParams<T> a) {
-  constexpr int NG = 8;
-  const int lane = threadIdx.x & 31;
-  const int F = a.F;
+struct ColGroup<T, false> {
+  using type = T;
+  static constexpr int C = 1;
+};
+__device__ __forceinline__ float dot_group(const float4& a, const float4& b, float s) {
+  return __fmaf_rn(a.w, b.w, __fmaf_rn(a.z, b.z, __fmaf_rn(a.y, b.y, __fmaf_rn(a.x, b.x, s))));
+}
+__device__ __forceinline__ double dot_group(const double2& a, const double2& b, double s) {
+  return __fma_rn(a.y, b.y, __fma_rn(a.x, b.x, s));
+}
+template <typename T>
+__device__ __forceinline__ T dot_group(T a, T b, T s) {
+  return fma_rn(a, b, s);
+}
+__device__ __forceinline__ void fill_group(float4& g, float v) { g = make_float4(v, v, v, v); }
+__device__ __forceinline__ void fill_group(double2& g, double v) { g = make_double2(v, v); }
+template <typename T>
+__device__ __forceinline__ void fill_group(T& g, T v) {
+  g = v;
+}
+template <typename T>
+__device__ __forceinline__ void fma_group(T v, T w, T (&acc)[1]) {
+  acc[0] = fma_rn(v, w, acc[0]);
+}
+template <typename V, typename T, int C>
+__device__ __forceinline__ V to_group(const T (&a)[C]) {
+  if constexpr (C == 1) return a[0];
+  else return group_of(a);
+}
+
+// First-order query side: G lanes per query (16 for up to 64 column groups'
+// worth of a half-warp, else 32), so a warp serves one or two.  For each 16
+// neighbours the lanes sweep the feature columns, 16 bytes each where the rows
+// allow, four rows in flight (eight of single columns); a reduce-scatter then leaves c_k = gfo[q] .
+// f[idx_k] of neighbour k0 + l in lane l, which does that neighbour's geometry.
+// dq = sum_k -2 c_k w_k v_k.
+//
+// Bound by the gathered feature rows (L2): one query per warp with 4-byte loads
+// took 37 us at B = 2, Q = 12288, K = 16, F = 64 and now takes 20 (26 with eight
+// rows in flight, which spills at three CTAs per SM).
+template <typename T, int G, bool VEC>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) query_order1_kernel(QueryParams<T> a) {
+  using V = typename ColGroup<T, VEC>::type;
+  constexpr int C = ColGroup<T, VEC>::C, NK = 16, RB = VEC ? 4 : 8;  // neighbours a turn, rows in flight
+  const int lane = threadIdx.x & 31, gl = lane % G;
   const SegHeader* sh = static_cast<const SegHeader*>(a.segs);
   if (sh && *a.status) return;
   const int64_t BQ = sh ? sh->grad_rows : (int64_t)a.B * a.Q;
@@ -586,89 +648,76 @@ __global__ void __launch_bounds__(256, 3) query_order1_kernel(QueryParams<T> a) 
     query_order1_scalar(a, sh, BQ);
     return;
   }
+  constexpr int N = 32 / G;  // queries of the warp
+  const int cols = a.F / C;
   const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = (gridDim.x * (int64_t)blockDim.x) >> 5;
-  for (int64_t bq = gw; bq < BQ; bq += nw) {
-    // the query's cloud: records, features, sizes and first entry
-    int K, P;
-    int64_t e0;
-    const T* recb;
-    const T* fb;
-    if (sh) {
-      const SegDesc* sd = seg_descs(a.segs);
-      const SegDesc g = sd[seg_of_row(sd, sh->nseg, bq)];
-      const CloudDesc c = cloud_descs(a.cs)[g.cloud];
-      K = g.K;
-      P = c.P;
-      e0 = g.e_off + (bq - g.q_off) * K;
-      recb = reinterpret_cast<const T*>(a.cs + reinterpret_cast<const CloudSetHeader*>(a.cs)->rec_off) +
-             c.p_off * kRecLen;
-      fb = a.f + c.p_off * F;
-    } else {
-      const int64_t b = bq / a.Q;
-      K = a.K;
-      P = a.P;
-      e0 = bq * K;
-      recb = a.rec + b * a.P * kRecLen;
-      fb = a.f + b * a.P * F;
-    }
+  for (int64_t base = gw * N; base < BQ; base += nw * N) {
+    const bool live = base + lane / G < BQ;
+    const int64_t bq = live ? base + lane / G : BQ - 1;
+    const SegDesc* sd = sh ? seg_descs(a.segs) : nullptr;
+    const QueryRow<T> r = sh ? segment_row(a, sd, seg_of_row(sd, sh->nseg, bq), bq) : uniform_row(a, bq);
     const T qx = a.q[bq * 3 + 0], qy = a.q[bq * 3 + 1], qz = a.q[bq * 3 + 2];
-    const T* grow = a.gfo ? a.gfo + bq * F : nullptr;
+    const V* grow = a.gfo ? reinterpret_cast<const V*>(a.gfo + bq * a.F) : nullptr;
+    const V* frow = reinterpret_cast<const V*>(r.fb);
     T acc[3] = {T(0), T(0), T(0)};
-    for (int k0 = 0; k0 < K; k0 += NG) {
-      const int nk = min(NG, K - k0);
-      int ik[NG];  // neighbour point index within the batch, -1 if none
+    // the two queries of a warp may differ in K (segments): both take every turn
+    int most = r.K;
+    if (N > 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, 16));
+    for (int k0 = 0; k0 < most; k0 += NK) {
+      const int km = k0 + (gl & (NK - 1));  // this lane's neighbour
+      const int64_t idx = km < r.K ? a.idxs[r.e0 + km] : -1;
+      const int mine = (idx >= 0 && idx < r.P) ? (int)idx : -1;
+      T part[NK];
 #pragma unroll
-      for (int kk = 0; kk < NG; ++kk) {
-        const int64_t idx = kk < nk ? a.idxs[e0 + k0 + kk] : -1;
-        ik[kk] = (idx >= 0 && idx < P) ? (int)idx : -1;
+      for (int kk = 0; kk < NK; ++kk) part[kk] = T(0);
+      for (int cb = 0; cb < cols; cb += G) {  // warp-uniform: the shuffles need every lane
+        const int c = cb + gl;
+        const bool col = c < cols;
+        V g{};
+        if (col) {
+          if (grow) g = grow[c];
+          else fill_group(g, T(1));
+        }
+#pragma unroll
+        for (int kb = 0; kb < NK; kb += RB) {
+          if (k0 + kb < most) {
+            V v[RB];
+            int ik[RB];
+#pragma unroll
+            for (int u = 0; u < RB; ++u) {
+              ik[u] = __shfl_sync(0xffffffffu, mine, kb + u, G);
+              if (col && ik[u] >= 0) v[u] = __ldg(frow + (int64_t)ik[u] * cols + c);
+            }
+#pragma unroll
+            for (int u = 0; u < RB; ++u)
+              if (col && ik[u] >= 0) part[kb + u] = dot_group(g, v[u], part[kb + u]);
+          }
+        }
       }
-      T part[NG];
+      // reduce-scatter: 16 values over 16 lanes -> lane l holds value l
 #pragma unroll
-      for (int kk = 0; kk < NG; ++kk) part[kk] = T(0);
-      for (int c = lane; c < F; c += 32) {
-        const T g = grow ? grow[c] : T(1);
-#pragma unroll
-        for (int kk = 0; kk < NG; ++kk)
-          if (ik[kk] >= 0) part[kk] = fma_rn(g, fb[(int64_t)ik[kk] * F + c], part[kk]);
-      }
-      // reduce-scatter: 8 values over 32 lanes -> lane holds value (lane >> 2) & 7
-#pragma unroll
-      for (int h = NG / 2, m = 16; h >= 1; h >>= 1, m >>= 1) {
-        const bool upper = (lane & m) != 0;
+      for (int h = NK / 2; h >= 1; h >>= 1) {
+        const bool upper = (lane & h) != 0;
 #pragma unroll
         for (int i = 0; i < h; ++i) {
           const T send = upper ? part[i] : part[i + h];
           const T keep = upper ? part[i + h] : part[i];
-          part[i] = keep + __shfl_xor_sync(0xffffffffu, send, m);
+          part[i] = keep + __shfl_xor_sync(0xffffffffu, send, h);
         }
       }
-      T c_own = part[0] + __shfl_xor_sync(0xffffffffu, part[0], 2);
-      c_own += __shfl_xor_sync(0xffffffffu, c_own, 1);
-      const int m_own = lane >> 2;
-      const int64_t e = e0 + k0 + m_own;
-      if ((lane & 3) == 0 && m_own < nk) {
-        if (a.coef_out) a.coef_out[e] = c_own;
-        const int64_t idx = a.idxs[e];
-        if (idx >= 0 && idx < P) {
-          T rr[kRecLen];
-          load_rec(recb + idx * kRecLen, rr);
-          const T* rec = rr;
-          Geo<T> geo;
-          geometry(qx, qy, qz, rec, geo);
-          const T w = a.w_in ? a.w_in[e] : geo.w;
-          const T sg[3] = {rec[kS0], rec[kS1], rec[kS2]};
-          T v[3];
-          rot_back(rec + kR00, sg, geo.u, v);
-          const T t = T(-2) * c_own * w;
-#pragma unroll
-          for (int mm = 0; mm < 3; ++mm) acc[mm] += t * v[mm];
-        }
+      if (G == 32) part[0] += __shfl_xor_sync(0xffffffffu, part[0], 16);
+      if (live && gl < NK && km < r.K) {
+        const int64_t e = r.e0 + km;
+        if (a.coef_out) a.coef_out[e] = part[0];
+        if (mine >= 0) add_dq(a, r.recb + (int64_t)mine * kRecLen, qx, qy, qz, e, part[0], acc);
       }
     }
 #pragma unroll
-    for (int mm = 0; mm < 3; ++mm) acc[mm] = warp_sum(acc[mm]);
-    if (lane == 0 && a.dq) {
+    for (int mm = 0; mm < 3; ++mm)
+#pragma unroll
+      for (int o = G / 2; o >= 1; o >>= 1) acc[mm] += __shfl_xor_sync(0xffffffffu, acc[mm], o);
+    if (live && gl == 0 && a.dq) {
       a.dq[bq * 3 + 0] = acc[0];
       a.dq[bq * 3 + 1] = acc[1];
       a.dq[bq * 3 + 2] = acc[2];
@@ -825,14 +874,34 @@ __global__ void __launch_bounds__(256) query_order2_kernel(QueryParams<T> a) {
   query_order2_body(a, blockIdx.x, gridDim.x);
 }
 
-// One warp per point row.  Lane j takes entry j of each 32-entry chunk of
-// the row for the per-entry geometry (15 point-side scalars, reduced over
-// the warp at the end); for df the warp then walks the chunk four entries at
-// a time with lanes spanning feature columns (NCOL per lane, coalesced gfo
-// rows, four rows in flight).  The entry order of a row is fixed (sorted),
-// so every sum has a fixed order.
-template <typename T, int ORDER, int NCOL>
-__device__ __forceinline__ void point_side_body(const PointParams<T>& a, int blk, int nblk) {
+// One entry of a point row: the query's offset, rotated offset, weight and
+// v = R^T diag(sigma) u, and for the second order its grad_grad_q.
+template <typename T, int ORDER>
+struct PointEntry {
+  Geo<T> geo;
+  T v[3], g[3], w;
+};
+template <typename T, int ORDER>
+__device__ __forceinline__ void point_entry(const PointParams<T>& a, const T (&pr)[kRecLen], int e, int64_t bq,
+                                            PointEntry<T, ORDER>& x) {
+  const T qx = a.q[bq * 3 + 0], qy = a.q[bq * 3 + 1], qz = a.q[bq * 3 + 2];
+  if (ORDER == 2)
+#pragma unroll
+    for (int m = 0; m < 3; ++m) x.g[m] = a.ggq[bq * 3 + m];
+  const T sg[3] = {pr[kS0], pr[kS1], pr[kS2]};
+  geometry(qx, qy, qz, pr, x.geo);
+  x.w = a.w_in ? a.w_in[e] : x.geo.w;
+  rot_back(pr + kR00, sg, x.geo.u, x.v);
+}
+
+// Point side, geometry: one warp per point row, lane j takes entry j of each
+// 32-entry chunk of the row and sums the 15 point-side scalars, reduced over
+// the warp at the end.  With a broadcast grad_f_out s this is the whole point
+// side: c = s * rowsum(f)[row] in every entry of the row, and df[i][c] = s *
+// sum_e wgt_e for every column.  The entry order of a row is fixed (sorted), so
+// every sum has a fixed order.
+template <typename T, int ORDER>
+__device__ __forceinline__ void point_geometry_body(const PointParams<T>& a, int blk, int nblk) {
   const int lane = threadIdx.x & 31;
   const int gw = (blk * blockDim.x + threadIdx.x) >> 5;
   const int nw = (nblk * blockDim.x) >> 5;
@@ -840,115 +909,62 @@ __device__ __forceinline__ void point_side_body(const PointParams<T>& a, int blk
   const int F = a.F, K = a.K;
   const int n_entries = a.B * a.Q * K;
   const bool want_geo = (a.needs & (KNNAG_NEED_DP | KNNAG_NEED_DSIGMA | KNNAG_NEED_DR)) != 0;
-  const bool want_df = (a.needs & KNNAG_NEED_DF) != 0;
+  const bool scalar_df = (a.needs & KNNAG_NEED_DF) != 0 && a.gfo_scalar;
   for (int row = gw; row < rows; row += nw) {
-    const T* rec = a.rec + (int64_t)row * kRecLen;
     T pr[kRecLen];
-#pragma unroll
-    for (int m = 0; m < kRecLen; ++m) pr[m] = rec[m];
+    load_rec(a.rec + (int64_t)row * kRecLen, pr);
     const T* r = pr + kR00;
     const T sg[3] = {pr[kS0], pr[kS1], pr[kS2]};
     const int start = a.rowptr[row], end = a.rowptr[row + 1];
-    T gp[3] = {T(0), T(0), T(0)}, gs[3] = {T(0), T(0), T(0)}, gR[9];
+    T gp[3] = {T(0), T(0), T(0)}, gs[3] = {T(0), T(0), T(0)}, gR[9], wsum = T(0), c_row = T(0);
 #pragma unroll
     for (int m = 0; m < 9; ++m) gR[m] = T(0);
-    // broadcast grad_f_out s: df[i][c] = s * sum_e wgt_e for every column
-    // (one pass, no gathers of grad_f_out rows); wsum is this lane's share
-    T wsum = T(0);
-    for (int c0 = 0; c0 == 0 || (want_df && !a.gfo_scalar && c0 < F); c0 += 32 * NCOL) {
-      T acc[NCOL];
+    if (a.gfo_scalar && want_geo && start < end) {
+      const int e = a.entries[start];
+      if (e >= 0 && e < n_entries) c_row = a.coef[e];
+    }
+    for (int j = start + lane; j < end; j += 32) {
+      const int e = a.entries[j];
+      if (e < 0 || e >= n_entries) continue;
+      PointEntry<T, ORDER> x;
+      point_entry<T, ORDER>(a, pr, e, e / K, x);
+      const T c = !want_geo ? T(0) : (a.gfo_scalar ? c_row : a.coef[e]);
+      const T cw = c * x.w;
+      if (ORDER == 1) {
+        wsum += x.w;
 #pragma unroll
-      for (int u = 0; u < NCOL; ++u) acc[u] = T(0);
-      for (int base = start; base < end; base += 32) {
-        const int j = base + lane;
-        int e = (j < end) ? a.entries[j] : -1;
-        const bool valid = e >= 0 && e < n_entries;
-        if (!valid) e = 0;
-        const int bq = e / K;
-        T wgt = T(0);
-        if (valid) {
-          const T qx = a.q[(int64_t)bq * 3 + 0], qy = a.q[(int64_t)bq * 3 + 1], qz = a.q[(int64_t)bq * 3 + 2];
-          Geo<T> geo;
-          geometry(qx, qy, qz, pr, geo);
-          const T w = a.w_in ? a.w_in[e] : geo.w;
-          T v[3];
-          rot_back(r, sg, geo.u, v);
-          const T c = (want_geo && c0 == 0) ? a.coef[e] : T(0);
-          if (ORDER == 1) {
-            wgt = w;
-            if (want_geo && c0 == 0) {
-              const T cw = c * w;
+        for (int m = 0; m < 3; ++m) gp[m] += T(2) * cw * x.v[m];
 #pragma unroll
-              for (int m = 0; m < 3; ++m) gp[m] += T(2) * cw * v[m];
+        for (int s2 = 0; s2 < 3; ++s2) {
+          gs[s2] -= cw * x.geo.u[s2] * x.geo.u[s2];
+          const T t = T(-2) * cw * sg[s2] * x.geo.u[s2];
 #pragma unroll
-              for (int s2 = 0; s2 < 3; ++s2) {
-                gs[s2] -= cw * geo.u[s2] * geo.u[s2];
-                const T t = T(-2) * cw * sg[s2] * geo.u[s2];
-#pragma unroll
-                for (int m = 0; m < 3; ++m) gR[3 * s2 + m] += t * geo.d[m];
-              }
-            }
-          } else {
-            const T g[3] = {a.ggq[(int64_t)bq * 3 + 0], a.ggq[(int64_t)bq * 3 + 1], a.ggq[(int64_t)bq * 3 + 2]};
-            const T A = g[0] * v[0] + g[1] * v[1] + g[2] * v[2];
-            wgt = T(-2) * w * A;
-            if (want_geo && c0 == 0) {
-              T rg[3];
-#pragma unroll
-              for (int s2 = 0; s2 < 3; ++s2) rg[s2] = r[3 * s2] * g[0] + r[3 * s2 + 1] * g[1] + r[3 * s2 + 2] * g[2];
-              const T cw = c * w;
-#pragma unroll
-              for (int m = 0; m < 3; ++m) {
-                const T mg = sg[0] * rg[0] * r[m] + sg[1] * rg[1] * r[3 + m] + sg[2] * rg[2] * r[6 + m];
-                gp[m] -= T(2) * cw * (T(2) * A * v[m] - mg);
-              }
-#pragma unroll
-              for (int s2 = 0; s2 < 3; ++s2) {
-                gs[s2] += T(2) * cw * geo.u[s2] * (geo.u[s2] * A - rg[s2]);
-                const T t = T(-2) * cw * sg[s2];
-#pragma unroll
-                for (int m = 0; m < 3; ++m)
-                  gR[3 * s2 + m] += t * (T(-2) * geo.u[s2] * geo.d[m] * A + geo.d[m] * rg[s2] + geo.u[s2] * g[m]);
-              }
-            }
-          }
+          for (int m = 0; m < 3; ++m) gR[3 * s2 + m] += t * x.geo.d[m];
         }
-        if (want_df && a.gfo_scalar) {
-          wsum += wgt;  // 0 for lanes without an entry
-        } else if (want_df) {
-          const int nvalid = min(32, end - base);
-          for (int j0 = 0; j0 < nvalid; j0 += 4) {
-            T val[4][NCOL], wj[4];
+      } else {
+        const T A = x.g[0] * x.v[0] + x.g[1] * x.v[1] + x.g[2] * x.v[2];
+        wsum += T(-2) * x.w * A;
+        T rg[3];
 #pragma unroll
-            for (int jj = 0; jj < 4; ++jj) {
-              const int src = min(j0 + jj, 31);
-              const int bqj = __shfl_sync(0xffffffffu, bq, src);
-              wj[jj] = (j0 + jj < nvalid) ? __shfl_sync(0xffffffffu, wgt, src) : T(0);
-              const T* grow = a.gfo + (int64_t)bqj * F;
+        for (int s2 = 0; s2 < 3; ++s2) rg[s2] = r[3 * s2] * x.g[0] + r[3 * s2 + 1] * x.g[1] + r[3 * s2 + 2] * x.g[2];
 #pragma unroll
-              for (int u = 0; u < NCOL; ++u) {
-                const int cc = c0 + lane + 32 * u;
-                val[jj][u] = (cc < F) ? grow[cc] : T(0);
-              }
-            }
+        for (int m = 0; m < 3; ++m) {
+          const T mg = sg[0] * rg[0] * r[m] + sg[1] * rg[1] * r[3 + m] + sg[2] * rg[2] * r[6 + m];
+          gp[m] -= T(2) * cw * (T(2) * A * x.v[m] - mg);
+        }
 #pragma unroll
-            for (int jj = 0; jj < 4; ++jj)
+        for (int s2 = 0; s2 < 3; ++s2) {
+          gs[s2] += T(2) * cw * x.geo.u[s2] * (x.geo.u[s2] * A - rg[s2]);
+          const T t = T(-2) * cw * sg[s2];
 #pragma unroll
-              for (int u = 0; u < NCOL; ++u)
-                if (j0 + jj < nvalid) acc[u] = fma_rn(wj[jj], val[jj][u], acc[u]);
-          }
+          for (int m = 0; m < 3; ++m)
+            gR[3 * s2 + m] += t * (T(-2) * x.geo.u[s2] * x.geo.d[m] * A + x.geo.d[m] * rg[s2] + x.geo.u[s2] * x.g[m]);
         }
       }
-      if (want_df && a.gfo_scalar) {
-        const T val = a.gfo[0] * warp_sum(wsum);
-        for (int cc = lane; cc < F; cc += 32) a.df[(int64_t)row * F + cc] = val;
-      } else if (want_df) {
-#pragma unroll
-        for (int u = 0; u < NCOL; ++u) {
-          const int cc = c0 + lane + 32 * u;
-          if (cc < F) a.df[(int64_t)row * F + cc] = acc[u];
-        }
-      }
+    }
+    if (scalar_df) {
+      const T val = a.gfo[0] * warp_sum(wsum);
+      for (int cc = lane; cc < F; cc += 32) a.df[(int64_t)row * F + cc] = val;
     }
     if (want_geo) {
       T vals[15];
@@ -973,21 +989,107 @@ __device__ __forceinline__ void point_side_body(const PointParams<T>& a, int blk
   }
 }
 
-template <typename T, int ORDER, int NCOL>
-__global__ void __launch_bounds__(256, 4) point_side_kernel(PointParams<T> a) {
-  point_side_body<T, ORDER, NCOL>(a, blockIdx.x, gridDim.x);
+// Point side, features: df[row] = sum_e wgt_e gfo[query of e], one warp per
+// point row.  Lane j computes entry j's weight of each 32-entry chunk; the warp
+// then walks the chunk with lanes spanning feature columns: G lanes per entry
+// (two entries side by side where 16 lanes hold the columns), 16 bytes each
+// where the rows allow, NV groups per lane, four entries in flight per half.
+template <typename T, int ORDER, int G, int NV, bool VEC>
+__device__ __forceinline__ void point_features_body(const PointParams<T>& a, int blk, int nblk) {
+  using V = typename ColGroup<T, VEC>::type;
+  constexpr int C = ColGroup<T, VEC>::C, H = 32 / G, RB = 4;
+  const int lane = threadIdx.x & 31, gl = lane % G, half = lane / G;
+  const int gw = (blk * blockDim.x + threadIdx.x) >> 5;
+  const int nw = (nblk * blockDim.x) >> 5;
+  const int rows = a.B * a.P;
+  const int F = a.F, K = a.K, cols = F / C;
+  const int n_entries = a.B * a.Q * K;
+  for (int row = gw; row < rows; row += nw) {
+    T pr[kRecLen];
+    load_rec(a.rec + (int64_t)row * kRecLen, pr);
+    const int start = a.rowptr[row], end = a.rowptr[row + 1];
+    for (int c0 = 0; c0 < cols; c0 += G * NV) {
+      T acc[NV][C];
+#pragma unroll
+      for (int u = 0; u < NV; ++u)
+#pragma unroll
+        for (int v = 0; v < C; ++v) acc[u][v] = T(0);
+      for (int base = start; base < end; base += 32) {
+        int bq = 0;
+        T wgt = T(0);
+        if (base + lane < end) {
+          const int e = a.entries[base + lane];
+          if (e >= 0 && e < n_entries) {
+            bq = e / K;
+            PointEntry<T, ORDER> x;
+            point_entry<T, ORDER>(a, pr, e, bq, x);
+            wgt = ORDER == 1 ? x.w : T(-2) * x.w * (x.g[0] * x.v[0] + x.g[1] * x.v[1] + x.g[2] * x.v[2]);
+          }
+        }
+        const int nvalid = min(32, end - base);
+        for (int j0 = 0; j0 < nvalid; j0 += RB * H) {
+          V val[RB][NV];
+          T wj[RB];
+#pragma unroll
+          for (int jj = 0; jj < RB; ++jj) {
+            const int src = j0 + jj * H + half;  // at most 31: 32 is a multiple of RB * H
+            const int bqj = __shfl_sync(0xffffffffu, bq, src);
+            wj[jj] = __shfl_sync(0xffffffffu, wgt, src);
+            const V* grow = reinterpret_cast<const V*>(a.gfo + (int64_t)bqj * F);
+#pragma unroll
+            for (int u = 0; u < NV; ++u) {
+              const int cc = c0 + gl + G * u;
+              if (src < nvalid && cc < cols) val[jj][u] = __ldg(grow + cc);
+            }
+          }
+#pragma unroll
+          for (int jj = 0; jj < RB; ++jj)
+#pragma unroll
+            for (int u = 0; u < NV; ++u)
+              if (j0 + jj * H + half < nvalid && c0 + gl + G * u < cols) fma_group(val[jj][u], wj[jj], acc[u]);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < NV; ++u) {
+        if (H == 2)
+#pragma unroll
+          for (int v = 0; v < C; ++v) acc[u][v] += __shfl_xor_sync(0xffffffffu, acc[u][v], 16);
+        const int cc = c0 + gl + G * u;
+        if (half == 0 && cc < cols) reinterpret_cast<V*>(a.df + (int64_t)row * F)[cc] = to_group<V>(acc[u]);
+      }
+    }
+  }
+}
+
+// The point side in one launch over two ranges of blocks: the first f_blocks
+// walk the feature rows, the rest sum the geometry.  A row's features are a
+// chain of dependent gathers (entries, queries, grad_f_out rows) and the
+// geometry needs many registers; apart, twice as many warps are in flight, each
+// with more rows of its own.  At B = 2, Q = 12288, P = 4096, K = 16, F = 64: 33
+// us with one warp doing both, 28 apart (31 with eight entries in flight per
+// half at four CTAs per SM, which spills).
+template <typename T, int ORDER, int G, int NV, bool VEC>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) point_side_kernel(PointParams<T> a, int f_blocks) {
+  if ((int)blockIdx.x < f_blocks)
+    point_features_body<T, ORDER, G, NV, VEC>(a, blockIdx.x, f_blocks);
+  else
+    point_geometry_body<T, ORDER>(a, blockIdx.x - f_blocks, gridDim.x - f_blocks);
 }
 
 // The second-order query side and point side in one launch: they read the
 // same inputs (ggq, coef, records) and write disjoint outputs, so the first
-// q_blocks CTAs run the query side and the rest the point side, side by side
-// instead of one after the other.
-template <typename T, int NCOL>
-__global__ void __launch_bounds__(256, 3) order2_fused_kernel(QueryParams<T> qa, PointParams<T> pa, int q_blocks) {
-  if ((int)blockIdx.x < q_blocks)
+// q_blocks CTAs run the query side, the next f_blocks the point features and
+// the rest the point geometry, side by side instead of one after the other.
+template <typename T, int G, int NV, bool VEC>
+__global__ void __launch_bounds__(256, 4) order2_fused_kernel(QueryParams<T> qa, PointParams<T> pa, int q_blocks,
+                                                              int f_blocks) {
+  const int blk = (int)blockIdx.x - q_blocks;
+  if (blk < 0)
     query_order2_body(qa, blockIdx.x, q_blocks);
+  else if (blk < f_blocks)
+    point_features_body<T, 2, G, NV, VEC>(pa, blk, f_blocks);
   else
-    point_side_body<T, 2, NCOL>(pa, blockIdx.x - q_blocks, gridDim.x - q_blocks);
+    point_geometry_body<T, 2>(pa, blk - f_blocks, gridDim.x - q_blocks - f_blocks);
 }
 
 // ------------------------------------------------------------------ host
@@ -1012,15 +1114,32 @@ BwdLayout bwd_layout(int B, int Q, int P, int F, int K, int dtype) {
 
 namespace {
 
+// First-order query side of `rows` queries: 16-byte loads where f and
+// grad_f_out rows are multiples of 16 bytes at 16-byte addresses; two queries
+// per warp where 16 lanes cover their columns in as few passes as 32 would (or
+// with no columns to sweep), which halves the idle lanes of the geometry.
+template <typename T>
+int launch_order1(const QueryParams<T>& p, int64_t rows, cudaStream_t st) {
+  constexpr int C = 16 / sizeof(T);
+  const bool vec = p.F % C == 0 && (uintptr_t)p.f % 16 == 0 && (uintptr_t)p.gfo % 16 == 0;
+  const int cols = vec ? p.F / C : p.F;
+  const bool half = (cols + 15) / 16 <= 2 * ((cols + 31) / 32) && cols <= 64;
+  const unsigned grid = blocks_for((half ? (rows + 1) / 2 : rows) * 32, 256);
+  if (vec && half) query_order1_kernel<T, 16, true><<<grid, 256, 0, st>>>(p);
+  else if (vec) query_order1_kernel<T, 32, true><<<grid, 256, 0, st>>>(p);
+  else if (half) query_order1_kernel<T, 16, false><<<grid, 256, 0, st>>>(p);
+  else query_order1_kernel<T, 32, false><<<grid, 256, 0, st>>>(p);
+  note_launches(1);
+  return cudaGetLastError() == cudaSuccess ? KNNAG_OK : KNNAG_ERR_CUDA;
+}
+
 template <typename T>
 int launch_query(const QueryParams<T>& p, int order, cudaStream_t st) {
   NvtxRange range("knnag:query_side");
   const int64_t warps = (int64_t)p.B * p.Q;
   const unsigned grid = blocks_for(warps * 32, 256);
-  if (order == 1)
-    query_order1_kernel<T><<<grid, 256, 0, st>>>(p);
-  else
-    query_order2_kernel<T><<<grid, 256, 0, st>>>(p);
+  if (order == 1) return launch_order1<T>(p, warps, st);
+  query_order2_kernel<T><<<grid, 256, 0, st>>>(p);
   note_launches(1);
   return cudaGetLastError() == cudaSuccess ? KNNAG_OK : KNNAG_ERR_CUDA;
 }
@@ -1043,9 +1162,7 @@ int ragged_grad_q_impl(const char* cs, const void* segs, const float* q, const f
   p.dq = dq;
   p.cs = cs;
   p.segs = segs;
-  query_order1_kernel<float><<<blocks_for(cap_q * 32, 256), 256, 0, st>>>(p);
-  note_launches(1);
-  return cudaGetLastError() == cudaSuccess ? KNNAG_OK : KNNAG_ERR_CUDA;
+  return launch_order1<float>(p, cap_q, st);
 }
 
 int launch_row_sums(const void* f, int64_t rows, int F, int dtype, void* out, cudaStream_t st) {
@@ -1059,18 +1176,48 @@ int launch_row_sums(const void* f, int64_t rows, int F, int dtype, void* out, cu
 
 namespace {
 
+// How the feature rows are walked: 16-byte groups where grad_f_out and df rows
+// allow, else single columns; 16 lanes per entry (two entries side by side)
+// where they hold the row, else 32 with up to two groups (eight single columns)
+// per lane and as many passes as the row takes.  (37 single columns, B = 3,
+// Q = 5003: 17 us with 32 lanes, 24 with 16 lanes of up to four columns.)  0: no rows to walk.
+template <typename T>
+int point_columns(const PointParams<T>& p) {
+  constexpr int C = 16 / sizeof(T);
+  if (p.gfo_scalar || !(p.needs & KNNAG_NEED_DF) || p.F == 0) return 0;
+  const bool vec = p.F % C == 0 && (uintptr_t)p.gfo % 16 == 0 && (uintptr_t)p.df % 16 == 0;
+  const int cols = vec ? p.F / C : p.F;
+  if (vec) return cols <= 16 ? 1 : cols <= 32 ? 2 : 3;
+  return cols <= 16 ? 4 : cols <= 32 ? 5 : cols <= 64 ? 6 : 7;
+}
+
+// Launches KERNEL<..., G, NV, VEC> for a point_columns() code.
+#define KNN_POINT_DISPATCH(code, LAUNCH)     \
+  switch (code) {                            \
+    case 2: LAUNCH(32, 1, true); break;      \
+    case 3: LAUNCH(32, 2, true); break;      \
+    case 4: LAUNCH(16, 1, false); break;     \
+    case 5: LAUNCH(32, 1, false); break;     \
+    case 6: LAUNCH(32, 2, false); break;     \
+    case 7: LAUNCH(32, 8, false); break;     \
+    default: LAUNCH(16, 1, true); break;     \
+  }
+
+template <typename T>
+bool point_geometry_wanted(const PointParams<T>& p) {
+  return (p.needs & (KNNAG_NEED_DP | KNNAG_NEED_DSIGMA | KNNAG_NEED_DR)) != 0 ||
+         ((p.needs & KNNAG_NEED_DF) && p.gfo_scalar);
+}
+
 template <typename T, int ORDER>
 int launch_point_o(const PointParams<T>& p, cudaStream_t st) {
-  const int64_t rows = (int64_t)p.B * p.P;
-  const unsigned grid = blocks_for(rows * 32, 256);
-  if (p.F <= 32)
-    point_side_kernel<T, ORDER, 1><<<grid, 256, 0, st>>>(p);
-  else if (p.F <= 64)
-    point_side_kernel<T, ORDER, 2><<<grid, 256, 0, st>>>(p);
-  else if (p.F <= 128)
-    point_side_kernel<T, ORDER, 4><<<grid, 256, 0, st>>>(p);
-  else
-    point_side_kernel<T, ORDER, 8><<<grid, 256, 0, st>>>(p);
+  const unsigned blocks = blocks_for((int64_t)p.B * p.P * 32, 256);
+  const int code = point_columns(p);
+  const unsigned fb = code ? blocks : 0, grid = fb + (point_geometry_wanted(p) ? blocks : 0);
+  if (!grid) return KNNAG_OK;
+#define KNN_LAUNCH(G, NV, VEC) point_side_kernel<T, ORDER, G, NV, VEC><<<grid, 256, 0, st>>>(p, (int)fb)
+  KNN_POINT_DISPATCH(code, KNN_LAUNCH)
+#undef KNN_LAUNCH
   note_launches(1);
   return cudaGetLastError() == cudaSuccess ? KNNAG_OK : KNNAG_ERR_CUDA;
 }
@@ -1078,16 +1225,12 @@ int launch_point_o(const PointParams<T>& p, cudaStream_t st) {
 template <typename T>
 int launch_order2_fused(const QueryParams<T>& qa, const PointParams<T>& pa, cudaStream_t st) {
   const unsigned qb = blocks_for((int64_t)qa.B * qa.Q * 32, 256);
-  const unsigned pb = blocks_for((int64_t)pa.B * pa.P * 32, 256);
-  const unsigned grid = qb + pb;
-  if (pa.F <= 32)
-    order2_fused_kernel<T, 1><<<grid, 256, 0, st>>>(qa, pa, (int)qb);
-  else if (pa.F <= 64)
-    order2_fused_kernel<T, 2><<<grid, 256, 0, st>>>(qa, pa, (int)qb);
-  else if (pa.F <= 128)
-    order2_fused_kernel<T, 4><<<grid, 256, 0, st>>>(qa, pa, (int)qb);
-  else
-    order2_fused_kernel<T, 8><<<grid, 256, 0, st>>>(qa, pa, (int)qb);
+  const unsigned blocks = blocks_for((int64_t)pa.B * pa.P * 32, 256);
+  const int code = point_columns(pa);
+  const unsigned fb = code ? blocks : 0, grid = qb + fb + (point_geometry_wanted(pa) ? blocks : 0);
+#define KNN_LAUNCH(G, NV, VEC) order2_fused_kernel<T, G, NV, VEC><<<grid, 256, 0, st>>>(qa, pa, (int)qb, (int)fb)
+  KNN_POINT_DISPATCH(code, KNN_LAUNCH)
+#undef KNN_LAUNCH
   note_launches(1);
   return cudaGetLastError() == cudaSuccess ? KNNAG_OK : KNNAG_ERR_CUDA;
 }
@@ -1205,9 +1348,11 @@ int backward_t(const BwdArgs& x, cudaStream_t st) {
     pp.dsigma = (T*)x.dsigma;
     pp.dR = (T*)x.dR;
     pp.gfo_scalar = gfo_scalar;
-    if (query2_pending && sizeof(T) == 4) {  // FP64 keeps separate launches (the fused one spills)
-      NvtxRange r2("knnag:query_side");
-      return launch_order2_fused<T>(qp, pp, st);
+    if constexpr (sizeof(T) == 4) {  // FP64 keeps separate launches (the fused one spills)
+      if (query2_pending) {
+        NvtxRange r2("knnag:query_side");
+        return launch_order2_fused<T>(qp, pp, st);
+      }
     }
     if (query2_pending && (rc = launch_query<T>(qp, 2, st))) return rc;
     rc = (x.order == 1) ? launch_point_o<T, 1>(pp, st) : launch_point_o<T, 2>(pp, st);

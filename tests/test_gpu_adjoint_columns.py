@@ -1,0 +1,45 @@
+"""The adjoint kernels at every way their feature rows are walked: 16-byte
+groups and single columns, 16 and 32 lanes per row, one pass and several, K on
+both sides of 16 and 32.
+
+The oracle is FP64 autograd at the same neighbours.  Tolerance: every output is
+a sum of products of FP32 factors, each with at most 40 roundings (keys 20,
+__expf about 4, the rest of the entry's geometry 16) and n terms added in FP32;
+relative to the sum of the terms' magnitudes that is (40 + n) 2^-24, with n at
+most F (dot products), K and the longest point row, here below 1700 in all, so
+1.1e-4 of the output's largest value bounds what cancellation leaves; the
+repository's bar for gradients, 1e-4, is used."""
+import pytest
+import torch
+
+import oracle as O
+from conftest import rel_err
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda:0")
+
+
+@pytest.mark.parametrize("F", [1, 15, 16, 33, 37, 64, 65, 68, 128, 132, 256, 300, 516])
+@pytest.mark.parametrize("K,dtype", [(5, torch.float32), (17, torch.float32), (40, torch.float32),
+                                     (9, torch.float64)])
+def test_both_orders_match_fp64_autograd(F, K, dtype):
+    from cuda_knn_aggregate import knn_aggregate_aniso, workloads as W
+
+    _, t = W.make("small", B=2, Q=61, P=150, F=F, K=K, seed=1000 * K + F, dtype=dtype)
+    x = [a.to(DEV).requires_grad_(True) for a in t]
+    g = torch.Generator().manual_seed(F)
+    gfo = torch.randn(2, 61, F, generator=g, dtype=torch.float64)
+    ggq = torch.randn(2, 61, 3, generator=g, dtype=torch.float64)
+    gfo_d = gfo.to(DEV, dtype).requires_grad_(True)
+    f_out, _, _, idxs = knn_aggregate_aniso(*x, K)
+    first = torch.autograd.grad(f_out, x, grad_outputs=gfo_d, create_graph=True)
+    second = torch.autograd.grad(first[0], [gfo_d] + x, grad_outputs=ggq.to(DEV, dtype))
+
+    y = [a.double().requires_grad_(True) for a in t]
+    gfo.requires_grad_(True)
+    fo, _ = O.aggregate64(*y, idxs.cpu())
+    want = torch.autograd.grad(fo, y, grad_outputs=gfo, create_graph=True)
+    want2 = torch.autograd.grad(want[0], [gfo] + y, grad_outputs=ggq)
+    tol = 1e-4 if dtype == torch.float32 else 1e-10
+    for a, b in zip(list(first) + list(second), list(want) + list(want2)):
+        assert rel_err(a.detach().cpu().numpy(), b.detach().numpy()) < tol
