@@ -28,6 +28,9 @@
 
 namespace knnag {
 
+// Rows up to which the fill scans the counts itself (64 KB of shared memory).
+constexpr size_t kFillScanRows = 16384;
+
 AdjLayout adj_layout(int B, int Q, int P, int K) {
   AdjLayout L{};
   const size_t n_rows = (size_t)B * P;
@@ -41,13 +44,20 @@ AdjLayout adj_layout(int B, int Q, int P, int K) {
   off += align256(n * 4);
   L.entries = off;
   off += align256(n * 4);
+  L.fill = off;
+  if (n_rows <= kFillScanRows) off += align256(n_rows * 4);
   L.total = off;
   return L;
 }
 
 // ----------------------------------------------------------------- CSR
 
-__global__ void adj_count_kernel(const int64_t* __restrict__ idxs, int n, int qk, int P, int* __restrict__ count) {
+// Counts the entries of every row; also zeroes the fused fill's cursors
+// (`rows` of them; none when cursor is null).
+__global__ void adj_count_kernel(const int64_t* __restrict__ idxs, int n, int qk, int P, int* __restrict__ count,
+                                 int* __restrict__ cursor, int rows) {
+  if (cursor)
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += gridDim.x * blockDim.x) cursor[r] = 0;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
     const int64_t idx = idxs[e];
     if (idx < 0 || idx >= P) continue;  // not a point index: no row holds it
@@ -232,6 +242,60 @@ __global__ void adj_fill_kernel(const int64_t* __restrict__ idxs, int n, int qk,
   }
 }
 
+// The scan and the fill in one launch, for at most kFillScanRows rows: every
+// CTA scans the counts into shared memory itself (read from L2) and fills its
+// share; the first also writes rowptr.  `cursor` (zeroed beforehand) ranks a
+// row's entries.  Two launches, the one-CTA scan first, took 18 us
+// at 8192 rows and 393216 entries and 14 at 4096 rows and 196608; one takes 17
+// and 10.  The sort sets the cursors back to
+// zero, so that a graph's backward can run again on the same counts.
+__global__ void __launch_bounds__(1024) adj_fill_scan_kernel(const int64_t* __restrict__ idxs, int n, int qk, int P,
+                                                             const int* __restrict__ count, int rows,
+                                                             int* __restrict__ cursor, int* __restrict__ rowptr,
+                                                             int* __restrict__ unsorted) {
+  extern __shared__ int start[];  // [rows]
+  __shared__ int warp_sums[33];
+  const int tid = threadIdx.x, per = (rows + 1023) / 1024;
+  // coalesced in, then thread t takes rows [t per, (t + 1) per)
+  for (int i = tid; i < rows; i += 1024) start[i] = count[i];
+  __syncthreads();
+  const int i0 = min(rows, tid * per), i1 = min(rows, i0 + per);
+  int local = 0;
+  for (int i = i0; i < i1; ++i) local += start[i];
+  int total;
+  int run = block_exclusive_scan_1024(local, warp_sums, total);
+  for (int i = i0; i < i1; ++i) {
+    const int c = start[i];
+    start[i] = run;
+    run += c;
+  }
+  __syncthreads();
+  if (blockIdx.x == 0) {
+    for (int i = tid; i < rows; i += 1024) rowptr[i] = start[i];
+    if (tid == 0) rowptr[rows] = total;
+  }
+  constexpr int U = 4;  // entries in flight per thread
+  for (int64_t e0 = blockIdx.x * 1024 + tid; e0 < n; e0 += (int64_t)gridDim.x * 1024 * U) {
+    int row[U], rank[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t e = e0 + (int64_t)u * gridDim.x * 1024;
+      const int64_t idx = e < n ? idxs[e] : -1;
+      row[u] = idx >= 0 && idx < P ? ((int)e / qk) * P + (int)idx : -1;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (row[u] >= 0) rank[u] = atomicAdd(&cursor[row[u]], 1);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (row[u] >= 0) {
+        const int end = row[u] + 1 < rows ? start[row[u] + 1] : total;
+        if ((unsigned)rank[u] < (unsigned)(end - start[row[u]]))  // always: the row's count
+          unsorted[start[row[u]] + rank[u]] = (int)(e0 + (int64_t)u * gridDim.x * 1024);
+      }
+  }
+}
+
 // Bitonic sort, ascending, of the 32*V ints of a warp: element lane + 32*h
 // sits in x[h].  Stages with a partner distance below 32 exchange through
 // shuffles, the others inside the lane.
@@ -277,72 +341,103 @@ __device__ __forceinline__ void sort_row_regs(const int* src, int n, int* dst, i
 }
 
 constexpr int kAdjSortWarps = 8;      // warps per CTA of adj_sort_kernel
-constexpr int kAdjSmemSort = 1024;    // longest row sorted in shared memory
+constexpr int kAdjLongRow = 256;      // rows beyond this are sorted by the whole CTA
+constexpr int kAdjRun = 8192;         // in shared memory, runs of at most this many
 
-// Sort every row by entry id, one warp per row (ids in a row are distinct:
-// a query selects a point at most once).  Rows of up to 256 entries are
-// bitonic-sorted in registers, rows of up to 1024 in the warp's shared
-// memory; longer rows place each id at the number of smaller ids in the row.
-__global__ void __launch_bounds__(kAdjSortWarps * 32) adj_sort_kernel(const int* __restrict__ rowptr,
-                                                                     const int* __restrict__ unsorted, int n_rows,
-                                                                     int* __restrict__ entries) {
-  __shared__ int sbuf[kAdjSortWarps][kAdjSmemSort];
+// Ascending bitonic sort of n ints in shared memory by the CTA, padded to a
+// power of two.
+__device__ __forceinline__ void cta_bitonic_sort(int* sb, const int* src, int n) {
+  int n2 = 512;
+  while (n2 < n) n2 <<= 1;
+  for (int i = threadIdx.x; i < n2; i += blockDim.x) sb[i] = i < n ? src[i] : 0x7fffffff;
+  __syncthreads();
+  for (int k = 2; k <= n2; k <<= 1)
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      for (int t = threadIdx.x; t < n2 / 2; t += blockDim.x) {
+        const int i = 2 * t - (t & (j - 1)), ixj = i + j;  // the t-th pair at distance j
+        const int a = sb[i], b = sb[ixj];
+        if ((a > b) == ((i & k) == 0)) {
+          sb[i] = b;
+          sb[ixj] = a;
+        }
+      }
+      __syncthreads();
+    }
+}
+
+// Sort every row by entry id (ids in a row are distinct: a query selects a
+// point at most once).  Rows of up to 256 entries take one warp and its
+// registers.  Longer ones (few points near many queries) take the whole CTA
+// after its warps' rows: up to kAdjRun entries in shared memory, beyond that in
+// sorted runs of kAdjRun, each id then placed at its rank, the sum of its ranks
+// in all runs (written back over `unsorted`).  One warp per row whatever its
+// length took 50 us where one has about 1000 entries (1000 rows in
+// all; now 8 us), and time quadratic in the length beyond 1024.
+__global__ void __launch_bounds__(kAdjSortWarps * 32) adj_sort_kernel(const int* __restrict__ rowptr, int* unsorted,
+                                                                     int n_rows, int* __restrict__ entries,
+                                                                     int* __restrict__ cursor) {
+  __shared__ int sb[kAdjRun];
+  __shared__ int more;
   const int lane = threadIdx.x & 31;
-  int* sb = sbuf[threadIdx.x >> 5];
   const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nw = (gridDim.x * blockDim.x) >> 5;
+  if (threadIdx.x == 0) more = 0;
+  __syncthreads();
+  bool any = false;
   for (int r = gw; r < n_rows; r += nw) {
     const int start = rowptr[r];
     const int n = rowptr[r + 1] - start;
     const int* src = unsorted + start;
     int* dst = entries + start;
+    if (cursor && lane == 0) cursor[r] = 0;
     if (n <= 32) {
       sort_row_regs<1>(src, n, dst, lane);
     } else if (n <= 64) {
       sort_row_regs<2>(src, n, dst, lane);
     } else if (n <= 128) {
       sort_row_regs<4>(src, n, dst, lane);
-    } else if (n <= 256) {
+    } else if (n <= kAdjLongRow) {
       sort_row_regs<8>(src, n, dst, lane);
-    } else if (n <= kAdjSmemSort) {
-      int n2 = 512;
-      while (n2 < n) n2 <<= 1;
-      for (int i = lane; i < n2; i += 32) sb[i] = i < n ? src[i] : 0x7fffffff;
-      __syncwarp();
-      for (int k = 2; k <= n2; k <<= 1) {
-        for (int j = k >> 1; j > 0; j >>= 1) {
-          for (int i = lane; i < n2; i += 32) {
-            const int ixj = i ^ j;
-            if (ixj > i) {
-              const int a = sb[i], b = sb[ixj];
-              if ((a > b) == ((i & k) == 0)) {
-                sb[i] = b;
-                sb[ixj] = a;
-              }
-            }
-          }
-          __syncwarp();
-        }
-      }
-      for (int i = lane; i < n; i += 32) dst[i] = sb[i];
-      __syncwarp();
     } else {
-      for (int base = 0; base < n; base += 32) {
-        const int i = base + lane;
-        const int v = (i < n) ? src[i] : 0;
-        int rank = 0;
-        for (int jb = 0; jb < n; jb += 32) {
-          const int uj = (jb + lane < n) ? src[jb + lane] : 0x7fffffff;
-          const int lim = min(32, n - jb);
-          for (int jj = 0; jj < lim; ++jj) {
-            const int u = __shfl_sync(0xffffffffu, uj, jj);
-            rank += (u < v || (u == v && jb + jj < i)) ? 1 : 0;  // stable even if ids repeat
-          }
-        }
-        if (i < n) dst[rank] = v;
-      }
+      any = true;
     }
   }
+  if (any && lane == 0) more = 1;
+  __syncthreads();
+  if (!more) return;
+  // the CTA's long rows, in the same order (uniform control flow)
+  for (int r0 = blockIdx.x * kAdjSortWarps; r0 < n_rows; r0 += nw)
+    for (int r = r0; r < min(n_rows, r0 + kAdjSortWarps); ++r) {
+      const int start = rowptr[r];
+      const int n = rowptr[r + 1] - start;
+      if (n <= kAdjLongRow) continue;
+      int* src = unsorted + start;
+      int* dst = entries + start;
+      for (int run = 0; run < n; run += kAdjRun) {
+        const int m = min(kAdjRun, n - run);
+        cta_bitonic_sort(sb, src + run, m);
+        int* out = n <= kAdjRun ? dst : src + run;
+        for (int i = threadIdx.x; i < m; i += blockDim.x) out[i] = sb[i];
+        __syncthreads();
+      }
+      if (n <= kAdjRun) continue;
+      for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const int x = src[i], own = i / kAdjRun;
+        int rank = i - own * kAdjRun;
+        for (int run = 0, t = 0; run < n; run += kAdjRun, ++t) {
+          if (t == own) continue;
+          int lo = 0, hi = min(kAdjRun, n - run);
+          while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (src[run + mid] < x) lo = mid + 1;
+            else hi = mid;
+          }
+          rank += lo;
+        }
+        dst[rank] = x;
+      }
+      __syncthreads();
+    }
 }
 
 namespace {
@@ -387,18 +482,34 @@ int launch_build_adjacency(const int64_t* idxs, int B, int Q, int P, int K, void
   int* unsorted = reinterpret_cast<int*>(base + L.unsorted);
   int* entries = reinterpret_cast<int*>(base + L.entries);
   const int n = B * Q * K, rows = B * P, qk = Q * K;  // sizes checked < 2^31 by the caller
+  const bool fused = (size_t)rows <= kFillScanRows;
+  int* fill = fused ? reinterpret_cast<int*>(base + L.fill) : nullptr;
   if (!counted) {  // else the forward counted the entries per row already
     if (cudaMemsetAsync(cursor, 0, (size_t)rows * 4, st) != cudaSuccess) return KNNAG_ERR_CUDA;
-    adj_count_kernel<<<blocks_for(n, 256), 256, 0, st>>>(idxs, n, qk, P, cursor);
+    adj_count_kernel<<<blocks_for(n, 256), 256, 0, st>>>(idxs, n, qk, P, cursor, fill, rows);
     note_launches(1);
   }
-  const int rc = launch_exclusive_scan(cursor, rows, rowptr, st);
-  if (rc) return rc;
-  adj_fill_kernel<<<blocks_for(n, 256), 256, 0, st>>>(idxs, n, qk, P, rowptr, cursor, unsorted);
+  if (fused) {
+    const size_t smem = (size_t)rows * 4;
+    if (smem > 47 * 1024 && cudaFuncSetAttribute(adj_fill_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)(kFillScanRows * 4)) != cudaSuccess)
+      return KNNAG_ERR_CUDA;
+    int64_t blocks = ((int64_t)n + 2047) / 2048;  // two entries per thread or more: the scan is repeated by every CTA
+    if (blocks > sm_count()) blocks = sm_count();
+    if (blocks < 1) blocks = 1;
+    adj_fill_scan_kernel<<<(unsigned)blocks, 1024, smem, st>>>(idxs, n, qk, P, cursor, rows,
+                                                              fill, rowptr, unsorted);
+    note_launches(1);
+  } else {
+    const int rc = launch_exclusive_scan(cursor, rows, rowptr, st);
+    if (rc) return rc;
+    adj_fill_kernel<<<blocks_for(n, 256), 256, 0, st>>>(idxs, n, qk, P, rowptr, cursor, unsorted);
+    note_launches(1);
+  }
   const int sort_threads = kAdjSortWarps * 32;
-  adj_sort_kernel<<<blocks_for((int64_t)rows * 32, sort_threads), sort_threads, 0, st>>>(rowptr, unsorted, rows,
-                                                                                       entries);
-  note_launches(2);
+  adj_sort_kernel<<<blocks_for((int64_t)rows * 32, sort_threads), sort_threads, 0, st>>>(
+      rowptr, unsorted, rows, entries, fill);
+  note_launches(1);
   return cudaGetLastError() == cudaSuccess ? KNNAG_OK : KNNAG_ERR_CUDA;
 }
 
@@ -446,6 +557,7 @@ struct QueryParams {
   // broadcast grad_f_out: gfo points to one value s, and c = s * frowsum[i]
   // (frowsum = per-point sum over the columns of f)
   const T* frowsum;
+  int* zero_status;  // optional (uniform calls): the backward's two status words, zeroed by the first CTA
 };
 
 template <typename T>
@@ -464,8 +576,15 @@ struct PointParams {
   T* df;
   T* dsigma;
   T* dR;
+  int* zero_status;  // as QueryParams
   bool gfo_scalar;  // gfo points to one value broadcast over [B,Q,F]
 };
+
+// The status words of a backward call: no kernel of it latches anything, so
+// whichever runs first may clear them for a caller that reads them.
+__device__ __forceinline__ void zero_status_words(int* status) {
+  if (status && blockIdx.x == 0 && threadIdx.x < 2) status[threadIdx.x] = 0;
+}
 
 // v = R^T diag(sigma) u
 template <typename T>
@@ -643,6 +762,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) query_order1_kern
   const int lane = threadIdx.x & 31, gl = lane % G;
   const SegHeader* sh = static_cast<const SegHeader*>(a.segs);
   if (sh && *a.status) return;
+  zero_status_words(a.zero_status);
   const int64_t BQ = sh ? sh->grad_rows : (int64_t)a.B * a.Q;
   if (a.frowsum) {
     query_order1_scalar(a, sh, BQ);
@@ -871,6 +991,7 @@ __device__ __forceinline__ void query_order2_body(const QueryParams<T>& a, int b
 
 template <typename T>
 __global__ void __launch_bounds__(256) query_order2_kernel(QueryParams<T> a) {
+  zero_status_words(a.zero_status);
   query_order2_body(a, blockIdx.x, gridDim.x);
 }
 
@@ -1070,6 +1191,7 @@ __device__ __forceinline__ void point_features_body(const PointParams<T>& a, int
 // half at four CTAs per SM, which spills).
 template <typename T, int ORDER, int G, int NV, bool VEC>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) point_side_kernel(PointParams<T> a, int f_blocks) {
+  zero_status_words(a.zero_status);
   if ((int)blockIdx.x < f_blocks)
     point_features_body<T, ORDER, G, NV, VEC>(a, blockIdx.x, f_blocks);
   else
@@ -1083,6 +1205,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) point_side_kernel
 template <typename T, int G, int NV, bool VEC>
 __global__ void __launch_bounds__(256, 4) order2_fused_kernel(QueryParams<T> qa, PointParams<T> pa, int q_blocks,
                                                               int f_blocks) {
+  zero_status_words(qa.zero_status);
   const int blk = (int)blockIdx.x - q_blocks;
   if (blk < 0)
     query_order2_body(qa, blockIdx.x, q_blocks);
@@ -1241,7 +1364,7 @@ int backward_t(const BwdArgs& x, cudaStream_t st) {
   const BwdLayout L = bwd_layout(x.B, x.Q, x.P, x.F, x.K, x.dtype);
   char* ws = static_cast<char*>(x.workspace);
   int rc = KNNAG_OK;
-  if (cudaMemsetAsync(ws + L.status, 0, 8, st) != cudaSuccess) return KNNAG_ERR_CUDA;
+  int* status = reinterpret_cast<int*>(ws + L.status);
   const void* rec = x.points;
   if (!rec) {
     rc = launch_pack_points(x.p, x.sigma, x.R, x.B, x.P, x.dtype, ws + L.rec, st);
@@ -1284,6 +1407,7 @@ int backward_t(const BwdArgs& x, cudaStream_t st) {
   qp.P = x.P;
   qp.F = x.F;
   qp.K = x.K;
+  qp.zero_status = status;
 
   if (x.order == 1) {
     T* cdst = coef_out ? coef_out : (need_coef ? coef_ws : nullptr);
@@ -1348,6 +1472,7 @@ int backward_t(const BwdArgs& x, cudaStream_t st) {
     pp.dsigma = (T*)x.dsigma;
     pp.dR = (T*)x.dR;
     pp.gfo_scalar = gfo_scalar;
+    pp.zero_status = status;
     if constexpr (sizeof(T) == 4) {  // FP64 keeps separate launches (the fused one spills)
       if (query2_pending) {
         NvtxRange r2("knnag:query_side");

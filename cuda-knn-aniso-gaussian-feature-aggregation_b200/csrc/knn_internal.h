@@ -242,9 +242,10 @@ FwdLayout fwd_layout(int B, int Q, int P, int K, int dtype, bool own_rec, bool i
 // K > 32 only); L.total > bytes when neither fits.
 FwdLayout fwd_layout_in(int B, int Q, int P, int K, int dtype, bool own_rec, size_t bytes, bool* indexed);
 
-// Adjacency (CSR) layout: rowptr [B*P+1] | cursor [B*P] | unsorted [N] | entries [N].
+// Adjacency (CSR) layout: rowptr [B*P+1] | cursor [B*P] (the counts) | unsorted
+// [N] | entries [N] | fill [B*P] (the fused fill's cursors; few rows only).
 struct AdjLayout {
-  size_t rowptr, cursor, unsorted, entries, total;
+  size_t rowptr, cursor, unsorted, entries, fill, total;
 };
 AdjLayout adj_layout(int B, int Q, int P, int K);
 
@@ -298,7 +299,8 @@ int backward_impl(const BwdArgs& x, cudaStream_t st);
 // Packs the point records; block 0 also zeroes zero_words[0..n_zero) (a
 // call's status words) so no separate memset is needed.
 int launch_pack_points(const void* p, const void* sigma, const void* R, int B, int P, int dtype, void* rec,
-                       cudaStream_t st, int* zero_words = nullptr, int n_zero = 0, int* zero_rows = nullptr);
+                       cudaStream_t st, int* zero_words = nullptr, int n_zero = 0, int* zero_rows = nullptr,
+                       int64_t zero_rows2 = 0);
 // Chunks per batch element of the FP32 packing kernel that also bounds the
 // points: chunk c of element b writes its box to parts[(b * kBoundParts +
 // c) * 8 ...] (min xyz, max xyz), which the cell kernels reduce.
@@ -306,7 +308,7 @@ constexpr int kBoundParts = 32;
 template <typename T>
 int launch_pack_points_bounded(const T* p, const T* sigma, const T* R, const T* q, int B, int Q, int P, T* rec,
                                float* parts, float* pf, float* qf, cudaStream_t st, int* zero_words, int n_zero,
-                               int* zero_rows, int* zero_cells, int64_t n_cells);
+                               int* zero_rows, int64_t zero_rows2, int* zero_cells, int64_t n_cells);
 // adjacency: optional buffer (adj_layout) whose per-point entry counts the
 // forward writes, for launch_build_adjacency(..., counted = true)
 int forward_impl(const void* q, const void* p, const void* f, const void* sigma, const void* R, int B, int Q,

@@ -55,8 +55,8 @@ template <typename T>
 __global__ void __launch_bounds__(256) pack_points_bounded_kernel(
     const T* __restrict__ p, const T* __restrict__ sigma, const T* __restrict__ R, const T* __restrict__ q, int Q,
     int P, T* __restrict__ rec, float* __restrict__ parts, float* __restrict__ pf, float* __restrict__ qf,
-    int* __restrict__ zero_words, int n_zero, int* __restrict__ zero_rows, int* __restrict__ zero_cells,
-    int64_t n_cells) {
+    int* __restrict__ zero_words, int n_zero, int* __restrict__ zero_rows, int64_t zero_rows2,
+    int* __restrict__ zero_cells, int64_t n_cells) {
   __shared__ float red[6][8];
   const int c = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (c == 0 && b == 0 && tid < n_zero) zero_words[tid] = 0;
@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(256) pack_points_bounded_kernel(
   for (int k = i0 + tid; k < i1; k += blockDim.x) {
     const int64_t i = (int64_t)b * P + k;
     pack_one<T>(p, sigma, R, i, rec);
-    if (zero_rows) zero_rows[i] = 0;
+    if (zero_rows) zero_rows[i] = zero_rows[i + zero_rows2] = 0;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
       const float v = (float)p[i * 3 + a];
@@ -102,15 +102,17 @@ __global__ void __launch_bounds__(256) pack_points_bounded_kernel(
 
 // rec[(b*P+i)*16 + field]: -p, R (row-major), sigma, pad.
 // zero_rows (optional): one int per point zeroed too (the adjacency's
-// per-point entry counts the forward accumulates).
+// per-point entry counts the forward accumulates), and the one zero_rows2
+// further (its fill cursors; 0 where it has none).
 template <typename T>
 __global__ void pack_points_kernel(const T* __restrict__ p, const T* __restrict__ sigma,
                                    const T* __restrict__ R, int64_t n_points, T* __restrict__ rec,
-                                   int* __restrict__ zero_words, int n_zero, int* __restrict__ zero_rows) {
+                                   int* __restrict__ zero_words, int n_zero, int* __restrict__ zero_rows,
+                                   int64_t zero_rows2) {
   if (blockIdx.x == 0 && (int)threadIdx.x < n_zero) zero_words[threadIdx.x] = 0;  // the call's status words
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n_points;
        i += (int64_t)gridDim.x * blockDim.x) {
-    if (zero_rows) zero_rows[i] = 0;
+    if (zero_rows) zero_rows[i] = zero_rows[i + zero_rows2] = 0;
     pack_one<T>(p, sigma, R, i, rec);
   }
 }
@@ -735,26 +737,27 @@ FwdLayout fwd_layout_in(int B, int Q, int P, int K, int dtype, bool own_rec, siz
 template <typename T>
 int launch_pack_points_bounded(const T* p, const T* sigma, const T* R, const T* q, int B, int Q, int P, T* rec,
                                float* parts, float* pf, float* qf, cudaStream_t st, int* zero_words, int n_zero,
-                               int* zero_rows, int* zero_cells, int64_t n_cells) {
+                               int* zero_rows, int64_t zero_rows2, int* zero_cells, int64_t n_cells) {
   pack_points_bounded_kernel<T><<<dim3(kBoundParts, B), 256, 0, st>>>(p, sigma, R, q, Q, P, rec, parts, pf, qf,
-                                                                      zero_words, n_zero, zero_rows, zero_cells,
+                                                                      zero_words, n_zero, zero_rows, zero_rows2, zero_cells,
                                                                       n_cells);
   note_launches(1);
   return cudaGetLastError() == cudaSuccess ? KNNAG_OK : KNNAG_ERR_CUDA;
 }
 
 int launch_pack_points(const void* p, const void* sigma, const void* R, int B, int P, int dtype, void* rec,
-                       cudaStream_t st, int* zero_words, int n_zero, int* zero_rows) {
+                       cudaStream_t st, int* zero_words, int n_zero, int* zero_rows, int64_t zero_rows2) {
   int dev = 0;
   cudaGetDevice(&dev);
   const int64_t n = (int64_t)B * P;
   if (dtype == KNNAG_F64)
     pack_points_kernel<double><<<grid_for(n, 256, dev), 256, 0, st>>>(
-        (const double*)p, (const double*)sigma, (const double*)R, n, (double*)rec, zero_words, n_zero, zero_rows);
+        (const double*)p, (const double*)sigma, (const double*)R, n, (double*)rec, zero_words, n_zero, zero_rows,
+        zero_rows2);
   else
     pack_points_kernel<float><<<grid_for(n, 256, dev), 256, 0, st>>>((const float*)p, (const float*)sigma,
                                                                      (const float*)R, n, (float*)rec, zero_words,
-                                                                     n_zero, zero_rows);
+                                                                     n_zero, zero_rows, zero_rows2);
   note_launches(1);
   return cudaGetLastError() == cudaSuccess ? KNNAG_OK : KNNAG_ERR_CUDA;
 }
@@ -779,6 +782,8 @@ static int forward_indexed_t(const T* q, const T* p, const T* f, const T* sigma,
   float* pf = reinterpret_cast<float*>(ws + L.pf);
   float* qf = reinterpret_cast<float*>(ws + L.qf);
   const int ntile = L.P_pad / kTilePoints;
+  const AdjLayout AL = adj_layout(B, Q, P, K);
+  const int64_t fill_off = AL.fill < AL.total ? (int64_t)(AL.fill - AL.cursor) / 4 : 0;
   int rc;
   {
     NvtxRange r("knnag:pack_points");
@@ -787,7 +792,7 @@ static int forward_indexed_t(const T* q, const T* p, const T* f, const T* sigma,
     // scatter's cursors when the scan is folded into it) are zeroed, padding
     // between them included
     rc = launch_pack_points_bounded<T>(p, sigma, R, q, B, Q, P, rec, reinterpret_cast<float*>(ws + L.bounds), pf, qf, st,
-                                       status, 2, adj_count, reinterpret_cast<int*>(ws + L.cell_count),
+                                       status, 2, adj_count, fill_off, reinterpret_cast<int*>(ws + L.cell_count),
                                        (int64_t)(L.cell_offset - L.cell_count) / 4 + (2 * (int64_t)B << (3 * L.bits)) + 1);
   }
   if (rc) return rc;
@@ -887,10 +892,12 @@ static int forward_t(const T* q, const T* p, const T* f, const T* sigma, const T
     return forward_indexed_t<T>(q, p, f, sigma, R, B, Q, P, F, K, f_out, w_out, dists, idxs, rec, ws, L, adj_count, st);
   // the exact kernel serves every query; the packing zeroes the status words
   // and the adjacency's entry counts
+  const AdjLayout AL = adj_layout(B, Q, P, K);
+  const int64_t fill_off = AL.fill < AL.total ? (int64_t)(AL.fill - AL.cursor) / 4 : 0;
   int rc;
   {
     NvtxRange r("knnag:pack_points");
-    rc = launch_pack_points(p, sigma, R, B, P, dtype, rec, st, reinterpret_cast<int*>(ws + L.status), 2, adj_count);
+    rc = launch_pack_points(p, sigma, R, B, P, dtype, rec, st, reinterpret_cast<int*>(ws + L.status), 2, adj_count, fill_off);
   }
   if (rc) return rc;
   return forward_exact_all<T>(q, rec, f, B, Q, P, F, K, f_out, w_out, dists, idxs, adj_count, st);

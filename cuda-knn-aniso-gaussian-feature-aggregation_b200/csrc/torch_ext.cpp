@@ -381,7 +381,7 @@ torch::Tensor build_adjacency_forked(const torch::Tensor& idxs, int64_t P, at::c
 // rowptr [B*P+1] and sorted entry ids [B*Q*K] views of an adjacency buffer.
 std::vector<torch::Tensor> adjacency_views(torch::Tensor adj, int64_t B, int64_t Q, int64_t P, int64_t K) {
   const size_t rows = (size_t)B * P, n = (size_t)B * Q * K;
-  // layout: rowptr | cursor | unsorted | entries, each rounded up to 256 bytes
+  // layout: rowptr | cursor | unsorted | entries | ..., each rounded up to 256 bytes
   const size_t a0 = ((rows + 1) * 4 + 255) / 256 * 256;
   const size_t a1 = (rows * 4 + 255) / 256 * 256;
   const size_t a2 = (n * 4 + 255) / 256 * 256;
@@ -427,6 +427,10 @@ constexpr int64_t kPointBits = KNNAG_NEED_DP | KNNAG_NEED_DF | KNNAG_NEED_DSIGMA
 // order for point gradients, so the adjacency is built now, beside the
 // first-order kernels (never passed to the C ABI).
 constexpr int64_t kPrebuildAdjacency = int64_t(1) << 20;
+// Entries from which that build runs on a forked stream: the fork costs the host
+// about 10 us (a stream, two events), the build beside the query kernel saves
+// less than that on the GPU below a million entries.
+constexpr int64_t kForkEntries = int64_t(1) << 20;
 
 torch::Tensor or_placeholder(const torch::Tensor& t, const torch::Tensor& like) {
   return t.defined() ? t : torch::empty({0}, like.options());
@@ -450,9 +454,10 @@ struct AggBackwardFn : public torch::autograd::Function<AggBackwardFn> {
                                torch::Tensor points, torch::Tensor adj_counted, int64_t needs) {
     torch::Tensor adj;
     at::cuda::CUDAEvent join;
-    const bool forked = (needs & kPrebuildAdjacency) && !(needs & kPointBits);
+    const bool prebuild = (needs & kPrebuildAdjacency) && !(needs & kPointBits);
+    const bool forked = prebuild && idxs.numel() >= kForkEntries;
     needs &= ~kPrebuildAdjacency;
-    if (needs & kPointBits) {
+    if ((needs & kPointBits) || (prebuild && !forked)) {
       const c10::cuda::CUDAGuard guard(idxs.device());
       adj = build_adjacency_impl(idxs, p.size(1), adj_counted, stream_of(idxs));
     }
