@@ -117,6 +117,34 @@ __device__ __forceinline__ void load_rec(const double* p, double (&r)[kRecLen]) 
   }
 }
 
+// A record row (64 B / 128 B, 16-byte aligned) with 128-bit stores.
+__device__ __forceinline__ void store_rec(float* dst, const float (&v)[kRecLen]) {
+#pragma unroll
+  for (int m = 0; m < kRecLen; m += 4)
+    *reinterpret_cast<float4*>(dst + m) = make_float4(v[m], v[m + 1], v[m + 2], v[m + 3]);
+}
+__device__ __forceinline__ void store_rec(double* dst, const double (&v)[kRecLen]) {
+#pragma unroll
+  for (int m = 0; m < kRecLen; m += 2) *reinterpret_cast<double2*>(dst + m) = make_double2(v[m], v[m + 1]);
+}
+
+// One record from p, sigma, R (the shared body of the packing kernels).
+template <typename T>
+__device__ __forceinline__ void pack_one(const T* __restrict__ p, const T* __restrict__ sigma,
+                                         const T* __restrict__ R, int64_t i, T* __restrict__ rec) {
+  T v[kRecLen];
+  v[kNPX] = -p[i * 3 + 0];
+  v[kNPY] = -p[i * 3 + 1];
+  v[kNPZ] = -p[i * 3 + 2];
+#pragma unroll
+  for (int m = 0; m < 9; ++m) v[kR00 + m] = R[i * 9 + m];
+  v[kS0] = sigma[i * 3 + 0];
+  v[kS1] = sigma[i * 3 + 1];
+  v[kS2] = sigma[i * 3 + 2];
+  v[kRecPad] = T(0);
+  store_rec(rec + i * kRecLen, v);
+}
+
 // Key of query (qx,qy,qz) against a per-point record in global memory.
 template <typename T>
 __device__ __forceinline__ T key_rec(T qx, T qy, T qz, const T* rec_g) {

@@ -200,6 +200,14 @@ int point_bits(int P);
 template <typename T>
 int launch_spatial_index(const float* qf, const float* pf, const T* rec, int B, int Q, int P, int P_pad, char* ws,
                          const FwdLayout& L, cudaStream_t st, bool tc_ops = false);
+// The records and the whole index in one launch, for elements that one cluster
+// of CTAs holds (knn_spatial.cu); also zeroes the status words and the
+// adjacency's counts.
+bool index_in_one_launch(int B, int Q, int P);
+template <typename T>
+int launch_index_cluster(const T* p, const T* sigma, const T* R, const T* q, int B, int Q, int P, T* rec, char* ws,
+                         const FwdLayout& L, cudaStream_t st, int* zero_words, int n_zero, int* zero_rows,
+                         int64_t zero_rows2);
 int launch_exclusive_scan(int* count, int n, int* out, cudaStream_t st);
 int launch_cloudset_index(char* cs, const CloudSetHeader& h, const CloudDesc* cd_dev, int max_p, int max_ntile,
                           int* cnt, int* perm_p, cudaStream_t st);

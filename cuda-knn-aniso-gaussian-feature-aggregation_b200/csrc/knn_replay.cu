@@ -316,13 +316,9 @@ int launch_v(const ExactParams<T>& a, int max_points, cudaStream_t st) {
   static_assert(sizeof(ReplayShared<T, V>) <= 227 * 1024, "shared memory");
   int dev = 0;
   cudaGetDevice(&dev);
-  static bool allowed[64];
-  if (dev < 0 || dev >= 64 || !allowed[dev]) {
-    if (cudaFuncSetAttribute(replay_list_kernel<T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
-      return KNNAG_ERR_CUDA;
-    if (dev >= 0 && dev < 64) allowed[dev] = true;
-  }
+  if (cudaFuncSetAttribute(replay_list_kernel<T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+      cudaSuccess)
+    return KNNAG_ERR_CUDA;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(num_sms(dev) / ranks * ranks));  // flagged queries are few; clusters loop over them
   cfg.blockDim = dim3(32 * kReplayWarps);

@@ -16,34 +16,6 @@ namespace knnag {
 
 // ------------------------------------------------------------------ packing
 
-// A record row (64 B / 128 B, 16-byte aligned) with 128-bit stores.
-__device__ __forceinline__ void store_rec(float* dst, const float (&v)[kRecLen]) {
-#pragma unroll
-  for (int m = 0; m < kRecLen; m += 4)
-    *reinterpret_cast<float4*>(dst + m) = make_float4(v[m], v[m + 1], v[m + 2], v[m + 3]);
-}
-__device__ __forceinline__ void store_rec(double* dst, const double (&v)[kRecLen]) {
-#pragma unroll
-  for (int m = 0; m < kRecLen; m += 2) *reinterpret_cast<double2*>(dst + m) = make_double2(v[m], v[m + 1]);
-}
-
-// One record from p, sigma, R (the shared body of the packing kernels).
-template <typename T>
-__device__ __forceinline__ void pack_one(const T* __restrict__ p, const T* __restrict__ sigma,
-                                         const T* __restrict__ R, int64_t i, T* __restrict__ rec) {
-  T v[kRecLen];
-  v[kNPX] = -p[i * 3 + 0];
-  v[kNPY] = -p[i * 3 + 1];
-  v[kNPZ] = -p[i * 3 + 2];
-#pragma unroll
-  for (int m = 0; m < 9; ++m) v[kR00 + m] = R[i * 9 + m];
-  v[kS0] = sigma[i * 3 + 0];
-  v[kS1] = sigma[i * 3 + 1];
-  v[kS2] = sigma[i * 3 + 2];
-  v[kRecPad] = T(0);
-  store_rec(rec + i * kRecLen, v);
-}
-
 // Packing of the search path, grid (kBoundParts, B): CTA (c, b) packs
 // chunk c of batch element b's points, writes the chunk's bounding box to
 // parts (what the cell kernels reduce to the element's box), zeroes the
@@ -785,18 +757,6 @@ static int forward_indexed_t(const T* q, const T* p, const T* f, const T* sigma,
   const AdjLayout AL = adj_layout(B, Q, P, K);
   const int64_t fill_off = AL.fill < AL.total ? (int64_t)(AL.fill - AL.cursor) / 4 : 0;
   int rc;
-  {
-    NvtxRange r("knnag:pack_points");
-    // also zeroes the status words and the adjacency's entry counts, and
-    // bounds the points; cell counts and offsets (the offsets are the
-    // scatter's cursors when the scan is folded into it) are zeroed, padding
-    // between them included
-    rc = launch_pack_points_bounded<T>(p, sigma, R, q, B, Q, P, rec, reinterpret_cast<float*>(ws + L.bounds), pf, qf, st,
-                                       status, 2, adj_count, fill_off, reinterpret_cast<int*>(ws + L.cell_count),
-                                       (int64_t)(L.cell_offset - L.cell_count) / 4 + (2 * (int64_t)B << (3 * L.bits)) + 1);
-  }
-  if (rc) return rc;
-  if (ntile > kSearchMaxTiles) return KNNAG_ERR_TOO_LARGE;
   int dev = 0;
   cudaGetDevice(&dev);
   SearchParams sp{};
@@ -804,12 +764,29 @@ static int forward_indexed_t(const T* q, const T* p, const T* f, const T* sigma,
   int G = choose_warp_shape(B, Q, dev);
   if (sizeof(T) == 4 && K <= 32) G = choose_splits(B, Q, dev, sp.stall_visit >= 0);
   if (G == kShapeTensorFilter && !search_tc_fits(ntile)) G = choose_warp_shape(B, Q, dev);
-  {
+  if (ntile > kSearchMaxTiles) return KNNAG_ERR_TOO_LARGE;
+  if (G != kShapeTensorFilter && index_in_one_launch(B, Q, P)) {
+    NvtxRange r("knnag:spatial_index");
+    rc = launch_index_cluster<T>(p, sigma, R, q, B, Q, P, rec, ws, L, st, status, 2, adj_count, fill_off);
+    if (rc) return rc;
+  } else {
+    {
+      NvtxRange r("knnag:pack_points");
+      // also zeroes the status words and the adjacency's entry counts, and
+      // bounds the points; cell counts and offsets (the offsets are the
+      // scatter's cursors when the scan is folded into it) are zeroed, padding
+      // between them included
+      rc = launch_pack_points_bounded<T>(
+          p, sigma, R, q, B, Q, P, rec, reinterpret_cast<float*>(ws + L.bounds), pf, qf, st, status, 2, adj_count,
+          fill_off, reinterpret_cast<int*>(ws + L.cell_count),
+          (int64_t)(L.cell_offset - L.cell_count) / 4 + (2 * (int64_t)B << (3 * L.bits)) + 1);
+    }
+    if (rc) return rc;
     NvtxRange r("knnag:spatial_index");
     rc = launch_spatial_index<T>(sizeof(T) == 4 ? reinterpret_cast<const float*>(q) : qf, pf, rec, B, Q, P, L.P_pad, ws,
                                  L, st, G == kShapeTensorFilter);
+    if (rc) return rc;
   }
-  if (rc) return rc;
   const int vec = F < (1 << 28) && (F % (16 / (int)sizeof(T)) == 0) && ((uintptr_t)f % 16 == 0) && ((uintptr_t)f_out % 16 == 0);
   if (G == kShapeTensorFilter) {
     NvtxRange r("knnag:search_tc");

@@ -14,6 +14,7 @@
 // The search visits tiles nearest-first by this bound and stops when the
 // bound exceeds every query's threshold; the order of points inside a cell
 // (atomic scatter) never changes a result, only the work done.
+#include <cooperative_groups.h>
 #include <math.h>
 
 #include <algorithm>
@@ -406,109 +407,131 @@ __device__ __forceinline__ float round_up_f(float v) { return v; }
 __device__ __forceinline__ float round_down(double v) { return __double2float_rd(v); }
 __device__ __forceinline__ float round_up_f(double v) { return __double2float_ru(v); }
 
+// A record through L2 (load_rec's read-only path is for data that the running
+// kernel does not write).
+__device__ __forceinline__ void load_rec_cg(const float* p, float (&r)[kRecLen]) {
+#pragma unroll
+  for (int i = 0; i < kRecLen / 4; ++i) {
+    const float4 x = __ldcg(reinterpret_cast<const float4*>(p) + i);
+    r[4 * i + 0] = x.x;
+    r[4 * i + 1] = x.y;
+    r[4 * i + 2] = x.z;
+    r[4 * i + 3] = x.w;
+  }
+}
+__device__ __forceinline__ void load_rec_cg(const double* p, double (&r)[kRecLen]) {
+#pragma unroll
+  for (int i = 0; i < kRecLen / 2; ++i) {
+    const double2 x = __ldcg(reinterpret_cast<const double2*>(p) + i);
+    r[2 * i + 0] = x.x;
+    r[2 * i + 1] = x.y;
+  }
+}
+
+// Shared memory of one tile.
 template <typename T>
-__global__ void __launch_bounds__(kTilePoints) tile_info_kernel(const T* __restrict__ rec,
-                                                                const int* __restrict__ perm,
-                                                                const CloudDesc* __restrict__ cd, int P, int ntile,
-                                                                T* __restrict__ pairs, float* __restrict__ tinfo,
-                                                                float* __restrict__ tbox, int64_t tplane,
-                                                                float4* __restrict__ sbox, float* __restrict__ tcops,
-                                                                float* __restrict__ tcinfo) {
-  const TileGroup g = tile_group(cd, blockIdx.y, P, ntile);
-  const int t = blockIdx.x;
-  if (t >= g.ntile) return;
-  __shared__ float red[kTilePoints / 32][8];
-  __shared__ __align__(16) T tile[kTilePoints * kRecLen];
-  const int k = threadIdx.x, lane = k & 31, warp = k >> 5;
+struct TileScratch {
+  T tile[kTilePoints * kRecLen];
+  float red[kTilePoints / 32][8];
+};
+
+// Tile t of group g by 128 threads (k: 0..127; whole warps).  Every thread of
+// the CTA must call it (it has a CTA barrier); those of an inactive group only
+// take part in that.
+template <typename T>
+__device__ __forceinline__ void tile_info_body(bool active, const T* rec, const int* perm, TileGroup g,
+                                               int t, int k, TileScratch<T>& sm, T* __restrict__ pairs,
+                                               float* __restrict__ tinfo, float* __restrict__ tbox, int64_t tplane,
+                                               float4* __restrict__ sbox) {
+  const int lane = k & 31, warp = k >> 5;
   float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
   float mu = INFINITY;
   bool bad = false;
-  const int pos = t * kTilePoints + k;
-  T* slot = tile + k;  // field f of point k at slot[f * kTilePoints]
-  if (pos >= g.P) {
+  if (active) {
+    const int pos = t * kTilePoints + k;
+    T* slot = sm.tile + k;  // field f of point k at slot[f * kTilePoints]
+    if (pos >= g.P) {
 #pragma unroll
-    for (int m = 0; m < kRecLen; ++m)
-      slot[m * kTilePoints] = m == kRecPad ? index_bits<T>(-1)
-                                           : ((m == kS0 || m == kS1 || m == kS2) ? T(__int_as_float(0x7fc00000)) : T(0));
-  } else {
-    const int idx = perm[g.p0 + pos];
-    const T* r = rec + (g.p0 + idx) * kRecLen;
-    T v[kRecLen];
-    load_rec(r, v);
+      for (int m = 0; m < kRecLen; ++m)
+        slot[m * kTilePoints] = m == kRecPad ? index_bits<T>(-1)
+                                             : ((m == kS0 || m == kS1 || m == kS2) ? T(__int_as_float(0x7fc00000)) : T(0));
+    } else {
+      const int idx = __ldcg(perm + g.p0 + pos);
+      const T* r = rec + (g.p0 + idx) * kRecLen;
+      T v[kRecLen];
+      load_rec_cg(r, v);  // another CTA of the cluster may have just written it
 #pragma unroll
-    for (int m = 0; m < kRecLen; ++m) slot[m * kTilePoints] = m == kRecPad ? index_bits<T>(idx) : v[m];
+      for (int m = 0; m < kRecLen; ++m) slot[m * kTilePoints] = m == kRecPad ? index_bits<T>(idx) : v[m];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      const T c = -v[kNPX + a];
-      mn[a] = fminf(mn[a], round_down(c));
-      mx[a] = fmaxf(mx[a], round_up_f(c));
-      if (!isfinite(mn[a]) || !isfinite(mx[a])) bad = true;
-    }
-    double M[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-    double err = 0.0;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      const double s = v[kS0 + a];
-      if (!(s >= 0.0)) bad = true;  // a negative (or NaN) precision: keys may be negative
-      double rn = 0.0;
-#pragma unroll
-      for (int m = 0; m < 3; ++m) {
-        const double ra = v[kR00 + 3 * a + m];
-        rn += ra * ra;
-#pragma unroll
-        for (int n2 = 0; n2 < 3; ++n2) M[m][n2] += s * ra * (double)v[kR00 + 3 * a + n2];
+      for (int a = 0; a < 3; ++a) {
+        const T c = -v[kNPX + a];
+        mn[a] = fminf(mn[a], round_down(c));
+        mx[a] = fmaxf(mx[a], round_up_f(c));
+        if (!isfinite(mn[a]) || !isfinite(mx[a])) bad = true;
       }
-      err += fabs(s) * rn;
-    }
-    const double lam = sym3_min_eig(M[0][0], M[1][1], M[2][2], M[0][1], M[0][2], M[1][2]);
-    const double scale = fabs(M[0][0]) + fabs(M[1][1]) + fabs(M[2][2]) + fabs(M[0][1]) + fabs(M[0][2]) + fabs(M[1][2]);
-    const double m = lam - 1e-9 * scale - 1e-5 * err;
-    if (!isfinite(m)) bad = true;
-    mu = fminf(mu, (m > 0.0 && isfinite(m)) ? (float)(m * (1.0 - 1e-6)) : 0.0f);
-  }
+      double M[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+      double err = 0.0;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
+      for (int a = 0; a < 3; ++a) {
+        const double s = v[kS0 + a];
+        if (!(s >= 0.0)) bad = true;  // a negative (or NaN) precision: keys may be negative
+        double rn = 0.0;
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      mn[a] = fminf(mn[a], __shfl_xor_sync(0xffffffffu, mn[a], o));
-      mx[a] = fmaxf(mx[a], __shfl_xor_sync(0xffffffffu, mx[a], o));
+        for (int m = 0; m < 3; ++m) {
+          const double ra = v[kR00 + 3 * a + m];
+          rn += ra * ra;
+#pragma unroll
+          for (int n2 = 0; n2 < 3; ++n2) M[m][n2] += s * ra * (double)v[kR00 + 3 * a + n2];
+        }
+        err += fabs(s) * rn;
+      }
+      const double lam = sym3_min_eig(M[0][0], M[1][1], M[2][2], M[0][1], M[0][2], M[1][2]);
+      const double scale = fabs(M[0][0]) + fabs(M[1][1]) + fabs(M[2][2]) + fabs(M[0][1]) + fabs(M[0][2]) + fabs(M[1][2]);
+      const double m = lam - 1e-9 * scale - 1e-5 * err;
+      if (!isfinite(m)) bad = true;
+      mu = fminf(mu, (m > 0.0 && isfinite(m)) ? (float)(m * (1.0 - 1e-6)) : 0.0f);
     }
-    mu = fminf(mu, __shfl_xor_sync(0xffffffffu, mu, o));
-  }
-  bad = __any_sync(0xffffffffu, bad);
-  if (lane == 0) {
-    for (int a = 0; a < 3; ++a) {
-      red[warp][a] = mn[a];
-      red[warp][3 + a] = mx[a];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        mn[a] = fminf(mn[a], __shfl_xor_sync(0xffffffffu, mn[a], o));
+        mx[a] = fmaxf(mx[a], __shfl_xor_sync(0xffffffffu, mx[a], o));
+      }
+      mu = fminf(mu, __shfl_xor_sync(0xffffffffu, mu, o));
     }
-    red[warp][6] = mu;
-    red[warp][7] = bad ? 1.0f : 0.0f;
-    float* o = tinfo + (g.t0 + t) * kTinfoFloats + 8 * (1 + warp);  // this warp's sub-box
-    for (int a = 0; a < 3; ++a) {
-      o[a] = mn[a];
-      o[3 + a] = mx[a];
+    bad = __any_sync(0xffffffffu, bad);
+    if (lane == 0) {
+      for (int a = 0; a < 3; ++a) {
+        sm.red[warp][a] = mn[a];
+        sm.red[warp][3 + a] = mx[a];
+      }
+      sm.red[warp][6] = mu;
+      sm.red[warp][7] = bad ? 1.0f : 0.0f;
+      float* o = tinfo + (g.t0 + t) * kTinfoFloats + 8 * (1 + warp);  // this warp's sub-box
+      for (int a = 0; a < 3; ++a) {
+        o[a] = mn[a];
+        o[3 + a] = mx[a];
+      }
+      o[6] = bad ? -1.0f : mu;  // +inf: no points (the box is empty)
+      o[7] = 0.0f;
+      sbox[(g.t0 + t) * 8 + warp] = make_float4(mn[0], mn[1], mn[2], o[6]);
+      sbox[(g.t0 + t) * 8 + 4 + warp] = make_float4(mx[0], mx[1], mx[2], 0.f);
     }
-    o[6] = bad ? -1.0f : mu;  // +inf: no points (the box is empty)
-    o[7] = 0.0f;
-    sbox[(g.t0 + t) * 8 + warp] = make_float4(mn[0], mn[1], mn[2], o[6]);
-    sbox[(g.t0 + t) * 8 + 4 + warp] = make_float4(mx[0], mx[1], mx[2], 0.f);
   }
   __syncthreads();
-  {
-    const float4* src = reinterpret_cast<const float4*>(tile);
-    float4* dst = reinterpret_cast<float4*>(pairs + (g.t0 + t) * kTilePoints * kRecLen);
-    for (int i = k; i < (int)(kTilePoints * kRecLen * sizeof(T) / 16); i += kTilePoints) dst[i] = src[i];
-  }
-  if constexpr (sizeof(T) == 4)
-    if (tcops) tc_tile_operand(tile, red, k, pos < g.P, tcops + (g.t0 + t) * kTcOpsFloats, tcinfo + (g.t0 + t) * kTcInfoFloats);
+  if (!active) return;
+  const float4* src = reinterpret_cast<const float4*>(sm.tile);
+  float4* dst = reinterpret_cast<float4*>(pairs + (g.t0 + t) * kTilePoints * kRecLen);
+  for (int i = k; i < (int)(kTilePoints * kRecLen * sizeof(T) / 16); i += kTilePoints) dst[i] = src[i];
   if (k == 0) {
     for (int w = 1; w < kTilePoints / 32; ++w) {
       for (int a = 0; a < 3; ++a) {
-        mn[a] = fminf(mn[a], red[w][a]);
-        mx[a] = fmaxf(mx[a], red[w][3 + a]);
+        mn[a] = fminf(mn[a], sm.red[w][a]);
+        mx[a] = fmaxf(mx[a], sm.red[w][3 + a]);
       }
-      mu = fminf(mu, red[w][6]);
-      bad = bad || red[w][7] != 0.0f;
+      mu = fminf(mu, sm.red[w][6]);
+      bad = bad || sm.red[w][7] != 0.0f;
     }
     float* o = tinfo + (g.t0 + t) * kTinfoFloats;
     for (int a = 0; a < 3; ++a) {
@@ -519,6 +542,202 @@ __global__ void __launch_bounds__(kTilePoints) tile_info_kernel(const T* __restr
     o[7] = 0.0f;
     for (int m = 0; m < 7; ++m) tbox[m * tplane + g.t0 + t] = o[m];
   }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kTilePoints) tile_info_kernel(const T* __restrict__ rec,
+                                                                const int* __restrict__ perm,
+                                                                const CloudDesc* __restrict__ cd, int P, int ntile,
+                                                                T* __restrict__ pairs, float* __restrict__ tinfo,
+                                                                float* __restrict__ tbox, int64_t tplane,
+                                                                float4* __restrict__ sbox, float* __restrict__ tcops,
+                                                                float* __restrict__ tcinfo) {
+  const TileGroup g = tile_group(cd, blockIdx.y, P, ntile);
+  const int t = blockIdx.x, k = threadIdx.x;
+  if (t >= g.ntile) return;
+  __shared__ __align__(16) TileScratch<T> sm;
+  tile_info_body<T>(true, rec, perm, g, t, k, sm, pairs, tinfo, tbox, tplane, sbox);
+  if constexpr (sizeof(T) == 4)
+    if (tcops)
+      tc_tile_operand(sm.tile, sm.red, k, t * kTilePoints + k < g.P, tcops + (g.t0 + t) * kTcOpsFloats,
+                      tcinfo + (g.t0 + t) * kTcInfoFloats);
+}
+
+// ------------------------------------------------------ index in one launch
+//
+// The whole index of a small uniform call -- packed records, bounds, the
+// counting sort of points and queries, tiles -- by one cluster of
+// kIndexCtas CTAs per batch element: the steps that are launches of their own
+// below are separated by cluster barriers here.  For elements of up to 4096
+// points (the coarse grid's cells fit shared memory) and 32768 queries.
+// What bounds it: latency, a handful of dependent memory round trips.  The four
+// launches took 21 us at B = 2, Q = 1000, P = 500 and 26 us at B = 2, Q = 12288,
+// P = 4096, gaps included; one takes 13 and 20, and a whole forward call of the
+// first size went from 40 us to 33.
+constexpr int kIndexCtas = 8;
+constexpr int kIndexThreads = 1024;
+constexpr int kIndexPoints = 4096;
+constexpr int kIndexCells = 512;  // 8^spatial_bits(kIndexPoints)
+constexpr int kIndexElements = 16;
+constexpr int kIndexPerThread = 4;
+constexpr int kIndexQueries = kIndexCtas * kIndexThreads * kIndexPerThread;
+constexpr int kIndexTiles = kIndexPoints / kTilePoints / kIndexCtas;  // tiles of a CTA
+
+template <typename T>
+struct IndexShared {
+  TileScratch<T> tile[kIndexTiles];
+  float box[6];                        // of this CTA's points
+  float red[6][kIndexThreads / 32];
+  int count[2][kIndexCells];           // this CTA's points and queries per cell
+  int start[2][kIndexCells];           // where they go; then the cursors
+  int first[kIndexCells + 1];          // of the element's sorted points, per cell
+  int wsum[2][kIndexThreads / 32];
+};
+
+template <typename T>
+struct IndexParams {
+  const T *p, *sigma, *R, *q;
+  int Q, P, bits, ntile;
+  T* rec;
+  int *zero_words, n_zero;
+  int* zero_rows;  // as pack_points_bounded_kernel
+  int64_t zero_rows2;
+  int *perm_p, *perm_q, *seed;
+  T* pairs;
+  float *tinfo, *tbox;
+  int64_t tplane;
+  float4* sbox;
+};
+
+template <typename T>
+__global__ void __launch_bounds__(kIndexThreads) index_cluster_kernel(IndexParams<T> a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  IndexShared<T>& sm = *reinterpret_cast<IndexShared<T>*>(smem_raw);
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int rank = (int)cluster.block_rank();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t b = blockIdx.x / kIndexCtas;
+  const int cells = 1 << (3 * a.bits);
+  if (blockIdx.x == 0 && tid < a.n_zero) a.zero_words[tid] = 0;
+  static_assert(2 * kIndexCells == kIndexThreads, "a thread per cell of either kind");
+  sm.count[tid / kIndexCells][tid % kIndexCells] = 0;
+  // ---- this CTA's points: records, box
+  const int share = (a.P + kIndexCtas - 1) / kIndexCtas;  // at most kIndexThreads
+  const int pi = tid < share && rank * share + tid < a.P ? rank * share + tid : -1;
+  float xyz[3] = {0.f, 0.f, 0.f};
+  {
+    float v[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+    if (pi >= 0) {
+      const int64_t i = b * a.P + pi;
+      pack_one<T>(a.p, a.sigma, a.R, i, a.rec);
+      if (a.zero_rows) a.zero_rows[i] = a.zero_rows[i + a.zero_rows2] = 0;
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        xyz[m] = (float)a.p[i * 3 + m];
+        v[m] = fminf(v[m], xyz[m]);  // NaN leaves the box alone
+        v[3 + m] = fmaxf(v[3 + m], xyz[m]);
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int m = 0; m < 6; ++m) {
+        const float w = __shfl_xor_sync(0xffffffffu, v[m], o);
+        v[m] = m < 3 ? fminf(v[m], w) : fmaxf(v[m], w);
+      }
+    if (lane == 0)
+#pragma unroll
+      for (int m = 0; m < 6; ++m) sm.red[m][warp] = v[m];
+    __syncthreads();
+    if (warp < 6) {
+      float w = sm.red[warp][lane];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const float x = __shfl_xor_sync(0xffffffffu, w, o);
+        w = warp < 3 ? fminf(w, x) : fmaxf(w, x);
+      }
+      if (lane == 0) sm.box[warp] = w;
+    }
+  }
+  cluster.sync();
+  // ---- the element's box; cells of this CTA's points and queries
+  float box[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+  for (int r = 0; r < kIndexCtas; ++r) {
+    const float* o = cluster.map_shared_rank(sm.box, r);
+#pragma unroll
+    for (int m = 0; m < 6; ++m) box[m] = m < 3 ? fminf(box[m], o[m]) : fmaxf(box[m], o[m]);
+  }
+  int pcell = 0, qcell[kIndexPerThread];
+  if (pi >= 0) {
+    pcell = (int)cell_of(xyz[0], xyz[1], xyz[2], box, a.bits);
+    atomicAdd(&sm.count[0][pcell], 1);
+  }
+#pragma unroll
+  for (int u = 0; u < kIndexPerThread; ++u) {
+    const int qi = (u * kIndexCtas + rank) * kIndexThreads + tid;
+    qcell[u] = 0;
+    if (qi < a.Q) {
+      const T* v = a.q + (b * a.Q + qi) * 3;
+      qcell[u] = (int)cell_of((float)v[0], (float)v[1], (float)v[2], box, a.bits);
+      atomicAdd(&sm.count[1][qcell[u]], 1);
+    }
+  }
+  cluster.sync();
+  // ---- scan: thread c < 2 * kIndexCells takes cell c of the points or queries
+  {
+    const int kind = tid >= kIndexCells, c = tid - kind * kIndexCells;
+    int before = 0, total = 0;
+#pragma unroll
+    for (int r = 0; r < kIndexCtas; ++r) {
+      const int n = c < cells ? cluster.map_shared_rank(&sm, r)->count[kind][c] : 0;
+      if (r < rank) before += n;
+      total += n;
+    }
+    int incl = total;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int n = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += n;
+    }
+    if (lane == 31) sm.wsum[0][warp] = incl;
+    __syncthreads();
+    if (warp == 0) {  // 16 warps of points, 16 of queries
+      const int n = sm.wsum[0][lane];
+      int w = n;
+#pragma unroll
+      for (int o = 1; o < 16; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, w, o);
+        if ((lane & 15) >= o) w += x;
+      }
+      sm.wsum[1][lane] = w - n;
+    }
+    __syncthreads();
+    const int off = sm.wsum[1][warp] + incl - total;
+    sm.start[kind][c] = off + before;
+    if (kind == 0) {
+      sm.first[c] = off;
+      if (c == kIndexCells - 1) sm.first[kIndexCells] = off + total;
+    }
+  }
+  __syncthreads();
+  // ---- scatter
+  if (pi >= 0) a.perm_p[b * a.P + atomicAdd(&sm.start[0][pcell], 1)] = pi;
+#pragma unroll
+  for (int u = 0; u < kIndexPerThread; ++u) {
+    const int qi = (u * kIndexCtas + rank) * kIndexThreads + tid;
+    if (qi < a.Q) {
+      const int64_t pos = b * a.Q + atomicAdd(&sm.start[1][qcell[u]], 1);
+      a.perm_q[pos] = qi;
+      a.seed[pos] = (sm.first[qcell[u]] + sm.first[qcell[u] + 1]) >> 1;  // the middle of the cell's points
+    }
+  }
+  cluster.sync();
+  // ---- tiles: 128 threads each
+  const int slot = tid / kTilePoints, t = rank + slot * kIndexCtas;
+  const bool active = slot < kIndexTiles && t < a.ntile;
+  tile_info_body<T>(active, a.rec, a.perm_p, TileGroup{b * a.P, b * a.ntile, a.P, a.ntile}, t, tid % kTilePoints,
+                    sm.tile[slot < kIndexTiles ? slot : 0], a.pairs, a.tinfo, a.tbox, a.tplane, a.sbox);
 }
 
 // Boxes of groups of 32 tiles (warp blockIdx.x of batch element or cloud
@@ -626,6 +845,63 @@ template int launch_spatial_index<float>(const float*, const float*, const float
                                          const FwdLayout&, cudaStream_t, bool);
 template int launch_spatial_index<double>(const float*, const float*, const double*, int, int, int, int, char*,
                                           const FwdLayout&, cudaStream_t, bool);
+
+// Elements that a cluster's shared memory and registers hold, and no more of
+// them than run at the same time (8 CTAs of a whole SM each): past that the
+// separate launches, which split the work by points and queries, are as fast.
+bool index_in_one_launch(int B, int Q, int P) {
+  return P <= kIndexPoints && Q <= kIndexQueries && B <= kIndexElements;
+}
+
+template <typename T>
+int launch_index_cluster(const T* p, const T* sigma, const T* R, const T* q, int B, int Q, int P, T* rec, char* ws,
+                         const FwdLayout& L, cudaStream_t st, int* zero_words, int n_zero, int* zero_rows,
+                         int64_t zero_rows2) {
+  IndexParams<T> a{};
+  a.p = p;
+  a.sigma = sigma;
+  a.R = R;
+  a.q = q;
+  a.Q = Q;
+  a.P = P;
+  a.bits = L.bits;
+  a.ntile = L.P_pad / kTilePoints;
+  a.rec = rec;
+  a.zero_words = zero_words;
+  a.n_zero = n_zero;
+  a.zero_rows = zero_rows;
+  a.zero_rows2 = zero_rows2;
+  a.perm_p = reinterpret_cast<int*>(ws + L.perm_p);
+  a.perm_q = reinterpret_cast<int*>(ws + L.perm_q);
+  a.seed = reinterpret_cast<int*>(ws + L.qseed);
+  a.pairs = reinterpret_cast<T*>(ws + L.pairs);
+  a.tinfo = reinterpret_cast<float*>(ws + L.tinfo);
+  a.tbox = reinterpret_cast<float*>(ws + L.tbox);
+  a.tplane = (int64_t)B * a.ntile;
+  a.sbox = reinterpret_cast<float4*>(ws + L.sbox);
+  const size_t smem = sizeof(IndexShared<T>);
+  if (smem > 48 * 1024 && cudaFuncSetAttribute(index_cluster_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)smem) != cudaSuccess)
+    return KNNAG_ERR_CUDA;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)B * kIndexCtas);
+  cfg.blockDim = dim3(kIndexThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = kIndexCtas;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, index_cluster_kernel<T>, a) != cudaSuccess) return KNNAG_ERR_CUDA;
+  note_launches(1);
+  return cudaGetLastError() == cudaSuccess ? KNNAG_OK : KNNAG_ERR_CUDA;
+}
+template int launch_index_cluster<float>(const float*, const float*, const float*, const float*, int, int, int, float*,
+                                         char*, const FwdLayout&, cudaStream_t, int*, int, int*, int64_t);
+template int launch_index_cluster<double>(const double*, const double*, const double*, const double*, int, int, int,
+                                          double*, char*, const FwdLayout&, cudaStream_t, int*, int, int*, int64_t);
 
 // Cloud-set index: bounds, Hilbert order, sorted tiles and tile boxes of
 // every cloud (records already packed); the cell offsets stay in the cloud

@@ -76,9 +76,13 @@ def _bits(t):
     ("far", torch.float32, 1, 300, 9000, 4, 48),
 ])
 def test_indexed_calls_equal_the_exact_kernel(kind, dtype, B, Q, P, F, K):
+    _compare(_inputs(kind, B, Q, P, F, dtype, seed=P + K), K)
+
+
+def _compare(x, K):
     from cuda_knn_aggregate import capi
 
-    x = _inputs(kind, B, Q, P, F, dtype, seed=P + K)
+    B, Q, P, F, dtype = x[0].shape[0], x[0].shape[1], x[1].shape[1], x[2].shape[2], x[0].dtype
     size = 8 if dtype == torch.float64 else 4
     r256 = lambda n: (n + 255) // 256 * 256  # noqa: E731
     lean = 256 + r256(B * Q * 4) + r256(B * P * 16 * size)
@@ -87,6 +91,22 @@ def test_indexed_calls_equal_the_exact_kernel(kind, dtype, B, Q, P, F, K):
     got, want = _call(x, K, full), _call(x, K, lean)
     for a, b in zip(got, want):
         assert torch.equal(_bits(a), _bits(b))
+
+
+@pytest.mark.parametrize("kind,dtype,B,Q,P", [
+    ("rand", torch.float32, 1, 1, 128),         # the fewest points that are indexed: one tile
+    ("rand", torch.float32, 3, 1023, 1025),     # tiles for all eight, one with two
+    ("rand", torch.float32, 1, 32768, 4096),    # the largest element of the one-launch index
+    ("rand", torch.float32, 1, 32769, 4096),    # past it by a query,
+    ("rand", torch.float32, 1, 500, 4097),      # by a point,
+    ("rand", torch.float32, 17, 40, 200),       # by an element
+    ("rand", torch.float64, 16, 65, 300),
+    ("rand", torch.float64, 1, 9000, 4096),
+    ("nan", torch.float64, 2, 40, 4096),
+    ("far", torch.float32, 2, 700, 4000),
+])
+def test_index_sizes(kind, dtype, B, Q, P):
+    _compare(_inputs(kind, B, Q, P, 4, dtype, seed=Q + P), 33)
 
 
 @pytest.mark.parametrize("kind,B,Q,P,K", [
