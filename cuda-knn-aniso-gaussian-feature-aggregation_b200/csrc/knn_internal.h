@@ -311,8 +311,9 @@ int launch_pack_points(const void* p, const void* sigma, const void* R, int B, i
                        int64_t zero_rows2 = 0);
 // Chunks per batch element of the FP32 packing kernel that also bounds the
 // points: chunk c of element b writes its box to parts[(b * kBoundParts +
-// c) * 8 ...] (min xyz, max xyz), which the cell kernels reduce.
-constexpr int kBoundParts = 32;
+// c) * 8 ...] (min xyz, max xyz), which the cell kernels reduce.  128 of them:
+// with 32, a quarter of the SMs packed B = 1, P = 131072 in 33 us; 128 take 12.
+constexpr int kBoundParts = 128;
 template <typename T>
 int launch_pack_points_bounded(const T* p, const T* sigma, const T* R, const T* q, int B, int Q, int P, T* rec,
                                float* parts, float* pf, float* qf, cudaStream_t st, int* zero_words, int n_zero,

@@ -124,19 +124,24 @@ __device__ __forceinline__ int seed_of(const CellJob& j, const GroupRange& r, co
 }
 
 // The box of group r: bnd's entry, or the reduction of its nparts partial
-// boxes (into shared memory, by the first threads of the CTA; all threads
+// boxes (into shared memory, by the first six warps of the CTA; all threads
 // of the CTA must call this).
 __device__ __forceinline__ const float* job_bounds(const CellJob& j, const float* bnd, const GroupRange& r,
                                                    float* gbs) {
   if (j.nparts <= 0) return group_bounds(j.m, bnd) + r.bnd * 8;
-  if (threadIdx.x < 6) {
-    const int a = threadIdx.x;
+  const int a = threadIdx.x >> 5, lane = threadIdx.x & 31;  // warp a: plane a of the partial boxes
+  if (a < 6) {
     float v = a < 3 ? INFINITY : -INFINITY;
-    for (int i = 0; i < j.nparts; ++i) {
-      const float x = bnd[((int64_t)r.bnd * j.nparts + i) * 8 + a];
-      v = a < 3 ? fminf(v, x) : fmaxf(v, x);
+    for (int i = lane; i < j.nparts; i += 32) {
+      const float w = __ldg(bnd + ((int64_t)r.bnd * j.nparts + i) * 8 + a);
+      v = a < 3 ? fminf(v, w) : fmaxf(v, w);
     }
-    gbs[a] = v;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float w = __shfl_xor_sync(0xffffffffu, v, o);
+      v = a < 3 ? fminf(v, w) : fmaxf(v, w);
+    }
+    if (lane == 0) gbs[a] = v;
   }
   __syncthreads();
   return gbs;
