@@ -27,6 +27,11 @@ def _inputs(kind, B, Q, P, F, dtype, seed):
     if kind == "ties":  # a coarse lattice, unit Gaussians: most keys are shared
         p, q = (p * 5).round() / 4, (q * 9).round() / 8
         sigma, R = torch.ones_like(sigma), torch.eye(3, dtype=torch.float64).expand(B, P, 3, 3).clone()
+    elif kind == "twins":  # a few points of the same place and shape, most of them far apart in the order
+        to = torch.arange(7, P, 41)
+        at = torch.randint(0, P, (len(to),), generator=g)
+        for v in (p, sigma, R):
+            v[:, to] = v[:, at]
     elif kind == "negative":
         sigma = sigma - 0.5
     elif kind == "nan":
@@ -68,6 +73,11 @@ def _bits(t):
     ("rand", torch.float32, 1, 33, 128, 4, 128),      # K == P
     ("ties", torch.float64, 1, 90, 600, 4, 9),
     ("ties", torch.float32, 1, 90, 600, 4, 64),
+    ("twins", torch.float64, 1, 300, 3000, 4, 1),      # replays: one slot,
+    ("twins", torch.float64, 1, 200, 4097, 4, 32),     # two CTAs a query, unmerged tails
+    ("twins", torch.float64, 1, 60, 33000, 4, 64),     # eight CTAs, three lengths of ranges
+    ("twins", torch.float32, 1, 200, 8193, 4, 33),
+    ("twins", torch.float32, 1, 60, 66000, 4, 128),    # every slot of the longest list
     ("negative", torch.float64, 1, 70, 900, 4, 12),
     ("negative", torch.float32, 1, 70, 900, 4, 40),
     ("nan", torch.float64, 1, 70, 900, 4, 12),
