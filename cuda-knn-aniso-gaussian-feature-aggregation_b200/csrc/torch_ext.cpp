@@ -436,6 +436,10 @@ torch::Tensor or_placeholder(const torch::Tensor& t, const torch::Tensor& like) 
   return t.defined() ? t : torch::empty({0}, like.options());
 }
 
+c10::optional<torch::Tensor> if_any(const torch::Tensor& t) {
+  return t.numel() > 0 ? c10::optional<torch::Tensor>(t) : c10::nullopt;
+}
+
 // A gradient that is one value broadcast over its shape (every dimension of
 // size > 1 has stride 0) -- what autograd passes for f_out.sum().  It is
 // handed to the kernels as that one value instead of being materialised.
@@ -447,8 +451,9 @@ bool is_broadcast_scalar(const torch::Tensor& g) {
 }
 
 struct AggBackwardFn : public torch::autograd::Function<AggBackwardFn> {
-  // differentiable inputs: gfo, q, p, f, sigma, R; then idxs, points and the
-  // adjacency counted by the forward (empty if none) (no grad)
+  // differentiable inputs: gfo, q, p, f, sigma, R; then idxs, points (empty if
+  // the forward keeps none) and the adjacency counted by the forward (empty if
+  // none) (no grad)
   static variable_list forward(AutogradContext* ctx, torch::Tensor gfo, torch::Tensor q, torch::Tensor p,
                                torch::Tensor f, torch::Tensor sigma, torch::Tensor R, torch::Tensor idxs,
                                torch::Tensor points, torch::Tensor adj_counted, int64_t needs) {
@@ -462,7 +467,7 @@ struct AggBackwardFn : public torch::autograd::Function<AggBackwardFn> {
       adj = build_adjacency_impl(idxs, p.size(1), adj_counted, stream_of(idxs));
     }
     if (forked) adj = build_adjacency_forked(idxs, p.size(1), join, adj_counted);
-    auto o = backward_impl(1, c10::nullopt, gfo, q, p, f, sigma, R, c10::nullopt, idxs, points,
+    auto o = backward_impl(1, c10::nullopt, gfo, q, p, f, sigma, R, c10::nullopt, idxs, if_any(points),
                            (adj.defined() && !forked) ? c10::optional<torch::Tensor>(adj) : c10::nullopt,
                            c10::nullopt, needs, true);
     if (forked) join.block(at::cuda::getCurrentCUDAStream(q.device().index()));
@@ -488,13 +493,39 @@ struct AggBackwardFn : public torch::autograd::Function<AggBackwardFn> {
     torch::Tensor adj;
     if (ctx->saved_data.count("adj")) adj = ctx->saved_data["adj"].toTensor();
     if ((needs & kPointBits) && !adj.defined()) adj = build_adjacency(s[6], s[2].size(1));
-    auto o = backward_impl(2, gg[0].contiguous(), s[0], s[1], s[2], s[3], s[4], s[5], c10::nullopt, s[6], s[7],
+    auto o = backward_impl(2, gg[0].contiguous(), s[0], s[1], s[2], s[3], s[4], s[5], c10::nullopt, s[6], if_any(s[7]),
                            adj.defined() ? c10::optional<torch::Tensor>(adj) : c10::nullopt,
                            ctx->saved_data["coef"].toTensor(), needs, false);
     for (int i = 0; i < 6; ++i) out[i] = o[i];
     return out;
   }
 };
+
+// The backward of an aggregation whose first five inputs are q, p, f, sigma, R
+// and which saved those and idxs.  keep_scalar: a gradient of one value is
+// handed on as that value.
+variable_list aggregate_backward(AutogradContext* ctx, const variable_list& g, size_t n_inputs, bool keep_scalar) {
+  variable_list out(n_inputs);
+  if (g.empty() || !g[0].defined()) return out;  // grad_w_out / grad_dists are not propagated
+  int64_t needs = 0;
+  for (int i = 0; i < 5; ++i)
+    if (ctx->needs_input_grad(i)) needs |= kNeedBits[i];
+  if (!needs) return out;
+  auto s = ctx->get_saved_variables();
+  const bool scalar = keep_scalar && is_broadcast_scalar(g[0]);
+  // create_graph with point inputs that require grad: the second order of
+  // this graph may want point gradients (the Eikonal step does)
+  const bool prebuild = torch::GradMode::is_enabled() &&
+                        (s[1].requires_grad() || s[2].requires_grad() || s[3].requires_grad() || s[4].requires_grad());
+  torch::Tensor points, counted;
+  if (ctx->saved_data.count("points")) points = ctx->saved_data["points"].toTensor();
+  if (ctx->saved_data.count("adj_counted")) counted = ctx->saved_data["adj_counted"].toTensor();
+  auto r = AggBackwardFn::apply(scalar ? g[0] : g[0].contiguous(), s[0], s[1], s[2], s[3], s[4], s[5],
+                                or_placeholder(points, s[0]), or_placeholder(counted, s[5]),
+                                needs | (scalar ? KNNAG_GFO_SCALAR : 0) | (prebuild ? kPrebuildAdjacency : 0));
+  for (int i = 0; i < 5; ++i) out[i] = (needs & kNeedBits[i]) ? r[i] : torch::Tensor();
+  return out;
+}
 
 struct AggFn : public torch::autograd::Function<AggFn> {
   static variable_list forward(AutogradContext* ctx, torch::Tensor q, torch::Tensor p, torch::Tensor f,
@@ -510,28 +541,29 @@ struct AggFn : public torch::autograd::Function<AggFn> {
     return {o[0], o[1], o[2], o[3]};
   }
 
-  static variable_list backward(AutogradContext* ctx, variable_list g) {
-    variable_list out(6);
-    if (g.empty() || !g[0].defined()) return out;  // grad_w_out / grad_dists are not propagated
-    int64_t needs = 0;
-    for (int i = 0; i < 5; ++i)
-      if (ctx->needs_input_grad(i)) needs |= kNeedBits[i];
-    if (!needs) return out;
-    auto s = ctx->get_saved_variables();
-    const bool scalar = is_broadcast_scalar(g[0]);
-    // create_graph with point inputs that require grad: the second order of
-    // this graph may want point gradients (the Eikonal step does)
-    const bool prebuild = torch::GradMode::is_enabled() &&
-                          (s[1].requires_grad() || s[2].requires_grad() || s[3].requires_grad() || s[4].requires_grad());
-    torch::Tensor counted;
-    if (ctx->saved_data.count("adj_counted")) counted = ctx->saved_data["adj_counted"].toTensor();
-    auto r = AggBackwardFn::apply(scalar ? g[0] : g[0].contiguous(), s[0], s[1], s[2], s[3], s[4], s[5],
-                                  ctx->saved_data["points"].toTensor(), or_placeholder(counted, s[5]),
-                                  needs | (scalar ? KNNAG_GFO_SCALAR : 0) | (prebuild ? kPrebuildAdjacency : 0));
-    for (int i = 0; i < 5; ++i) out[i] = (needs & kNeedBits[i]) ? r[i] : torch::Tensor();
-    return out;
-  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) { return aggregate_backward(ctx, g, 6, true); }
 };
+
+// The lookup variant: what the fused op's backward gives at the looked-up
+// indices, no gradient for the table.  A broadcast gradient is materialised, as
+// the Python class does: the results of both are equal to the bit.
+struct LookupFn : public torch::autograd::Function<LookupFn> {
+  static variable_list forward(AutogradContext* ctx, torch::Tensor q, torch::Tensor p, torch::Tensor f,
+                               torch::Tensor sigma, torch::Tensor R, torch::Tensor table, int64_t K) {
+    auto o = knn_lookup_aggregate_aniso_forward(q, p, f, sigma, R, table, K);
+    ctx->save_for_backward({q, p, f, sigma, R, o[3]});
+    ctx->set_materialize_grads(false);
+    return o;
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list g) { return aggregate_backward(ctx, g, 7, false); }
+};
+
+std::vector<torch::Tensor> knn_aggregate_aniso_lookup_autograd(torch::Tensor q, torch::Tensor p, torch::Tensor f,
+                                                               torch::Tensor sigma, torch::Tensor R,
+                                                               torch::Tensor knn_table, int64_t K) {
+  return LookupFn::apply(q, p, f, sigma, R, knn_table, K);
+}
 
 std::vector<torch::Tensor> knn_aggregate_aniso_autograd(torch::Tensor q, torch::Tensor p, torch::Tensor f,
                                                         torch::Tensor sigma, torch::Tensor R, int64_t K) {
@@ -552,6 +584,8 @@ PYBIND11_MODULE(_C, m) {
   m.def("forward_ex", &forward_ex, "forward that also returns the packed point records");
   m.def("knn_aggregate_aniso_autograd", &knn_aggregate_aniso_autograd,
         "differentiable forward (C++ autograd Functions; gradients computed only where the graph task uses them)");
+  m.def("knn_aggregate_aniso_lookup_autograd", &knn_aggregate_aniso_lookup_autograd,
+        "lookup aggregate with C++ autograd nodes");
   m.def("build_adjacency", &build_adjacency, "point -> entry adjacency (CSR) of idxs");
   m.def("adjacency_views", &adjacency_views, "rowptr / entry views of an adjacency buffer");
   m.def("backward_ex", &backward_ex, "first-order adjoint with selectable outputs; also returns coef");

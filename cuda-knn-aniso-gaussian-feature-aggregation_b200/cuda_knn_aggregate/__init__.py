@@ -153,7 +153,15 @@ class KNNAnisotropicAggregate(torch.autograd.Function):
 
 class KNNLookupAnisotropicAggregate(KNNAnisotropicAggregate):
     """Lookup variant (reference ``__init__.py:120-165``); gradients as the
-    fused op's at the looked-up indices, none for the table."""
+    fused op's at the looked-up indices, none for the table.  ``apply`` on this
+    class itself runs the extension's C++ autograd nodes, as its base's does."""
+
+    @classmethod
+    def apply(cls, *args, **kwargs):
+        if cls is KNNLookupAnisotropicAggregate and not kwargs and len(args) == 7:
+            q, p, f, sigma, R, knn_table, K = args
+            return tuple(_C.knn_aggregate_aniso_lookup_autograd(q, p, f, sigma, R, knn_table, int(K)))
+        return super().apply(*args, **kwargs)
 
     @staticmethod
     def forward(ctx, q, p, f, sigma, R, knn_table, K):

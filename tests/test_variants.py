@@ -300,3 +300,38 @@ def test_precomputed_is_the_fused_ops_sum(B, Q, F, K):
     got = C._C.knn_precomputed_aggregate_aniso_forward(q, p, f, s, R, idx, K)
     for a, b in zip(got, (fo, w, d)):
         assert torch.equal(a, b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("Q,P,F,K", [(1, 1, 1, 1), (65, 40, 6, 7), (700, 300, 16, 12)])
+def test_lookup_nodes_are_the_python_functions(Q, P, F, K):
+    """The extension's autograd nodes and the Python classes (which a subclass
+    runs) launch the same kernels: every output and gradient is equal, of both
+    orders, and only inputs that need one get one."""
+    import cuda_knn_aggregate as C
+
+    class Sub(C.KNNLookupAnisotropicAggregate):
+        pass
+
+    g = torch.Generator().manual_seed(Q)
+    shapes = [(2, Q, 3), (2, P, 3), (2, P, F), (2, P, 3), (2, P, 3, 3)]
+    x = [torch.rand(*s, generator=g).cuda() for s in shapes]
+    table = torch.randint(0, P, (P, K), generator=g).cuda()
+    up = torch.rand(2, Q, F, generator=g).cuda()
+
+    def step(fn, frozen):
+        ins = [t.clone().requires_grad_(i != frozen) for i, t in enumerate(x)]
+        out = fn(*ins, table, K)
+        assert not out[3].requires_grad
+        first = torch.autograd.grad(out[0], [t for t in ins if t.requires_grad], up, retain_graph=True)
+        got = [*out, *first]
+        if frozen != 0:
+            (dq,) = torch.autograd.grad(out[0].sum(), ins[0], create_graph=True)
+            dq.pow(2).sum().backward()
+            got += [dq, *(t.grad for t in ins if t.grad is not None)]
+            assert frozen is None or ins[frozen].grad is None
+        return got
+
+    for frozen in (None, 0, 2):
+        a, b = step(C.knn_aggregate_aniso_lookup, frozen), step(Sub.apply, frozen)
+        assert len(a) == len(b) and all(torch.equal(u, v) for u, v in zip(a, b))
