@@ -33,11 +33,13 @@
 
 namespace knnag {
 
-// 8 MiB: the forward's scratch is about 276 bytes per point (records, search
-// tiles, spatial-index keys and permutation, tile infos, the tensor-core
-// filter's tile operands) plus 19 bytes per query (flag list, query
-// permutation, seed positions, search plan): up to ~31k points with few
-// queries, or ~15k points with ~230k queries.
+// 8 MiB: the FP32 forward's scratch is about 270 bytes per point (records,
+// search tiles, the sort's cells or in their place the tensor-core filter's tile
+// operands, permutation, tile infos and boxes) plus 19 bytes per query (flag
+// list, query permutation, seed positions, search plan): up to ~31k points with
+// few queries, or ~15k points with ~230k queries.  FP64 and K > 32 use the index
+// where it fits and else the exact kernel, which needs the records and the flag
+// list alone.
 constexpr size_t kNoallocScratchBytes = size_t(8) << 20;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoallocScratchBytes];

@@ -1,6 +1,8 @@
-// Forward path: point packing, the fused kNN search + aggregation kernel
-// (FP32, K <= 32), and the exact MinK kernel that replays the reference's
-// selection rules for flagged queries (and serves FP64 and K > 32).
+// Forward path: point packing, the plan of the tensor-core search, the exact
+// MinK kernel that applies the reference's selection rules to every query (calls
+// without an index), workspace layout and the call's order of kernels.  The
+// searches are in knn_search_warp.cu and knn_search_tc.cu, the replay of flagged
+// queries in knn_replay.cu.
 //
 // Replaces csrc/forward.cu:56-110 (kernel), csrc/forward.cu:286-338
 // (launcher) and csrc/mink.cuh of the reference.
@@ -650,6 +652,9 @@ FwdLayout fwd_layout(int B, int Q, int P, int K, int dtype, bool own_rec, bool i
     const size_t ntiles = (size_t)B * (L.P_pad / kTilePoints);
     L.pairs = off;
     off += align256((size_t)B * L.P_pad * kRecLen * esz);
+    // what the sort alone uses, and in the same place what the tile-info kernel
+    // writes after it: the tensor-core filter's B operands
+    const size_t sort_at = off;
     L.bounds = off;  // per element kBoundParts partial boxes
     off += align256((size_t)B * kBoundParts * 8 * 4);
     // point and query cells of each batch element, sorted together
@@ -657,6 +662,8 @@ FwdLayout fwd_layout(int B, int Q, int P, int K, int dtype, bool own_rec, bool i
     off += align256(2 * (size_t)B * cells * 4);
     L.cell_offset = off;
     off += align256((2 * (size_t)B * cells + 1) * 4);
+    L.tcops = sort_at;
+    if (dtype == KNNAG_F32 && K <= 32) off = std::max(off, sort_at + align256(ntiles * kTcOpsBytes));
     L.perm_p = off;  // perm_q follows perm_p without a gap (one scatter fills both)
     L.perm_q = off + (size_t)B * P * 4;
     off += align256((size_t)B * P * 4 + (size_t)B * Q * 4);
@@ -685,9 +692,7 @@ FwdLayout fwd_layout(int B, int Q, int P, int K, int dtype, bool own_rec, bool i
       off += align256(nb_max * 4);
       L.items = off;
       off += align256(nb_max * 16);
-      // tensor-core filter: B operands and bound terms of every tile
-      L.tcops = off;
-      off += align256(ntiles * kTcOpsBytes);
+      // tensor-core filter: bound terms of every tile
       L.tcinfo = off;
       off += align256(ntiles * kTcInfoBytes);
     }
