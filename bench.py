@@ -575,13 +575,13 @@ def fp32_peak_tflops(device):
     return best
 
 
-# DRAM bytes (read + write) of one search_f32_kernel<16,2,16> launch at the
+# DRAM bytes (read + write) of one search_warp_kernel<float,1> launch at the
 # table workload, from the ncu capture summarised in
-# profiles/search_f32_table.md (dram__bytes_read.sum + dram__bytes_write.sum
+# profiles/search_table.md (dram__bytes_read.sum + dram__bytes_write.sum
 # of one launch); update it with that summary whenever the search kernel
 # changes.
-SEARCH_TRAFFIC_BYTES = 3230720
-SEARCH_TRAFFIC_SOURCE = "ncu capture of one search_f32_kernel<16,2,16> launch (profiles/search_f32_table.md)"
+SEARCH_TRAFFIC_BYTES = 3185408
+SEARCH_TRAFFIC_SOURCE = "ncu capture of one search_warp_kernel<float,1> launch (profiles/search_table.md)"
 
 CONFIG = {"workload": "table: B=2 Q=12288 P=4096 F=64 K=16, fwd + dq(create_graph) + Eikonal backward",
           "l2": "flushed between timed steps (256 MiB write)"}
@@ -680,7 +680,7 @@ def run_ours(args):
     pairs = shape.B * shape.Q * shape.P
     peak = fp32_peak_tflops(device)
     achieved = FLOP_PER_PAIR * pairs / search_s / 1e12
-    roofline = {"bound": "fp32", "kernel": "search_f32_kernel", "achieved": achieved, "peak": peak,
+    roofline = {"bound": "fp32", "kernel": "search_warp_kernel", "achieved": achieved, "peak": peak,
                 "unit": "TFLOP/s", "frac": achieved / peak,
                 "peak_source": "measured: FFMA-bound probe kernel in bench.py (MEASURED_PEAKS.json has no FP32 figure)",
                 "algorithmic": f"{FLOP_PER_PAIR} FLOP x {pairs} (q,p) pairs per launch",

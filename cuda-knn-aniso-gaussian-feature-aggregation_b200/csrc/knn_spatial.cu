@@ -11,8 +11,8 @@
 // |q - p|^2 * sum_a |sigma_a| |R_a|^2).  With every sigma >= 0 every key is
 // >= 0, so mu = 0 still bounds; a tile holding a negative or non-finite
 // value gets mu = -1: no bound at all (its keys may be negative).
-// The search visits tiles nearest-first by this bound and stops when the
-// bound exceeds every query's threshold; the order of points inside a cell
+// The searches skip tiles, and 32-point sub-boxes of them, whose bound exceeds
+// the thresholds; the order of points inside a cell
 // (atomic scatter) never changes a result, only the work done.
 #include <cooperative_groups.h>
 #include <math.h>

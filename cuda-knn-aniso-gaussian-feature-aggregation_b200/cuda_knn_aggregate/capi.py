@@ -286,7 +286,7 @@ def fp32_peak_probe(out, blocks, iters):
 
 
 def set_search_splits(splits):
-    """Process-wide split count of the uniform search (0: automatic)."""
+    """Process-wide launch shape of the uniform search (0: automatic; see ``tuning``)."""
     _check(lib().knnag_set_search_splits(int(splits)))
 
 

@@ -25,9 +25,8 @@ import torch
 
 from . import capi
 
-# search launch shapes (the C ABI's `splits` code): 1, 2, 4 -> 4, 2, 1 warps of
-# 32 queries per CTA; 8 -> 2 warps of 16; 16 -> 4 warps of 8; 32 -> 1 warp of
-# 16; 64 -> 1 warp of 8
+# search launch shapes (the C ABI's `splits` code): queries per work item, 128,
+# 64, 32, 32, 32, 16, 8
 _SPLITS = (1, 2, 4, 8, 16, 32, 64)
 
 
@@ -135,9 +134,9 @@ class CloudSet:
 
 
 def default_splits(total_queries, device=None):
-    """Search launch shape by the warps the queries give at 32 per warp (the
-    uniform op's rule): many -> 128-query CTAs; few -> fewer queries per
-    warp, for more warps."""
+    """Search launch shape by the warps the queries give at 32 per warp: many ->
+    work items of 128 queries, fewer -> of 32 (the search itself takes four
+    queries at a time from either)."""
     sms = torch.cuda.get_device_properties(device or torch.cuda.current_device()).multi_processor_count \
         if torch.cuda.is_available() else 148
     warps32 = (int(total_queries) + 31) // 32

@@ -3,12 +3,11 @@
 The tuned knobs change only the time, never a result:
 
 * ``splits``, the search launch shape (the C ABI's
-  ``knnag_set_search_splits``): 1, 2, 4 -> 4, 2, 1 warps of 32 queries per
-  CTA; 8 -> 2 warps of 16 queries; 16 -> 4 warps of 8; 32 -> 1 warp of 16;
-  64 -> 1 warp of 8 -- queries per CTA and per warp; 128 -> the tensor-core
-  filtered search (128 queries per CTA, two threads per query);
-* the K register layout: the list length is the K bucket (8, 16, 32) --
-  part of the shape bucket, not a free knob.
+  ``knnag_set_search_splits``): 1, 2 -> 16, 8 queries per warp; 4, 8, 16 -> 4;
+  32 -> 2; 64 -> 1; 128 -> the tensor-core filtered search (128 queries per
+  CTA, two threads per query);
+* the K register layout: one list register per lane up to K = 32, two up to
+  64, four up to 128 -- by K, not a free knob.
 
 ``autotune_search(...)`` times every candidate on the caller's inputs (the
 median of CUDA-event timings of the forward) and keeps the fastest, keyed by

@@ -345,15 +345,15 @@ long long knnag_launch_count(void);
 
 /* Tuning: launch shape of the FP32 search of every later knnag_forward /
  * knnag_forward_noalloc in the process (the autotuner sets it from timings
- * cached per shape bucket): 1, 2, 4 -> CTAs of 4, 2, 1 warps of 32 queries;
- * 8 -> 2 warps of 16 queries; 16 -> 4 warps of 8 queries; 32 -> 1 warp of
- * 16; 64 -> 1 warp of 8 (fewer queries per warp give more warps for small
- * query sets); 128 -> the tensor-core filtered search (approximate keys of
- * 128 queries x 128 points per tcgen05 MMA, exact keys for the candidates);
- * 0 restores the automatic choice (the tensor-core search for grids of more
- * than 8 waves of its CTAs, else by the warps the query set gives).  Results
- * do not depend on it.  Returns KNNAG_ERR_ARG for other values.  Codes 1-64
- * are also the `splits` of segment tables.  No reference counterpart. */
+ * cached per shape bucket): 1, 2 -> 16, 8 queries per warp; 4, 8, 16 -> 4;
+ * 32 -> 2; 64 -> 1 (fewer queries per warp give more warps for small query
+ * sets); 128 -> the tensor-core filtered search (approximate keys of 128
+ * queries x 128 points per tcgen05 MMA, exact keys for the candidates); 0
+ * restores the automatic choice (4 queries per warp, 2 or 1 where the query
+ * set would leave the chip short of warps).  Results do not depend on it.
+ * Returns KNNAG_ERR_ARG for other values.  Codes 1-64 are also the `splits` of
+ * segment tables: work items of 128, 64, 32 (4, 8, 16), 16, 8 queries.  No
+ * reference counterpart. */
 int knnag_set_search_splits(int splits);
 int knnag_get_search_splits(void);
 
