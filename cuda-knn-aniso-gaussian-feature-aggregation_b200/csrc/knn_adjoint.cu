@@ -641,12 +641,50 @@ __device__ __forceinline__ QueryRow<T> segment_row(const QueryParams<T>& a, cons
   return QueryRow<T>{g.K, c.P, g.e_off + (bq - g.q_off) * g.K, c.p_off, rec + c.p_off * kRecLen, a.f + c.p_off * a.F};
 }
 
+// Each lane's record `idx` (any valid one where the lane has none) of `recb`, for
+// all lanes of a warp; the four lanes of a quad have the same recb.  FP32: the
+// quad loads its four records together, 16 bytes a lane, so that a load
+// instruction touches 8 lines instead of 32, and transposes.  At B = 1,
+// Q = 524288, K = 16 the broadcast query side takes 153 us with it and 183
+// without, the second order's launch 283 and 296.
+__device__ __forceinline__ void load_rec_quad(const float* recb, int idx, float (&r)[kRecLen]) {
+  const int t = threadIdx.x & 3;
+  float4 d[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int i = __shfl_sync(0xffffffffu, idx, u, 4);
+    d[u] = __ldg(reinterpret_cast<const float4*>(recb + (int64_t)i * kRecLen) + t);
+  }
+  // d[u] holds part t of the quad's record u; exchanged to part u of record t
+  auto swap = [](float4& x, float4& y, bool upper, int o) {  // y of the lower lane with x of the upper
+    float4 v = upper ? x : y;
+    v.x = __shfl_xor_sync(0xffffffffu, v.x, o);
+    v.y = __shfl_xor_sync(0xffffffffu, v.y, o);
+    v.z = __shfl_xor_sync(0xffffffffu, v.z, o);
+    v.w = __shfl_xor_sync(0xffffffffu, v.w, o);
+    if (upper) x = v;
+    else y = v;
+  };
+  swap(d[0], d[1], t & 1, 1);
+  swap(d[2], d[3], t & 1, 1);
+  swap(d[0], d[2], t & 2, 2);
+  swap(d[1], d[3], t & 2, 2);
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    r[4 * u + 0] = d[u].x;
+    r[4 * u + 1] = d[u].y;
+    r[4 * u + 2] = d[u].z;
+    r[4 * u + 3] = d[u].w;
+  }
+}
+__device__ __forceinline__ void load_rec_quad(const double* recb, int idx, double (&r)[kRecLen]) {
+  load_rec(recb + (int64_t)idx * kRecLen, r);
+}
+
 // One neighbour's share of dq: -2 c w v.
 template <typename T>
-__device__ __forceinline__ void add_dq(const QueryParams<T>& a, const T* rec_g, T qx, T qy, T qz, int64_t e, T c,
-                                       T (&acc)[3]) {
-  T rec[kRecLen];
-  load_rec(rec_g, rec);
+__device__ __forceinline__ void add_dq(const QueryParams<T>& a, const T (&rec)[kRecLen], T qx, T qy, T qz, int64_t e,
+                                       T c, T (&acc)[3]) {
   Geo<T> geo;
   geometry(qx, qy, qz, rec, geo);
   const T w = a.w_in ? a.w_in[e] : geo.w;
@@ -665,8 +703,16 @@ __device__ __forceinline__ void add_dq(const QueryParams<T>& a, const T* rec_g, 
 // for them and not by a chain of dependent loads per row.
 constexpr int kRowBlock = 8;
 
+// Bound by the latency of a neighbour's index and record: a kernel of its own, at
+// four CTAs per SM (5: 218 us where 4 take 153 at the sizes above, 6: 242; as a
+// branch of query_order1_kernel at three: 207), table workload 13.0 -> 10.4 us,
+// 24 ragged clouds 149 -> 129.
 template <typename T>
-__device__ __forceinline__ void query_order1_scalar(const QueryParams<T>& a, const SegHeader* sh, int64_t BQ) {
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) query_order1_broadcast_kernel(QueryParams<T> a) {
+  const SegHeader* sh = static_cast<const SegHeader*>(a.segs);
+  if (sh && *a.status) return;
+  zero_status_words(a.zero_status);
+  const int64_t BQ = sh ? sh->grad_rows : (int64_t)a.B * a.Q;
   const int lane = threadIdx.x & 31;
   const int lpq = (!sh && a.K <= 16) ? 16 : 32;  // lanes per query
   const int qpw = 32 / lpq, sub = lane / lpq, kl = lane % lpq;
@@ -682,19 +728,24 @@ __device__ __forceinline__ void query_order1_scalar(const QueryParams<T>& a, con
       T acc[3] = {T(0), T(0), T(0)};
       if (sh)
         while (s + 1 < sh->nseg && sd[s + 1].q_off <= bq) ++s;
-      if (bq < BQ) {
-        const QueryRow<T> r = sh ? segment_row(a, sd, s, bq) : uniform_row(a, bq);
-        const T qx = a.q[bq * 3 + 0], qy = a.q[bq * 3 + 1], qz = a.q[bq * 3 + 2];
-        for (int k = kl; k < r.K; k += lpq) {
-          const int64_t e = r.e0 + k;
-          const int64_t idx = a.idxs[e];
-          T c = T(0);
-          if (idx >= 0 && idx < r.P) {
-            c = sg0 * a.frowsum[r.pbase + idx];
-            add_dq(a, r.recb + idx * kRecLen, qx, qy, qz, e, c, acc);
-          }
-          if (a.coef_out) a.coef_out[e] = c;
+      const bool live = bq < BQ;
+      const QueryRow<T> r = sh ? segment_row(a, sd, s, bq) : uniform_row(a, live ? bq : base);
+      const T* qp = a.q + (live ? bq : base) * 3;
+      const T qx = qp[0], qy = qp[1], qz = qp[2];
+      for (int k0 = 0; k0 < r.K; k0 += lpq) {  // K is the same for the warp's queries
+        const int k = k0 + kl;
+        const int64_t e = r.e0 + k;
+        const int64_t idx = live && k < r.K ? a.idxs[e] : -1;
+        const bool ok = idx >= 0 && idx < r.P;
+        T rec[kRecLen];
+        if (!sh) load_rec_quad(r.recb, ok ? (int)idx : 0, rec);
+        else if (ok) load_rec(r.recb + idx * kRecLen, rec);  // small K: idle lanes would load for nothing
+        T c = T(0);
+        if (ok) {
+          c = sg0 * a.frowsum[r.pbase + idx];
+          add_dq(a, rec, qx, qy, qz, e, c, acc);
         }
+        if (a.coef_out && live && k < r.K) a.coef_out[e] = c;
       }
 #pragma unroll
       for (int mm = 0; mm < 3; ++mm)
@@ -764,10 +815,6 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) query_order1_kern
   if (sh && *a.status) return;
   zero_status_words(a.zero_status);
   const int64_t BQ = sh ? sh->grad_rows : (int64_t)a.B * a.Q;
-  if (a.frowsum) {
-    query_order1_scalar(a, sh, BQ);
-    return;
-  }
   constexpr int N = 32 / G;  // queries of the warp
   const int cols = a.F / C;
   const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
@@ -830,7 +877,11 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) query_order1_kern
       if (live && gl < NK && km < r.K) {
         const int64_t e = r.e0 + km;
         if (a.coef_out) a.coef_out[e] = part[0];
-        if (mine >= 0) add_dq(a, r.recb + (int64_t)mine * kRecLen, qx, qy, qz, e, part[0], acc);
+        if (mine >= 0) {
+          T rec[kRecLen];
+          load_rec(r.recb + (int64_t)mine * kRecLen, rec);
+          add_dq(a, rec, qx, qy, qz, e, part[0], acc);
+        }
       }
     }
 #pragma unroll
@@ -862,15 +913,17 @@ __device__ __forceinline__ void query_order2_half(const QueryParams<T>& a, int64
   for (int64_t base = gw * 2; base < BQ; base += nw * 2) {
     const int64_t bq = base + sub;
     T acc[3] = {T(0), T(0), T(0)};
-    if (bq < BQ && k < K && a.coef_in) {
-      const int64_t b = bq / a.Q;
+    if (a.coef_in) {  // uniform
+      const int64_t row = bq < BQ ? bq : base;
+      const int64_t b = row / a.Q;
       const int64_t e = bq * K + k;
-      const int64_t idx = a.idxs[e];
-      if (idx >= 0 && idx < P) {
+      const int64_t idx = bq < BQ && k < K ? a.idxs[e] : -1;
+      const bool ok = idx >= 0 && idx < P;
+      T rr[kRecLen];
+      load_rec_quad(a.rec + b * P * kRecLen, ok ? (int)idx : 0, rr);
+      if (ok) {
         const T qx = a.q[bq * 3 + 0], qy = a.q[bq * 3 + 1], qz = a.q[bq * 3 + 2];
         const T g[3] = {a.ggq[bq * 3 + 0], a.ggq[bq * 3 + 1], a.ggq[bq * 3 + 2]};
-        T rr[kRecLen];
-        load_rec(a.rec + (b * P + idx) * kRecLen, rr);
         const T* rec = rr;
         Geo<T> geo;
         geometry(qx, qy, qz, rec, geo);
@@ -1243,6 +1296,12 @@ namespace {
 // with no columns to sweep), which halves the idle lanes of the geometry.
 template <typename T>
 int launch_order1(const QueryParams<T>& p, int64_t rows, cudaStream_t st) {
+  if (p.frowsum) {
+    const bool pairs = !p.segs && p.K <= 16;
+    query_order1_broadcast_kernel<T><<<blocks_for((pairs ? (rows + 1) / 2 : rows) * 32, 256), 256, 0, st>>>(p);
+    note_launches(1);
+    return cudaGetLastError() == cudaSuccess ? KNNAG_OK : KNNAG_ERR_CUDA;
+  }
   constexpr int C = 16 / sizeof(T);
   const bool vec = p.F % C == 0 && (uintptr_t)p.f % 16 == 0 && (uintptr_t)p.gfo % 16 == 0;
   const int cols = vec ? p.F / C : p.F;

@@ -43,3 +43,39 @@ def test_both_orders_match_fp64_autograd(F, K, dtype):
     tol = 1e-4 if dtype == torch.float32 else 1e-10
     for a, b in zip(list(first) + list(second), list(want) + list(want2)):
         assert rel_err(a.detach().cpu().numpy(), b.detach().numpy()) < tol
+
+
+@pytest.mark.parametrize("B,Q,P,K", [(1, 1, 1, 1), (3, 5, 40, 3), (1, 33, 200, 15), (2, 77, 300, 16), (1, 61, 90, 17),
+                                     (1, 9, 70, 33)])
+def test_broadcast_gradient_query_sides(B, Q, P, K):
+    """The Eikonal step's query sides (a broadcast f_out gradient, then dq's
+    own gradient) where quads of lanes that share their record loads are cut:
+    K around multiples of 4, of a half-warp and a warp, an odd number of
+    queries, indices out of range beside good ones.  FP64 autograd of the plain
+    formula, tolerance as for every gradient here."""
+    from cuda_knn_aggregate import _C
+
+    g = torch.Generator().manual_seed(Q + K)
+    r = lambda *s: torch.rand(*s, generator=g)  # noqa: E731
+    x = [r(B, Q, 3), r(B, P, 3), r(B, P, 6), r(B, P, 3), r(B, P, 3, 3)]
+    idx = torch.randint(0, P, (B, Q, K), generator=g)
+    ggq = torch.randn(B, Q, 3, generator=g)
+    gfo = torch.ones(B, Q, 6)
+    first, second = O.grads64(*[t.double() for t in x], idx, gfo.double(), ggq.double())
+    dev = [t.cuda() for t in x]
+    need = _C.NEED_DQ | 64  # KNNAG_GFO_SCALAR
+    one = torch.ones(1, device="cuda").expand(B, Q, 6)  # one value, broadcast
+    out = _C.backward_ex(one, *dev, idx.cuda(), None, None, need)
+    assert _rel(out[0], first[0]) < 1e-4
+    two = _C.backward2_ex(ggq.cuda(), one, *dev, idx.cuda(), None, None, out[5], need)
+    assert _rel(two[1], second[1]) < 1e-4
+    if K > 1:  # an entry that is out of range counts for nothing
+        bad = idx.clone()
+        bad[:, :, 1] = P
+        part = _C.backward_ex(one, *dev, bad.cuda(), None, None, need)
+        alone = _C.backward_ex(one, *dev, idx[:, :, 1:2].contiguous().cuda(), None, None, need)
+        assert _rel(part[0] + alone[0], first[0]) < 1e-4
+
+
+def _rel(a, b):
+    return float((a.cpu().double() - b).norm() / b.norm())
