@@ -583,7 +583,7 @@ constexpr int kIndexCtas = 8;
 constexpr int kIndexThreads = 1024;
 constexpr int kIndexPoints = 4096;
 constexpr int kIndexCells = 512;  // 8^spatial_bits(kIndexPoints)
-constexpr int kIndexElements = 16;
+constexpr int kIndexElements = 8;
 constexpr int kIndexPerThread = 4;
 constexpr int kIndexQueries = kIndexCtas * kIndexThreads * kIndexPerThread;
 constexpr int kIndexTiles = kIndexPoints / kTilePoints / kIndexCtas;  // tiles of a CTA
@@ -852,8 +852,9 @@ template int launch_spatial_index<double>(const float*, const float*, const doub
                                           const FwdLayout&, cudaStream_t, bool);
 
 // Elements that a cluster's shared memory and registers hold, and no more of
-// them than run at the same time (8 CTAs of a whole SM each): past that the
-// separate launches, which split the work by points and queries, are as fast.
+// them than find room at the same time (8 CTAs of a whole SM each, side by
+// side): a graph-replayed forward at Q = 1000, P = 500 took 38 us with one
+// launch and 40 with four at B = 8, but 55 and 49 at B = 16, 85 and 78 at 32.
 bool index_in_one_launch(int B, int Q, int P) {
   return P <= kIndexPoints && Q <= kIndexQueries && B <= kIndexElements;
 }

@@ -109,7 +109,9 @@ def _compare(x, K):
     ("rand", torch.float32, 1, 32768, 4096),    # the largest element of the one-launch index
     ("rand", torch.float32, 1, 32769, 4096),    # past it by a query,
     ("rand", torch.float32, 1, 500, 4097),      # by a point,
-    ("rand", torch.float32, 17, 40, 200),       # by an element
+    ("rand", torch.float32, 8, 40, 200),        # the most elements,
+    ("rand", torch.float32, 9, 40, 200),        # and one more
+    ("rand", torch.float32, 17, 40, 200),
     ("rand", torch.float64, 16, 65, 300),
     ("rand", torch.float64, 1, 9000, 4096),
     ("nan", torch.float64, 2, 40, 4096),
