@@ -170,6 +170,21 @@ __device__ __forceinline__ float2 key_pair(float2 qx2, float2 qy2, float2 qz2, c
                     __ffma2_rn(__fmul2_rn(j, j), pr[kS0], __fmul2_rn(__fmul2_rn(k, k), pr[kS1])));
 }
 
+// Lower bound of the keys (of type T) of points with bound factor mu at a
+// distance of at least sqrt(d2), both FP32, whose range is narrower than that of
+// FP64 keys; NaN where the points have no bound (mu is NaN), so that "bound >
+// threshold" is false.  The factor covers the rounding of d2 and of the product;
+// the terms taken off, what squares and the product lose below the normal floats.
+// A d2 beyond the floats counts as about FLT_MAX, and so does a bound of FP64 keys;
+// FP32 keys whose bound exceeds the floats do so themselves.
+constexpr float kBoundMax = 3.4e38f;
+template <typename T>
+__device__ __forceinline__ float key_bound(float mu, float d2) {
+  const float lb = __fmaf_rn(mu, __fmaf_rn(fminf(d2, kBoundMax), 0.99999f, -1e-30f), -2e-38f);
+  if (sizeof(T) == 4) return lb;
+  return lb > kBoundMax ? kBoundMax : lb;  // NaN stays
+}
+
 // 16-byte groups of feature columns.
 template <typename T>
 struct Group16;

@@ -111,20 +111,17 @@ __device__ __forceinline__ void seed_warp(float4* tab, int my_seed, bool valid, 
 }
 
 // Lower bound on the key of any query in box [bmin, bmax] against any point
-// of a tile (its box ti[0..5], bound factor mu = ti[6]): mu * dist(box,
-// tile box)^2, shrunk by 1e-5 for the rounding of this product; -inf when
-// the tile has no bound (mu < 0).
+// of a tile (its box ti[0..5], bound factor mu = ti[6]): see key_bound;
+// -inf when the tile has no bound (mu < 0).
 __device__ __forceinline__ float tile_lower_bound(const float* ti, const float* bmin, const float* bmax) {
-  const float mu = ti[6];
-  if (!(mu >= 0.f)) return -INFINITY;
   float d2 = 0.f;
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     const float g = fmaxf(fmaxf(ti[c] - bmax[c], bmin[c] - ti[3 + c]), 0.f);
     d2 = __fmaf_rn(g, g, d2);
   }
-  const float lb = mu * d2 * 0.99999f;
-  return lb >= 0.f ? lb : 0.f;  // NaN: 0 (keys are >= 0 when mu >= 0)
+  const float lb = key_bound<float>(ti[6], d2);
+  return ti[6] >= 0.f ? fmaxf(lb, 0.f) : -INFINITY;
 }
 
 }  // namespace knnag

@@ -189,8 +189,8 @@ __device__ __forceinline__ void list_push(T (&k)[V], int (&p)[V], T nk, int np, 
 }
 
 // Lower bound of the keys of a query box [lo, hi] against a box of points
-// (min xyz, mu), (max xyz): mu * distance^2, shrunk by 1e-5 for the rounding
-// of this product; -inf when the points have no bound (mu < 0).
+// (min xyz, mu), (max xyz): see key_bound.
+template <typename T>
 __device__ __forceinline__ float box_bound(const float (&mn)[3], const float (&mx)[3], float mu, const float (&lo)[3],
                                            const float (&hi)[3]) {
   float d2 = 0.f;
@@ -199,8 +199,7 @@ __device__ __forceinline__ float box_bound(const float (&mn)[3], const float (&m
     const float g = fmaxf(fmaxf(mn[c] - hi[c], lo[c] - mx[c]), 0.f);
     d2 = __fmaf_rn(g, g, d2);
   }
-  const float lb = mu * d2 * 0.99999f;
-  return mu >= 0.f ? (lb >= 0.f ? lb : 0.f) : -INFINITY;
+  return key_bound<T>(mu, d2);
 }
 
 // What a unit of queries is searched against, and where its results go.
@@ -254,6 +253,7 @@ struct __align__(16) WarpShared {
 };
 
 // Box planes of tile or group t.
+template <typename T>
 __device__ __forceinline__ float plane_bound(const float* box, int64_t plane, int t, const float (&lo)[3],
                                              const float (&hi)[3]) {
   float mn[3], mx[3];
@@ -262,7 +262,7 @@ __device__ __forceinline__ float plane_bound(const float* box, int64_t plane, in
     mn[c] = __ldg(box + c * plane + t);
     mx[c] = __ldg(box + (3 + c) * plane + t);
   }
-  return box_bound(mn, mx, __ldg(box + 6 * plane + t), lo, hi);
+  return box_bound<T>(mn, mx, __ldg(box + 6 * plane + t), lo, hi);
 }
 
 // The unit's queries: sorted positions [s0, s0 + n), n <= kUnit.
@@ -432,9 +432,9 @@ __device__ __forceinline__ void search_unit(const WarpSearchParams<T>& a, const 
   const int groups = (it.ntile + 31) >> 5;
   home = min(home, groups - 1);
   if (groups > 2) {
-    int best = 0x7fffffff, bestg = 0;  // bound (its bits: it is >= 0 or the group has none) and group of this lane
+    int best = 0x7fffffff, bestg = 0;  // bound (its bits, 0 for none) and group of this lane
     for (int g = lane; g < groups; g += 32) {
-      const int lb = __float_as_int(fmaxf(plane_bound(it.gbox, it.gplane, g, blo, bhi), 0.f));
+      const int lb = __float_as_int(fmaxf(plane_bound<T>(it.gbox, it.gplane, g, blo, bhi), 0.f));
       if (lb < best || (lb == best && g == home)) {
         best = lb;
         bestg = g;
@@ -449,7 +449,7 @@ __device__ __forceinline__ void search_unit(const WarpSearchParams<T>& a, const 
   {
     const int t = home * 32 + lane;
     float lb = INFINITY;
-    if (t < it.ntile) lb = plane_bound(it.tbox, it.tplane, t, blo, bhi);
+    if (t < it.ntile) lb = plane_bound<T>(it.tbox, it.tplane, t, blo, bhi);
     T tmax = tau[0];
 #pragma unroll
     for (int j = 1; j < U; ++j) tmax = fmax(tmax, tau[j]);
@@ -480,7 +480,7 @@ __device__ __forceinline__ void search_unit(const WarpSearchParams<T>& a, const 
       for (int j = 0; j < U; ++j) {
         const UnitQuery<T> uq = sm.q[j];
         const float lo[3] = {lo_of(uq.x), lo_of(uq.y), lo_of(uq.z)}, hi[3] = {hi_of(uq.x), hi_of(uq.y), hi_of(uq.z)};
-        lb[j] = box_bound(mn, mx, b0.w, lo, hi);
+        lb[j] = box_bound<T>(mn, mx, b0.w, lo, hi);
         // not those of the window
         need[j] = __ballot_sync(kFull, in && !((T)lb[j] > tau[j]) &&
                                            (unsigned)(code * 32 - uq.win) >= (unsigned)W);
@@ -551,7 +551,7 @@ __device__ __forceinline__ void search_unit(const WarpSearchParams<T>& a, const 
         if (gbase >= groups) break;
         const int g = gbase + lane;
         bool keep = g < groups && g != home;
-        if (groups > 2 && keep) keep = !((T)plane_bound(it.gbox, it.gplane, g, blo, bhi) > tmax);
+        if (groups > 2 && keep) keep = !((T)plane_bound<T>(it.gbox, it.gplane, g, blo, bhi) > tmax);
         gmask = __ballot_sync(kFull, keep);
       }
       if (gmask == 0) {
@@ -560,7 +560,7 @@ __device__ __forceinline__ void search_unit(const WarpSearchParams<T>& a, const 
       }
       const int t = (gbase + __ffs(gmask) - 1) * 32 + lane;
       gmask &= gmask - 1;
-      const bool keep = t < it.ntile && !((T)plane_bound(it.tbox, it.tplane, t, blo, bhi) > tmax);
+      const bool keep = t < it.ntile && !((T)plane_bound<T>(it.tbox, it.tplane, t, blo, bhi) > tmax);
       const unsigned b = __ballot_sync(kFull, keep);
       if (keep) sm.tiles[nt + __popc(b & ((1u << lane) - 1u))] = t;
       nt += __popc(b);

@@ -8,9 +8,13 @@
 //               - 1e-5 * sum_a |sigma_a| |R_a|^2,
 // where lambda_min is computed in double and the second term covers the
 // rounding of the FP32 key (|key_fp32 - key_exact| <= ~12 * 2^-24 *
-// |q - p|^2 * sum_a |sigma_a| |R_a|^2).  With every sigma >= 0 every key is
-// >= 0, so mu = 0 still bounds; a tile holding a negative or non-finite
-// value gets mu = -1: no bound at all (its keys may be negative).
+// |q - p|^2 * sum_a |sigma_a| |R_a|^2, as long as the rotated offsets' squares
+// are normal floats: at distances that count for a bound, above 1e-15, their
+// lost digits are covered too where |R_a| >= 3e-5; a point with a shorter row
+// gets 0).  mu is rounded down to FP32, FLT_MAX at most.  With every sigma >= 0
+// every key is >= 0, so mu = 0 still bounds; a tile holding a negative or
+// non-finite value has no bound at all (its keys may be negative): mu = NaN, in
+// the tile infos -1.
 // The searches skip tiles, and 32-point sub-boxes of them, whose bound exceeds
 // the thresholds; the order of points inside a cell
 // (atomic scatter) never changes a result, only the work done.
@@ -476,6 +480,7 @@ __device__ __forceinline__ void tile_info_body(bool active, const T* rec, const 
       }
       double M[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
       double err = 0.0;
+      bool short_row = false;
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
         const double s = v[kS0 + a];
@@ -489,12 +494,13 @@ __device__ __forceinline__ void tile_info_body(bool active, const T* rec, const 
           for (int n2 = 0; n2 < 3; ++n2) M[m][n2] += s * ra * (double)v[kR00 + 3 * a + n2];
         }
         err += fabs(s) * rn;
+        if (sizeof(T) == 4 && s != 0.0 && rn < 1e-9) short_row = true;
       }
       const double lam = sym3_min_eig(M[0][0], M[1][1], M[2][2], M[0][1], M[0][2], M[1][2]);
       const double scale = fabs(M[0][0]) + fabs(M[1][1]) + fabs(M[2][2]) + fabs(M[0][1]) + fabs(M[0][2]) + fabs(M[1][2]);
       const double m = lam - 1e-9 * scale - 1e-5 * err;
       if (!isfinite(m)) bad = true;
-      mu = fminf(mu, (m > 0.0 && isfinite(m)) ? (float)(m * (1.0 - 1e-6)) : 0.0f);
+      mu = fminf(mu, m > 0.0 && isfinite(m) && !short_row ? __double2float_rd(m * (1.0 - 1e-6)) : 0.0f);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -520,7 +526,7 @@ __device__ __forceinline__ void tile_info_body(bool active, const T* rec, const 
       }
       o[6] = bad ? -1.0f : mu;  // +inf: no points (the box is empty)
       o[7] = 0.0f;
-      sbox[(g.t0 + t) * 8 + warp] = make_float4(mn[0], mn[1], mn[2], o[6]);
+      sbox[(g.t0 + t) * 8 + warp] = make_float4(mn[0], mn[1], mn[2], bad ? NAN : mu);
       sbox[(g.t0 + t) * 8 + 4 + warp] = make_float4(mx[0], mx[1], mx[2], 0.f);
     }
   }
@@ -545,7 +551,8 @@ __device__ __forceinline__ void tile_info_body(bool active, const T* rec, const 
     }
     o[6] = bad ? -1.0f : (mu < INFINITY ? mu : 0.0f);  // -1: the tile has no key bound
     o[7] = 0.0f;
-    for (int m = 0; m < 7; ++m) tbox[m * tplane + g.t0 + t] = o[m];
+    for (int m = 0; m < 6; ++m) tbox[m * tplane + g.t0 + t] = o[m];
+    tbox[6 * tplane + g.t0 + t] = bad ? NAN : o[6];
   }
 }
 
@@ -747,7 +754,7 @@ __global__ void __launch_bounds__(kIndexThreads) index_cluster_kernel(IndexParam
 
 // Boxes of groups of 32 tiles (warp blockIdx.x of batch element or cloud
 // blockIdx.y): the search tests a group before its tiles.  mu is the least of
-// the group's tiles, -1 where one has no bound.
+// the group's tiles, NaN where one has no bound.
 __global__ void __launch_bounds__(32) group_box_kernel(const CloudDesc* __restrict__ cd, int ntile, int ngroup,
                                                        const float* __restrict__ tbox, int64_t tplane,
                                                        float* __restrict__ gbox, int64_t gplane) {
@@ -759,6 +766,7 @@ __global__ void __launch_bounds__(32) group_box_kernel(const CloudDesc* __restri
   float v[7];
 #pragma unroll
   for (int m = 0; m < 7; ++m) v[m] = t < nt ? tbox[m * tplane + t0 + t] : (m >= 3 && m < 6 ? -INFINITY : INFINITY);
+  const bool none = __any_sync(0xffffffffu, v[6] != v[6]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
@@ -769,7 +777,8 @@ __global__ void __launch_bounds__(32) group_box_kernel(const CloudDesc* __restri
   if (lane == 0) {
     const int64_t g0 = (cd ? first_group(t0, b) : (int64_t)b * ngroup) + gi;
 #pragma unroll
-    for (int m = 0; m < 7; ++m) gbox[m * gplane + g0] = v[m];
+    for (int m = 0; m < 6; ++m) gbox[m * gplane + g0] = v[m];
+    gbox[6 * gplane + g0] = none ? NAN : v[6];
   }
 }
 

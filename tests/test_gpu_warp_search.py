@@ -165,3 +165,53 @@ def test_flagged_queries_replay_as_the_cpu_oracle(P, K, order):
     _, _, d_ref, i_ref = O.forward_f32(*x, K, with_features=False)
     assert np.array_equal(out[3].cpu().numpy(), i_ref)
     assert np.array_equal(out[2].cpu().numpy().view(np.int32), d_ref.view(np.int32))
+
+
+def _scaled(dtype, Q, P, at, row, sig, seed):
+    """Unit-cube clouds with rotations, coordinates times `at`, rows of R times `row`, sigma times `sig`."""
+    g = torch.Generator().manual_seed(seed)
+    q = torch.rand(1, Q, 3, generator=g, dtype=torch.float64) * at
+    p = torch.rand(1, P, 3, generator=g, dtype=torch.float64) * at
+    f = torch.rand(1, P, 4, generator=g, dtype=torch.float64)
+    sigma = (torch.rand(1, P, 3, generator=g, dtype=torch.float64) + 0.5) * sig
+    R = torch.linalg.qr(torch.randn(1, P, 3, 3, generator=g, dtype=torch.float64))[0] * row
+    return [t.to(dtype).contiguous() for t in (q, p, f, sigma, R)]
+
+
+# Scales at which the bounds that cull tiles leave the range of FP32 (they are
+# FP32 for FP64 calls too) while every key is finite and almost all differ.
+@pytest.mark.parametrize("dtype,K,at,row,sig", [
+    (torch.float64, 16, 1e21, 1, 1),         # squared distances above the largest float
+    (torch.float64, 16, 1e21, 1, 1e-42),     # and the bound factor below the normal ones
+    (torch.float64, 16, 1e21, 1, 1e-44),
+    (torch.float64, 16, 1, 1, 1e39),         # the bound factor above the largest float
+    (torch.float64, 33, 1e10, 1, 1e25),      # the product
+    (torch.float64, 16, 3e-22, 1, 1),        # squared distances among the subnormal ones
+    (torch.float64, 16, 3e-20, 1, 1e30),
+    (torch.float64, 65, 1e-160, 1, 1),       # below them
+    (torch.float64, 16, 1e40, 1, 1),         # coordinates above the largest float
+    (torch.float64, 16, 1, 1e-7, 1),         # short rows
+    (torch.float32, 40, 1e21, 1e-3, 1),
+    (torch.float32, 40, 1e-4, 1e10, 1e20),
+    (torch.float32, 40, 3e-20, 1, 1),        # subnormal keys
+    (torch.float32, 40, 3e-20, 1, 1e30),
+    (torch.float32, 40, 1e-18, 1e-3, 1e30),  # squares of rotated offsets among the subnormal ones
+    (torch.float32, 40, 1e-14, 1e-7, 1e30),
+])
+def test_bounds_at_scales_beyond_the_floats_range(dtype, K, at, row, sig):
+    x = [t.to(DEV) for t in _scaled(dtype, 200, 4096, at, row, sig, seed=K)]
+    _compare(x, K)
+
+
+@pytest.mark.parametrize("at,row,sig", [
+    (1e21, 1e-3, 1), (1e-4, 1e10, 1e20), (3e-20, 1, 1), (3e-20, 1, 1e30), (1e-18, 1e-3, 1e30), (1e-14, 1e-7, 1e30),
+])
+def test_scaled_forward_matches_the_cpu_oracle(at, row, sig):
+    from cuda_knn_aggregate import capi
+
+    x = _scaled(torch.float32, 200, 4096, at, row, sig, seed=5)
+    out = _call([t.to(DEV) for t in x], 16, capi.lib().knnag_forward_workspace_bytes(1, 200, 4096, 4, 16, capi.F32))
+    _, _, d_ref, i_ref = O.forward_f32(*x, 16, with_features=False)
+    assert np.isfinite(d_ref).all()
+    assert np.array_equal(out[3].cpu().numpy(), i_ref)
+    assert np.array_equal(out[2].cpu().numpy().view(np.int32), d_ref.view(np.int32))
