@@ -139,14 +139,15 @@ __device__ __forceinline__ void sort_group(int (&v)[R], int r) {
 }
 
 // Sortable int of a key's leading bits with the window slot in its low bits.
+// The sum makes -0 the +0 it equals.
 template <int BITS>
 __device__ __forceinline__ int tagged(float key, int slot) {
-  const int b = __float_as_int(key);
+  const int b = __float_as_int(__fadd_rn(key, 0.f));
   return ((b ^ ((b >> 31) & 0x7fffffff)) & ~((1 << BITS) - 1)) | slot;
 }
 template <int BITS>
 __device__ __forceinline__ int tagged(double key, int slot) {
-  const int b = __double2hiint(key);
+  const int b = __double2hiint(__dadd_rn(key, 0.0));
   return ((b ^ ((b >> 31) & 0x7fffffff)) & ~((1 << BITS) - 1)) | slot;
 }
 

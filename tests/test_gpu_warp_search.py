@@ -215,3 +215,23 @@ def test_scaled_forward_matches_the_cpu_oracle(at, row, sig):
     assert np.isfinite(d_ref).all()
     assert np.array_equal(out[3].cpu().numpy(), i_ref)
     assert np.array_equal(out[2].cpu().numpy().view(np.int32), d_ref.view(np.int32))
+
+
+@pytest.mark.parametrize("dtype,P,K", [
+    (torch.float32, 64, 32), (torch.float32, 128, 64), (torch.float64, 200, 128), (torch.float32, 256, 128),
+])
+def test_zeros_of_either_sign_tie(dtype, P, K):
+    """K - 1 negative keys, then +0 and -0: equal, so the first of the two
+    points in index order takes the last place of a full list."""
+    from cuda_knn_aggregate import capi
+
+    q, p, f, _, R = _scaled(dtype, 9, P, 1, 1, 1, seed=K)
+    sigma = torch.ones(1, P, 3, dtype=dtype)
+    sigma[:, 1:K] = -1
+    sigma[:, 0], sigma[:, K] = 0.0, -0.0
+    x = [q, p, f, sigma, R]
+    if P >= 128:
+        _compare([t.to(DEV) for t in x], K)
+    if dtype == torch.float32:
+        out = _call([t.to(DEV) for t in x], K, capi.lib().knnag_forward_workspace_bytes(1, 9, P, 4, K, capi.F32))
+        assert np.array_equal(out[3].cpu().numpy(), O.forward_f32(*x, K, with_features=False)[3])
