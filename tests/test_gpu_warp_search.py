@@ -235,3 +235,54 @@ def test_zeros_of_either_sign_tie(dtype, P, K):
     if dtype == torch.float32:
         out = _call([t.to(DEV) for t in x], K, capi.lib().knnag_forward_workspace_bytes(1, 9, P, 4, K, capi.F32))
         assert np.array_equal(out[3].cpu().numpy(), O.forward_f32(*x, K, with_features=False)[3])
+
+
+@pytest.mark.parametrize("dtype,B,Q,P,F,K", [
+    (torch.float64, 1, 400, 128, 5, 1),      # one chunk of points
+    (torch.float64, 1, 400, 512, 4, 32),     # K <= 32: a whole one,
+    (torch.float64, 3, 160, 513, 4, 9),      # and a point more; several clouds
+    (torch.float64, 1, 170, 385, 4, 64),     # K <= 64,
+    (torch.float64, 1, 170, 1537, 4, 65),    # K <= 128
+    (torch.float32, 1, 400, 768, 4, 33), (torch.float32, 2, 300, 1537, 4, 64), (torch.float32, 1, 200, 1025, 4, 128),
+    (torch.float32, 1, 500, 33000, 4, 40),   # clusters of eight CTAs
+    (torch.float64, 90, 11, 150, 4, 3),      # sixteen queries of two or three clouds
+    (torch.float64, 2, 2100000, 128, 1, 2),  # more rows than are put in order
+])
+def test_many_flagged_queries(dtype, B, Q, P, F, K):
+    _compare(_inputs("ties", B, Q, P, F, dtype, seed=P + K), K)
+
+
+@pytest.mark.parametrize("B,Q,P,K", [(1, 400, 1024, 32), (5, 100, 1025, 7), (1, 190, 12000, 16), (2, 160000, 130, 3)])
+def test_many_flagged_queries_match_the_cpu_oracle(B, Q, P, K):
+    from cuda_knn_aggregate import capi
+
+    x = _inputs("ties", B, Q, P, 4, torch.float32, seed=Q + P)
+    out = _call(x, K, capi.lib().knnag_forward_workspace_bytes(B, Q, P, 4, K, capi.F32))
+    _, _, d_ref, i_ref = O.forward_f32(*[t.cpu() for t in x], K, with_features=False)
+    assert np.array_equal(out[3].cpu().numpy(), i_ref)
+    assert np.array_equal(out[2].cpu().numpy().view(np.int32), d_ref.view(np.int32))
+
+
+def test_many_flagged_queries_of_ragged_clouds():
+    """Segments of tied clouds of very different sizes, each equal to the uniform op's call."""
+    from cuda_knn_aggregate import knn_aggregate_aniso
+    from cuda_knn_aggregate.ragged import CloudSet, ragged_forward
+
+    sizes = [40, 700, 5, 20000, 1025, 3000, 64]
+    xs = [_inputs("ties", 1, 1, P, 4, torch.float32, seed=P) for P in sizes]
+    cloud = lambda k: torch.cat([x[k][0] for x in xs]).contiguous()  # noqa: E731
+    clouds = CloudSet(cloud(1), cloud(3), cloud(4), cloud(2), sizes)
+    order = [3, 0, 1, 2, 1, 4, 5, 6, 3, 5]
+    Qs = [90, 33, 301, 7, 1, 160, 200, 64, 45, 500]
+    Ks = [16, 32, 3, 5, 1, 12, 8, 32, 9, 31]
+    qs = [_inputs("ties", 1, Q, 1, 1, torch.float32, seed=Q)[0][0] for Q in Qs]
+    out = ragged_forward(clouds, torch.cat(qs).contiguous(), order, Qs, Ks)
+    q0 = e0 = 0
+    for c, Q, K, q in zip(order, Qs, Ks, qs):
+        _, p, f, sigma, R = xs[c]
+        f_out, w, dists, idxs = knn_aggregate_aniso(q[None], p, f, sigma, R, K)
+        for got, want in ((out.f_out[q0:q0 + Q], f_out[0]), (out.w_out[e0:e0 + Q * K], w[0].reshape(-1)),
+                          (out.dists[e0:e0 + Q * K], dists[0].reshape(-1))):
+            assert torch.equal(_bits(got), _bits(want))
+        assert torch.equal(out.idxs[e0:e0 + Q * K], idxs[0].reshape(-1))
+        q0, e0 = q0 + Q, e0 + Q * K
