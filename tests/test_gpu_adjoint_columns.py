@@ -79,3 +79,33 @@ def test_broadcast_gradient_query_sides(B, Q, P, K):
 
 def _rel(a, b):
     return float((a.cpu().double() - b).norm() / b.norm())
+
+
+@pytest.mark.parametrize("F", [64, 512, 5, 70])  # 16 and 32 lanes a query, 16-byte columns; the same with single ones
+def test_ragged_gradients_of_a_given_grad_f_out(F):
+    """Segments of K 3, 17 and 32 over clouds of different sizes, odd query
+    counts, so that a warp serves queries of two segments; a query's sums do not
+    depend on its neighbour in the warp: equal to the uniform op's to the bit."""
+    from cuda_knn_aggregate import knn_aggregate_aniso
+    from cuda_knn_aggregate.ragged import CloudSet, ragged_forward
+
+    g = torch.Generator().manual_seed(F)
+    sizes = [300, 33, 1000, 70]
+    P = sum(sizes)
+    p, sigma, f = (torch.rand(P, n, generator=g).cuda() for n in (3, 3, F))
+    R = torch.linalg.qr(torch.randn(P, 3, 3, generator=g))[0].contiguous().cuda()
+    clouds = CloudSet(p, sigma, R, f, sizes)
+    order, Qs, Ks = [0, 1, 2, 3, 1, 0], [7, 5, 41, 1, 33, 9], [17, 32, 3, 32, 3, 17]
+    q = torch.rand(sum(Qs), 3, generator=g).cuda()
+    gfo = torch.randn(sum(Qs), F, generator=g).cuda()
+    res = ragged_forward(clouds, q, order, Qs, Ks, grad_q=[True] * 5 + [False], grad_f_out=gfo)
+    q0 = 0
+    for i, (c, Q, K) in enumerate(zip(order, Qs, Ks)):
+        rows = slice(sum(sizes[:c]), sum(sizes[:c + 1]))
+        qi = q[q0:q0 + Q].clone()[None].requires_grad_(True)
+        f_out = knn_aggregate_aniso(qi, *(t[rows].clone()[None] for t in (p, f, sigma, R)), K)[0]
+        assert torch.equal(res.f_out[q0:q0 + Q], f_out[0].detach())
+        if i < 5:
+            (dq,) = torch.autograd.grad(f_out, qi, gfo[q0:q0 + Q].clone()[None])
+            assert torch.equal(res.dq[q0:q0 + Q], dq[0])
+        q0 += Q
