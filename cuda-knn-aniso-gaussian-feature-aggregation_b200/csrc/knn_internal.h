@@ -168,7 +168,7 @@ inline bool search_setting_ok(int shape) { return search_shape_ok(shape) || shap
 // the caller passed no points buffer) | pair tiles (FP32 fast path).
 struct FwdLayout {
   size_t status, flag_list, rec, pairs, total;
-  // spatial index (FP32 search path): bound parts [B*kBoundParts*8], cell counts / offsets
+  // spatial index (FP32 search path): bound parts [B*bound_parts(B)*8], cell counts / offsets
   // [B*cells(+1)], point and query permutations, tile boxes [B*ntile*8]
   size_t bounds, cell_count, cell_offset, perm_p, perm_q, tinfo;
   size_t qseed;  // [B*Q] ints: seed positions of the sorted queries
@@ -309,11 +309,17 @@ int backward_impl(const BwdArgs& x, cudaStream_t st);
 int launch_pack_points(const void* p, const void* sigma, const void* R, int B, int P, int dtype, void* rec,
                        cudaStream_t st, int* zero_words = nullptr, int n_zero = 0, int* zero_rows = nullptr,
                        int64_t zero_rows2 = 0);
-// Chunks per batch element of the FP32 packing kernel that also bounds the
-// points: chunk c of element b writes its box to parts[(b * kBoundParts +
-// c) * 8 ...] (min xyz, max xyz), which the cell kernels reduce.  128 of them:
-// with 32, a quarter of the SMs packed B = 1, P = 131072 in 33 us; 128 take 12.
-constexpr int kBoundParts = 128;
+// Chunks per batch element of the packing kernel that also bounds the points:
+// chunk c of element b writes its box to parts[(b * bound_parts(B) + c) * 8 ...]
+// (min xyz, max xyz), which the cell kernels reduce.  128 for few elements (with
+// 32, a quarter of the SMs packed B = 1, P = 131072 in 33 us; 128 take 12), for
+// many no more than the chip's eight CTAs per SM: at B = 512, P = 64 128
+// chunks an element take 91 us, 32 29 us, the two of this rule 5 us.
+inline int bound_parts(int B) {
+  int n = 128;
+  while (n > 1 && (int64_t)n * B > 8 * 148) n /= 2;
+  return n;
+}
 template <typename T>
 int launch_pack_points_bounded(const T* p, const T* sigma, const T* R, const T* q, int B, int Q, int P, T* rec,
                                float* parts, float* pf, float* qf, cudaStream_t st, int* zero_words, int n_zero,

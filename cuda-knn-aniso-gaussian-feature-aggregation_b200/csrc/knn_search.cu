@@ -18,7 +18,7 @@ namespace knnag {
 
 // ------------------------------------------------------------------ packing
 
-// Packing of the search path, grid (kBoundParts, B): CTA (c, b) packs
+// Packing of the search path, grid (bound_parts(B), B): CTA (c, b) packs
 // chunk c of batch element b's points, writes the chunk's bounding box to
 // parts (what the cell kernels reduce to the element's box), zeroes the
 // chunk's adjacency counts (zero_rows, optional) and its share of the cell
@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(256) pack_points_bounded_kernel(
   for (int64_t i = flat; i < n_cells; i += nthreads) zero_cells[i] = 0;
   if constexpr (sizeof(T) == 8)
     for (int64_t i = flat; i < (int64_t)gridDim.y * Q * 3; i += nthreads) qf[i] = (float)q[i];
-  const int chunk = (P + kBoundParts - 1) / kBoundParts;
+  const int chunk = (int)(((int64_t)P + gridDim.x - 1) / gridDim.x);
   const int i0 = min(P, c * chunk), i1 = min(P, i0 + chunk);
   float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
   for (int k = i0 + tid; k < i1; k += blockDim.x) {
@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(256) pack_points_bounded_kernel(
   if (tid < 6) {
     float v = tid < 3 ? INFINITY : -INFINITY;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v = tid < 3 ? fminf(v, red[tid][w]) : fmaxf(v, red[tid][w]);
-    parts[((int64_t)b * kBoundParts + c) * 8 + tid] = v;
+    parts[((int64_t)b * gridDim.x + c) * 8 + tid] = v;
   }
 }
 
@@ -657,8 +657,8 @@ FwdLayout fwd_layout(int B, int Q, int P, int K, int dtype, bool own_rec, bool i
     // what the sort alone uses, and in the same place what the tile-info kernel
     // writes after it: the tensor-core filter's B operands
     const size_t sort_at = off;
-    L.bounds = off;  // per element kBoundParts partial boxes
-    off += align256((size_t)B * kBoundParts * 8 * 4);
+    L.bounds = off;  // per element bound_parts(B) partial boxes
+    off += align256((size_t)B * bound_parts(B) * 8 * 4);
     // point and query cells of each batch element, sorted together
     L.cell_count = off;
     off += align256(2 * (size_t)B * cells * 4);
@@ -717,7 +717,7 @@ template <typename T>
 int launch_pack_points_bounded(const T* p, const T* sigma, const T* R, const T* q, int B, int Q, int P, T* rec,
                                float* parts, float* pf, float* qf, cudaStream_t st, int* zero_words, int n_zero,
                                int* zero_rows, int64_t zero_rows2, int* zero_cells, int64_t n_cells) {
-  pack_points_bounded_kernel<T><<<dim3(kBoundParts, B), 256, 0, st>>>(p, sigma, R, q, Q, P, rec, parts, pf, qf,
+  pack_points_bounded_kernel<T><<<dim3(bound_parts(B), B), 256, 0, st>>>(p, sigma, R, q, Q, P, rec, parts, pf, qf,
                                                                       zero_words, n_zero, zero_rows, zero_rows2, zero_cells,
                                                                       n_cells);
   note_launches(1);

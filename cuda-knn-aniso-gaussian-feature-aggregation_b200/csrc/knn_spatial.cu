@@ -820,14 +820,15 @@ int launch_spatial_index(const float* qf, const float* pf, const T* rec, int B, 
   const int ntile = P_pad / kTilePoints;
   GroupMap pm{P, bits, nullptr, nullptr, nullptr, nullptr, nullptr};
   GroupMap qm{Q, bits, nullptr, nullptr, nullptr, nullptr, nullptr};
-  // the packing kernel wrote kBoundParts partial boxes per element (reduced
+  // the packing kernel wrote bound_parts(B) partial boxes per element (reduced
   // by the cell kernels) and zeroed the cell counts.  Points and queries in
   // one counting sort: their cells are scanned together, so the queries'
   // positions start after all points' and land in perm_q, which follows perm_p
   const int64_t nc = 2 * (int64_t)B * cells;
-  const CellJob jp = sizeof(T) == 4 ? CellJob{reinterpret_cast<const float*>(rec) + kNPX, kRecLen, 1, pm, 0, kBoundParts}
-                                    : CellJob{pf, 3, 0, pm, 0, kBoundParts};
-  const CellJob jq{qf, 3, 0, qm, B * cells, kBoundParts, reinterpret_cast<int*>(ws + L.qseed), (int64_t)B * P};
+  const int nparts = bound_parts(B);
+  const CellJob jp = sizeof(T) == 4 ? CellJob{reinterpret_cast<const float*>(rec) + kNPX, kRecLen, 1, pm, 0, nparts}
+                                    : CellJob{pf, 3, 0, pm, 0, nparts};
+  const CellJob jq{qf, 3, 0, qm, B * cells, nparts, reinterpret_cast<int*>(ws + L.qseed), (int64_t)B * P};
   const dim3 grid(grid_x(P > Q ? P : Q, sms, B), B, 2);
   cell_count_kernel<<<grid, 256, 0, st>>>(jp, jq, bnd, cnt);
   if (nc <= kScatterScanMax) {

@@ -140,6 +140,23 @@ def test_forward_matches_the_cpu_oracle(kind, B, Q, P, K):
     assert np.array_equal(d.view(np.int32)[~np.isnan(d)], d_ref.view(np.int32)[~np.isnan(d)])
 
 
+@pytest.mark.parametrize("B,Q,P,K", [
+    (9, 7, 3, 2),        # 128 chunks of an element's points, most of them empty
+    (10, 5, 200, 3),     # 64
+    (75, 5, 70, 5),      # 8
+    (593, 3, 33, 4),     # 1
+    (1200, 2, 300, 3),   # 1, and more of them than run at a time
+])
+def test_many_elements_match_the_cpu_oracle(B, Q, P, K):
+    from cuda_knn_aggregate import capi
+
+    x = _inputs("rand", B, Q, P, 4, torch.float32, seed=B)
+    out = _call(x, K, capi.lib().knnag_forward_workspace_bytes(B, Q, P, 4, K, capi.F32))
+    _, _, d_ref, i_ref = O.forward_f32(*[t.cpu() for t in x], K, with_features=False)
+    assert np.array_equal(out[3].cpu().numpy(), i_ref)
+    assert np.array_equal(out[2].cpu().numpy().view(np.int32), d_ref.view(np.int32))
+
+
 @pytest.mark.parametrize("P,K,order", [
     (700, 12, "lattice"),       # one CTA per query, first ranges only
     (9000, 32, "lattice"),      # two CTAs, two ranges per warp
