@@ -110,7 +110,7 @@ int knnag_version(void) { return 10000; }
 size_t knnag_forward_workspace_bytes(int B, int Q, int P, int F, int K, int dtype) {
   (void)F;
   if (B < 0 || Q < 0 || P < 0 || K < 1) return 0;
-  return fwd_layout(B, Q, P, K, dtype, true, forward_indexed(B, P, K, dtype)).total;
+  return fwd_layout(B, Q, P, K, dtype, true, forward_indexed(B, Q, P, K, dtype)).total;
 }
 
 size_t knnag_points_bytes(int B, int P, int dtype) {

@@ -181,9 +181,15 @@ struct FwdLayout {
 // Whether a call is served through the spatial index (else by the exact
 // kernel).  FP64 and K > 32 had only the exact kernel and its small
 // workspace: they take the index where its padded tiles at most double the
-// points and the launches' grids hold the batch.
-inline bool forward_indexed(int B, int P, int K, int dtype) {
+// points and the launches' grids hold the batch.  A few FP64 queries of a small
+// cloud and few neighbours stay with the exact kernel, one or two per SM and hardly
+// a turn of MinK each: 296 queries take 12 us there and 23 through the index at P =
+// 128, K = 1, 25 and 27 at P = 200, K = 8, 23 and 27 at P = 128, K = 16, but 29 and
+// 29 at P = 200, K = 16; 740 of them 27 and 25 at P = 128, K = 8.  MinK's turns grow
+// with the points where these come ever nearer (P = 200: 57 and 21), so P is bound too.
+inline bool forward_indexed(int B, int Q, int P, int K, int dtype) {
   if (dtype == KNNAG_F32 && K <= 32) return true;
+  if (dtype == KNNAG_F64 && (int64_t)B * Q <= 256 && P <= 256 && (int64_t)K * P <= 2048) return false;
   return K <= kWarpSearchMaxK && P >= kTilePoints && B <= 65535 && (int64_t)P <= (int64_t)kSearchMaxTiles * kTilePoints;
 }
 // Grid bits per axis of n elements: 8^bits cells hold at most 8 of them each on

@@ -704,7 +704,7 @@ FwdLayout fwd_layout(int B, int Q, int P, int K, int dtype, bool own_rec, bool i
 }
 
 FwdLayout fwd_layout_in(int B, int Q, int P, int K, int dtype, bool own_rec, size_t bytes, bool* indexed) {
-  *indexed = forward_indexed(B, P, K, dtype);
+  *indexed = forward_indexed(B, Q, P, K, dtype);
   FwdLayout L = fwd_layout(B, Q, P, K, dtype, own_rec, *indexed);
   if (*indexed && L.total > bytes && (dtype == KNNAG_F64 || K > 32)) {
     *indexed = false;

@@ -40,6 +40,22 @@ def test_workspace_queries():
     assert lib.knnag_backward_workspace_bytes(2, 12288, 4096, 64, 16, capi.F64) > 0
 
 
+@pytest.mark.parametrize("B,Q,P,K,dtype,exact", [
+    (1, 1, 127, 9, 1, True), (1, 256, 128, 16, 1, True), (4, 64, 256, 8, 1, True), (1, 256, 256, 1, 1, True),
+    (1, 257, 128, 1, 1, False), (4, 65, 128, 1, 1, False), (1, 1, 257, 1, 1, False), (1, 1, 128, 17, 1, False),
+    (1, 1, 1 << 21, 9, 1, False), (1, 1, 128, 33, 0, False), (1, 1, 127, 33, 0, True),
+])
+def test_which_calls_have_no_index(B, Q, P, K, dtype, exact):
+    """The exact kernel serves a call alone where its records and flag list are all the workspace there is."""
+    from cuda_knn_aggregate import capi
+
+    assert (capi.F32, capi.F64) == (0, 1)
+    r256 = lambda n: (n + 255) // 256 * 256  # noqa: E731
+    lean = 256 + r256(B * Q * 4) + r256(B * P * 16 * (8 if dtype else 4))
+    got = capi.lib().knnag_forward_workspace_bytes(B, Q, P, 4, K, dtype)
+    assert (got == lean) if exact else (got > lean)
+
+
 def test_validation_before_device_work():
     from cuda_knn_aggregate import capi
 
