@@ -15,30 +15,27 @@
 
 namespace knnag {
 
-// A warp takes four queries.  The K (query, neighbour) pairs of all four first:
-// key from the packed record, w = exp(-key) (-> dists, w_out); then
-// f_out = sum_k w_k f[idx_k] in k order, 8 lanes per query side by side (16
-// bytes a lane where the rows allow), eight rows in flight.  The neighbour
-// index comes from `idxs` [B,Q,K] or, for the lookup, from `table` [P,K] at
-// row nearest[b*Q+q] (and is written to idxs_out).  An index outside [0, P)
-// contributes nothing (w = 0, dist = +inf).
+// A warp takes N queries (4, 2 or 1).  The K (query, neighbour) pairs of all of
+// them first: key from the packed record, w = exp(-key) (-> dists, w_out); then
+// f_out = sum_k w_k f[idx_k] in k order, 32 / N lanes per query side by side: 16
+// bytes a lane and eight rows in flight (VEC, where the rows allow) or one column a
+// lane.  The neighbour index comes from `idxs` [B,Q,K] or, for the lookup, from
+// `table` [P,K] at row nearest[b*Q+q] (and is written to idxs_out).  An index
+// outside [0, P) contributes nothing (w = 0, dist = +inf).
 //
-// Bound by the gathered rows, which L2 serves (K * 4 F bytes per query): with a
-// warp per query and scalar loads 28 us at B = 2, Q = 12288, K = 16, F = 64,
-// now 24 us.
-constexpr int kGatherQueries = 4;
-
-template <typename T>
-__global__ void __launch_bounds__(256) gather_aggregate_kernel(const T* __restrict__ q, const T* __restrict__ f,
-                                                              const T* __restrict__ rec,
-                                                              const int64_t* __restrict__ idxs,
-                                                              const int64_t* __restrict__ table,
-                                                              const int* __restrict__ nearest, int tstride, int B,
-                                                              int Q, int P, int F, int K, int vec,
-                                                              T* __restrict__ f_out, T* __restrict__ w_out,
-                                                              T* __restrict__ dists, int64_t* __restrict__ idxs_out) {
+// Bound by the gathered rows, which L2 serves (K * F values per query).  With the
+// packing of the points, at B = 2, Q = 12288, K = 16: F = 64 31 us with a query a
+// warp and a column a lane, 25 with four queries; F = 256 82 and, with a query a warp
+// and 16 bytes a lane, 47.  Three CTAs per SM for the rows in flight (two: 27 and 64).
+template <typename T, int N, bool VEC>
+__global__ void __launch_bounds__(256, VEC ? 3 : 5)
+    gather_aggregate_kernel(const T* __restrict__ q, const T* __restrict__ f, const T* __restrict__ rec,
+                            const int64_t* __restrict__ idxs, const int64_t* __restrict__ table,
+                            const int* __restrict__ nearest, int tstride, int B, int Q, int P, int F, int K,
+                            T* __restrict__ f_out, T* __restrict__ w_out, T* __restrict__ dists,
+                            int64_t* __restrict__ idxs_out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int N = kGatherQueries, G = 32 / N;  // queries of the warp, lanes per query
+  constexpr int G = 32 / N;  // lanes per query
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane / G, gl = lane % G;
   T* sw = reinterpret_cast<T*>(smem_raw) + (size_t)(warp * N + sub) * K;
   int* si = reinterpret_cast<int*>(reinterpret_cast<T*>(smem_raw) + (size_t)(blockDim.x >> 5) * N * K) +
@@ -48,7 +45,7 @@ __global__ void __launch_bounds__(256) gather_aggregate_kernel(const T* __restri
   const int64_t nw = (gridDim.x * (int64_t)blockDim.x) >> 5;
   for (int64_t base = gw * N; base < BQ; base += nw * N) {
     const int64_t bq = base + sub;
-    const int64_t b = bq / Q;
+    const int64_t b = (unsigned)bq / (unsigned)Q;  // queries are counted in 32 bits
     if (bq < BQ) {
       const T qx = q[bq * 3 + 0], qy = q[bq * 3 + 1], qz = q[bq * 3 + 2];
       const int64_t row = table ? (int64_t)nearest[bq] : 0;
@@ -70,9 +67,9 @@ __global__ void __launch_bounds__(256) gather_aggregate_kernel(const T* __restri
     __syncwarp();
     if (bq < BQ) {
       const T* fb = f + b * P * F;
-      constexpr int RB = 8, C = 16 / sizeof(T);
-      if (vec) {
+      if constexpr (VEC) {
         using V = typename Group16<T>::type;
+        constexpr int RB = 8, C = 16 / sizeof(T);
         const int cols = F / C;
         for (int c = gl; c < cols; c += G) {
           T acc[C];
@@ -92,7 +89,6 @@ __global__ void __launch_bounds__(256) gather_aggregate_kernel(const T* __restri
       } else {
         for (int c = gl; c < F; c += G) {
           T acc = T(0);
-#pragma unroll 8
           for (int k = 0; k < K; ++k)
             if (si[k] >= 0) acc = fma_rn(__ldg(fb + (int64_t)si[k] * F + c), sw[k], acc);
           f_out[bq * F + c] = acc;
@@ -249,25 +245,53 @@ int launch_nearest(const T* q, const T* p, int B, int Q, int P, int* nearest, cu
   return cudaGetLastError() == cudaSuccess ? KNNAG_OK : KNNAG_ERR_CUDA;
 }
 
+template <typename T, int N, bool VEC>
+int launch_gather_n(const T* q, const T* f, const T* rec, const int64_t* idxs, const int64_t* table, const int* nearest,
+                    int tstride, int B, int Q, int P, int F, int K, T* f_out, T* w_out, T* dists, int64_t* idxs_out,
+                    cudaStream_t st) {
+  const size_t per_query = (size_t)K * (sizeof(T) + sizeof(int));
+  int cta_warps = 8;  // fewer where the neighbours of 8 x N queries do not fit
+  while (cta_warps > 1 && cta_warps * N * per_query > 100 * 1024) cta_warps /= 2;
+  const size_t smem = cta_warps * N * per_query;
+  if (smem > 48 * 1024 && cudaFuncSetAttribute(gather_aggregate_kernel<T, N, VEC>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    return KNNAG_ERR_CUDA;
+  const int64_t warps = ((int64_t)B * Q + N - 1) / N;
+  gather_aggregate_kernel<T, N, VEC><<<variant_blocks(warps, cta_warps), 32 * cta_warps, smem, st>>>(
+      q, f, rec, idxs, table, nearest, tstride, B, Q, P, F, K, f_out, w_out, dists, idxs_out);
+  note_launches(1);
+  return cudaGetLastError() == cudaSuccess ? KNNAG_OK : KNNAG_ERR_CUDA;
+}
+
+// Queries per warp, and 16 bytes or a column a lane.  Lanes for the columns of a
+// row and no more, four queries also where a query is little work, but never so
+// few warps that the chip waits for them (12 per SM): F = 700, K = 16 at 1000 queries
+// 49, 27 and 19 us with four, two and one; F = 128, K = 64 at 12288 88, 68 and 51,
+// K = 4 14 in all ways; F = 16, K = 16 14, 17 and 19.  A query a warp and a column
+// a lane for FP64 rows of more than 128 bytes (F = 128, K = 16 at 100000 queries: 204
+// us, 16-byte groups 246 to 258) unless a query is little work (F = 24, K = 4: 49, four
+// queries 41), and for long lists of narrow rows (F = 16, K = 64: 203, 213).
 template <typename T>
 int launch_gather(const T* q, const T* f, const T* rec, const int64_t* idxs, const int64_t* table, const int* nearest,
                   int tstride, int B, int Q, int P, int F, int K, T* f_out, T* w_out, T* dists, int64_t* idxs_out,
                   cudaStream_t st) {
-  const size_t per_query = (size_t)K * (sizeof(T) + sizeof(int));
-  if (8 * per_query > 200 * 1024) return KNNAG_ERR_TOO_LARGE;
-  int cta_warps = 8;  // fewer where the neighbours of 8 x 4 queries do not fit
-  while (cta_warps > 1 && cta_warps * kGatherQueries * per_query > 100 * 1024) cta_warps /= 2;
-  const size_t smem = cta_warps * kGatherQueries * per_query;
-  if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(gather_aggregate_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-          cudaSuccess)
-    return KNNAG_ERR_CUDA;
-  const int vec = F % (int)(16 / sizeof(T)) == 0 && (uintptr_t)f % 16 == 0 && (uintptr_t)f_out % 16 == 0;
-  const int64_t warps = ((int64_t)B * Q + kGatherQueries - 1) / kGatherQueries;
-  gather_aggregate_kernel<T><<<variant_blocks(warps, cta_warps), 32 * cta_warps, smem, st>>>(q, f, rec, idxs, table, nearest, tstride, B, Q, P,
-                                                                       F, K, vec, f_out, w_out, dists, idxs_out);
-  note_launches(1);
-  return cudaGetLastError() == cudaSuccess ? KNNAG_OK : KNNAG_ERR_CUDA;
+  if (8 * (size_t)K * (sizeof(T) + sizeof(int)) > 200 * 1024) return KNNAG_ERR_TOO_LARGE;
+  constexpr int C = 16 / sizeof(T);
+  const int64_t enough = (int64_t)B * Q / (12 * 148);  // queries per warp that leave 12 warps per SM
+  const bool vec = F % C == 0 && (uintptr_t)f % 16 == 0 && (uintptr_t)f_out % 16 == 0;
+  const int cols = vec ? F / C : F;
+  const int64_t work = (int64_t)K * cols;
+  auto go = launch_gather_n<T, 1, false>;
+  if (cols <= 8 && !(vec && K > 32)) {
+    if (enough >= 2) go = vec ? launch_gather_n<T, 4, true> : launch_gather_n<T, 4, false>;
+  } else if constexpr (sizeof(T) == 8) {
+    if (vec && work <= 128 && enough >= 8) go = launch_gather_n<T, 4, true>;
+  } else if (vec && cols > 8) {
+    if (work <= 256 && enough >= 4) go = launch_gather_n<T, 4, true>;
+    else if ((work <= 256 || cols <= 16) && enough >= 2) go = launch_gather_n<T, 2, true>;
+    else go = launch_gather_n<T, 1, true>;
+  }
+  return go(q, f, rec, idxs, table, nearest, tstride, B, Q, P, F, K, f_out, w_out, dists, idxs_out, st);
 }
 }  // namespace
 

@@ -303,6 +303,41 @@ def test_precomputed_is_the_fused_ops_sum(B, Q, F, K):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dtype,B,Q,F,K", [
+    (torch.float32, 1, 3555, 16, 9),     # four queries a warp, three left over: 16 bytes a lane,
+    (torch.float32, 3, 1185, 3, 40),     # a column a lane
+    (torch.float32, 1, 7105, 64, 16),    # four of longer rows and little work
+    (torch.float32, 1, 3561, 64, 17),    # two, one left over
+    (torch.float32, 1, 3551, 64, 4),     # one, too few queries for more
+    (torch.float32, 2, 75, 260, 5),      # one, three passes over the columns
+    (torch.float32, 1, 3600, 32, 33), (torch.float32, 1, 37, 33, 33),  # one, a column a lane
+    (torch.float64, 1, 3555, 16, 9), (torch.float64, 1, 3553, 5, 40), (torch.float64, 1, 14209, 24, 10),
+    (torch.float64, 1, 14209, 24, 11), (torch.float64, 1, 300, 64, 9),
+])
+def test_precomputed_splits(dtype, B, Q, F, K):
+    """However the gather splits its work, its outputs at the fused op's indices
+    are the fused op's bit for bit, and with indices outside [0, P) among them a
+    few queries' outputs are what a call of those queries alone gives."""
+    import cuda_knn_aggregate as C
+
+    P = 600
+    q, p, f, s, R = [t.to(dtype).cuda() for t in _cloud(B, Q, P, F, seed=F + K)]
+    fo, w, d, idx = C.knn_aggregate_aniso(q, p, f, s, R, K)
+    got = C._C.knn_precomputed_aggregate_aniso_forward(q, p, f, s, R, idx, K)
+    for a, b in zip(got, (fo, w, d)):
+        assert torch.equal(a, b)
+    idx = idx.clone()
+    idx[:, ::3, 0], idx[:, 1::5, K - 1], idx[:, ::7, K // 2] = -1, P, 1 << 40
+    got = C._C.knn_precomputed_aggregate_aniso_forward(q, p, f, s, R, idx, K)
+    outside = (idx < 0) | (idx >= P)
+    assert (got[1][outside] == 0).all() and got[2][outside].isinf().all()
+    few = slice(Q - 21, Q)
+    alone = C._C.knn_precomputed_aggregate_aniso_forward(q[:, few].contiguous(), p, f, s, R, idx[:, few].contiguous(), K)
+    for a, b in zip(got, alone):
+        assert torch.equal(a[:, few], b)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("Q,P,F,K", [(1, 1, 1, 1), (65, 40, 6, 7), (700, 300, 16, 12)])
 def test_lookup_nodes_are_the_python_functions(Q, P, F, K):
     """The extension's autograd nodes and the Python classes (which a subclass
