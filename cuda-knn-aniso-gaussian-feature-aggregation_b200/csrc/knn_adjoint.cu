@@ -699,9 +699,12 @@ __device__ __forceinline__ void add_dq(const QueryParams<T>& a, const T (&rec)[k
 // First-order query side with a broadcast grad_f_out s: c_k = s *
 // rowsum(f)[idx_k] needs no F-wide dot product, so each lane takes one
 // neighbour, and a warp serves two queries when K <= 16.  A warp of a ragged
-// call takes kRowBlock consecutive rows, so that the segment is looked up once
-// for them and not by a chain of dependent loads per row.
+// call takes up to kRowBlock consecutive rows, so that the segment is looked up once
+// for them and not by a chain of dependent loads per row; one row where there are
+// no more than the warps that run at a time, which otherwise idle (50 rows, K =
+// 40: 7 us, eight to a warp 23).
 constexpr int kRowBlock = 8;
+constexpr int kBroadcastWarps = 148 * 4 * 8;  // that run at a time
 
 // Bound by the latency of a neighbour's index and record: a kernel of its own, at
 // four CTAs per SM (5: 218 us where 4 take 153 at the sizes above, 6: 242; as a
@@ -720,7 +723,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) query_order1_broa
   const int64_t nw = (gridDim.x * (int64_t)blockDim.x) >> 5;
   const T sg0 = a.gfo ? a.gfo[0] : T(1);  // ragged calls: no grad_f_out means all ones
   const SegDesc* sd = sh ? seg_descs(a.segs) : nullptr;
-  const int rows = sh ? kRowBlock : qpw;  // of a warp's turn
+  // of a warp's turn
+  const int rows = sh ? (int)min((BQ + kBroadcastWarps - 1) / kBroadcastWarps, (int64_t)kRowBlock) : qpw;
   for (int64_t turn = gw * rows; turn < BQ; turn += nw * rows) {
     int s = sh ? seg_of_row(sd, sh->nseg, turn) : 0;
     for (int64_t base = turn; base < BQ && base < turn + rows; base += qpw) {

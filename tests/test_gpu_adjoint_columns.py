@@ -109,3 +109,32 @@ def test_ragged_gradients_of_a_given_grad_f_out(F):
             (dq,) = torch.autograd.grad(f_out, qi, gfo[q0:q0 + Q].clone()[None])
             assert torch.equal(res.dq[q0:q0 + Q], dq[0])
         q0 += Q
+
+
+@pytest.mark.parametrize("scale", [1, 19, 160])  # one, two and eight rows a warp's turn
+def test_ragged_gradients_of_the_sum(scale):
+    """grad_f_out of ones: a warp takes one to eight consecutive rows, of
+    several segments where these are short, some without a gradient at the end;
+    equal to the uniform op's to the bit."""
+    from cuda_knn_aggregate import knn_aggregate_aniso
+    from cuda_knn_aggregate.ragged import CloudSet, ragged_forward
+
+    g = torch.Generator().manual_seed(scale)
+    sizes = [300, 33, 1000, 70]
+    P = sum(sizes)
+    p, sigma, f = (torch.rand(P, n, generator=g).cuda() for n in (3, 3, 8))
+    R = torch.linalg.qr(torch.randn(P, 3, 3, generator=g))[0].contiguous().cuda()
+    clouds = CloudSet(p, sigma, R, f, sizes)
+    order, Ks = [0, 1, 2, 3, 1, 2, 3, 0], [17, 32, 3, 32, 3, 16, 1, 8]
+    Qs = [7, 1, 41 * scale + 1, 2, 3, 211 * scale, 5, 9]
+    q = torch.rand(sum(Qs), 3, generator=g).cuda()
+    res = ragged_forward(clouds, q, order, Qs, Ks, grad_q=[True] * 7 + [False])
+    q0 = 0
+    for i, (c, Q, K) in enumerate(zip(order, Qs, Ks)):
+        if i < 7:
+            rows = slice(sum(sizes[:c]), sum(sizes[:c + 1]))
+            qi = q[q0:q0 + Q].clone()[None].requires_grad_(True)
+            f_out = knn_aggregate_aniso(qi, *(t[rows].clone()[None] for t in (p, f, sigma, R)), K)[0]
+            (dq,) = torch.autograd.grad(f_out.sum(), qi)
+            assert torch.equal(res.dq[q0:q0 + Q], dq[0])
+        q0 += Q
