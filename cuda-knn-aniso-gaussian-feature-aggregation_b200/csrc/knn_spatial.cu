@@ -945,10 +945,13 @@ int launch_cloudset_index(char* cs, const CloudSetHeader& h, const CloudDesc* cd
   tile_info_kernel<float><<<dim3(max_ntile, C), kTilePoints, 0, st>>>(
       rec, perm_p, cd_dev, 0, 0, pairs, tinfo, reinterpret_cast<float*>(cs + h.tbox_off), h.total_tiles,
       reinterpret_cast<float4*>(cs + h.sbox_off), nullptr, nullptr);
-  group_box_kernel<<<dim3((max_ntile + 31) / 32, C), 32, 0, st>>>(
-      cd_dev, 0, 0, reinterpret_cast<const float*>(cs + h.tbox_off), h.total_tiles,
-      reinterpret_cast<float*>(cs + h.gbox_off), tile_groups(h.total_tiles, C));
-  note_launches(5);  // + 1 scan
+  note_launches(4);  // + 1 scan
+  if (max_ntile > 64) {  // the search reads the boxes of clouds with more than two groups
+    group_box_kernel<<<dim3((max_ntile + 31) / 32, C), 32, 0, st>>>(
+        cd_dev, 0, 0, reinterpret_cast<const float*>(cs + h.tbox_off), h.total_tiles,
+        reinterpret_cast<float*>(cs + h.gbox_off), tile_groups(h.total_tiles, C));
+    note_launches(1);
+  }
   return cudaGetLastError() == cudaSuccess ? KNNAG_OK : KNNAG_ERR_CUDA;
 }
 

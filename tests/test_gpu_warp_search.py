@@ -303,3 +303,25 @@ def test_many_flagged_queries_of_ragged_clouds():
             assert torch.equal(_bits(got), _bits(want))
         assert torch.equal(out.idxs[e0:e0 + Q * K], idxs[0].reshape(-1))
         q0, e0 = q0 + Q, e0 + Q * K
+
+
+def test_group_boxes_of_ragged_clouds():
+    """Boxes of groups of 32 tiles are built where a cloud has more than two
+    groups, and only there: a launch less with at most 8192 points."""
+    from cuda_knn_aggregate import capi, knn_aggregate_aniso
+    from cuda_knn_aggregate.ragged import CloudSet, ragged_forward
+
+    launches = []
+    for sizes in ([8192, 300], [8193, 300]):
+        xs = [_inputs("rand", 1, 60, P, 4, torch.float32, seed=P) for P in sizes]
+        cloud = lambda k: torch.cat([x[k][0] for x in xs]).contiguous()  # noqa: E731
+        clouds = CloudSet(cloud(1), cloud(3), cloud(4), cloud(2), sizes)
+        before = capi.launch_count()
+        clouds.build()
+        launches.append(capi.launch_count() - before)
+        out = ragged_forward(clouds, cloud(0), [0, 1], [60, 60], [24, 24])
+        for i, x in enumerate(xs):
+            f_out, w, dists, idxs = knn_aggregate_aniso(*x, 24)
+            assert torch.equal(out.f_out[60 * i:60 * i + 60], f_out[0])
+            assert torch.equal(out.idxs[1440 * i:1440 * i + 1440], idxs[0].reshape(-1))
+    assert launches[0] == launches[1] - 1
