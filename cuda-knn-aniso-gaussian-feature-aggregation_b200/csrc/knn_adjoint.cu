@@ -484,7 +484,7 @@ int launch_build_adjacency(const int64_t* idxs, int B, int Q, int P, int K, void
   const int n = B * Q * K, rows = B * P, qk = Q * K;  // sizes checked < 2^31 by the caller
   const bool fused = (size_t)rows <= kFillScanRows;
   int* fill = fused ? reinterpret_cast<int*>(base + L.fill) : nullptr;
-  if (!counted) {  // else the forward counted the entries per row already
+  if (!counted || n == 0) {  // else the forward counted the entries per row already (of no queries it counts nothing)
     if (cudaMemsetAsync(cursor, 0, (size_t)rows * 4, st) != cudaSuccess) return KNNAG_ERR_CUDA;
     adj_count_kernel<<<blocks_for(n, 256), 256, 0, st>>>(idxs, n, qk, P, cursor, fill, rows);
     note_launches(1);

@@ -59,3 +59,23 @@ def test_counted_forward_and_a_second_backward(P, dtype, K):
     for _ in range(2):
         again = torch.autograd.grad(f_out, x, grad_outputs=g, retain_graph=True)
         assert all(torch.equal(a, b) for a, b in zip(first, again))
+
+
+@pytest.mark.parametrize("P", [50, 20000])  # the scan folded into the fill, and not
+def test_no_queries(P):
+    """A forward of no queries counts nothing; its adjacency has empty rows
+    whatever the buffer held before."""
+    from cuda_knn_aggregate import _C, capi, knn_aggregate_aniso
+
+    lib, K = capi.lib(), 3
+    adj = torch.full((lib.knnag_adjacency_bytes(2, 0, P, K),), 0x11, dtype=torch.uint8, device=DEV)
+    idxs = torch.empty(2, 0, K, dtype=torch.int64, device=DEV)
+    assert lib.knnag_build_adjacency_counted(capi._p(idxs), 2, 0, P, K, capi._p(adj), capi._stream(DEV)) == 0
+    assert not _C.adjacency_views(adj, 2, 0, P, K)[0].any()
+    x = [torch.rand(2, n, *s, device=DEV).requires_grad_(True) for n, s in ((0, (3,)), (P, (3,)), (P, (4,)), (P, (3,)),
+                                                                            (P, (3, 3)))]
+    f_out = knn_aggregate_aniso(*x, K)[0]
+    assert f_out.shape == (2, 0, 4)
+    with pytest.raises(RuntimeError, match="invalid argument"):  # no gradients of nothing, as before
+        torch.autograd.grad(f_out.sum(), x)
+    torch.cuda.synchronize()
