@@ -29,6 +29,7 @@
 #include <math.h>
 
 #include <algorithm>
+#include <atomic>
 
 #include "knn_common.cuh"
 #include "knn_internal.h"
@@ -833,8 +834,8 @@ int launch_v(const ExactParams<T>& a, int max_points, cudaStream_t st) {
   cfg.numAttrs = 1;
   // as many clusters as run at a time (eight CTAs find room 15 times, not 18),
   // which loop over the queries
-  static int resident[64][kReplayMaxRanks + 1];
-  int clusters = dev >= 0 && dev < 64 ? resident[dev][ranks] : 0;
+  static std::atomic<int> resident[64][kReplayMaxRanks + 1];  // by device; threads that meet find the same value
+  int clusters = dev >= 0 && dev < 64 ? resident[dev][ranks].load(std::memory_order_relaxed) : 0;
   if (!clusters) {
     cfg.gridDim = dim3((unsigned)(num_sms(dev) / ranks * ranks));
     if (cudaOccupancyMaxActiveClusters(&clusters, replay_list_kernel<T, V>, &cfg) != cudaSuccess || clusters < 1) {
@@ -842,7 +843,7 @@ int launch_v(const ExactParams<T>& a, int max_points, cudaStream_t st) {
       clusters = num_sms(dev) / ranks;
     }
     clusters = std::max(1, std::min(clusters, num_sms(dev) / ranks));
-    if (dev >= 0 && dev < 64) resident[dev][ranks] = clusters;
+    if (dev >= 0 && dev < 64) resident[dev][ranks].store(clusters, std::memory_order_relaxed);
   }
   cfg.gridDim = dim3((unsigned)(clusters * ranks));
   // A pass takes about as long as one round of clusters over up to 24576 points
